@@ -13,24 +13,40 @@
 // tensor memory; the hidden activations entering layer 2, layer 3 and the
 // output layer are split into bf16(h) + bf16(h - bf16(h)), two MMAs into one
 // accumulator (with h rounded once to BF16, training on 1e3-photon Poisson data
-// stalled at about 3x the residual an FP32 MLP reached); one CTA handles tiles of 128 coordinates and loops over
-// tiles (persistent).  256 threads: warp w reads TMEM lane quarter w & 3 (tile
-// rows 32 (w & 3) .. +31) and does the elementwise work of half w >> 2 of each
-// layer's complex units, so the sin / cos / exp chains between two MMAs are
-// split over 8 warps.
+// stalled at about 3x the residual an FP32 MLP reached).
 //
-// Backward (training): the kernel recomputes the forward of its tile (keeping
-// the FP32 h2, h3 in shared memory for the gradient steps), then
-//   G_h3 = Wo_r^T G_y,  G_z = conj(i w h) G_h (complex layers),
-//   G_z1 = Re(conj(G_h1) i w1 h1),  G_h(prev) = W_r^T G_z,  G_x = W1^T G_z1
-// on the tensor core, and accumulates the weight gradients
+// A tile of 128 coordinates is a chain of dependent MMA -> elementwise steps, so
+// the SM is kept busy by several tiles in flight, and the chain is kept short:
+//  * the output layer's MMA runs with the next tile's first one; G_h3 = Wo_r^T G_y
+//    comes with z3;
+//  * sin, cos and exp run at 16 results a clock, and rintf and the conversion of a
+//    single float to BF16 share their unit: the range reduction rounds by adding
+//    1.5 2^23 and conversions are done in pairs, off that unit;
+//  * the arithmetic between is packed two floats to an instruction.
+// One CTA per SM with several slots of 256 threads, each with a tile, buffers,
+// TMEM columns and a barrier of its own.  Forward (k_cmlp_fwd): four slots, three
+// MMA steps a tile.  Backward (k_cmlp_bwd): two slots, six MMA steps a tile:
+//   z1 | z2 | z3, G_h3 -> G_z3 | G_h2 -> G_z2 | G_h1 -> G_z1 | G_x
+//   G_z = conj(i w h) G_h (complex layers), G_z1 = Re(conj(G_h1) i w1 h1),
+//   G_h(prev) = W_r^T G_z, G_x = W1^T G_z1,
+// with the weight gradients
 //   sum_c [G_z3 | G_z2]_c^T [h2 | h1 | 1]_c,   sum_c G_z1_c^T [x | 1]_c,
 //   sum_c G_y_c^T [h3 | 1]_c
-// in TMEM across all its tiles (the appended ones column yields the bias
-// gradients).  Each CTA writes its raw accumulators once; k_cmlp_reduce sums
-// the CTA partials in a fixed order and folds the real-form blocks back into
-// complex gradients (G_W = (P+S) + i(R-Q) for [[P,Q],[R,S]]) -- deterministic,
-// no atomics.  Gradients follow torch's complex convention.
+// accumulated in TMEM across all the CTA's tiles in tile order (the appended
+// ones column yields the bias gradients).  In a tile's 256 threads, warp w
+// reads TMEM lane quarter w & 3 (tile rows 32 (w & 3) .. +31) and does the
+// elementwise work of half w >> 2 of each layer's complex units.
+// Measured on B200, 4,194,304 coordinates: forward 495 us (820 as four serial
+// steps, two CTAs per SM, rintf and single conversions), backward 1312 us (1905
+// as nine serial steps, one tile in flight).  The forward is bound by its 256
+// sin / cos / exp results per coordinate (236 us) and issue (60 %); the backward
+// by latency with two tiles in flight (issue 35 %), which is all that shared
+// memory (100 KB a tile) and TMEM (256 accumulator columns + 128 a tile) hold.
+//
+// Each CTA writes its raw accumulators once; k_cmlp_reduce sums the CTA
+// partials in a fixed order and folds the real-form blocks back into complex
+// gradients (G_W = (P+S) + i(R-Q) for [[P,Q],[R,S]]) -- deterministic, no
+// atomics.  Gradients follow torch's complex convention.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -42,51 +58,21 @@
 namespace pty {
 namespace cm {
 
-constexpr int kThreads = 256;
 constexpr int GRP = 2048;  // one group of 8 bf16 features x 128 rows
 
-// ---- shared-memory map (bytes) --------------------------------------------
+// ---- packed operand blob (bytes) ---------------------------------------------
 constexpr int S_W1 = 0;             // W1  [32 out][32 in]   K-major, LBO 512
 constexpr int S_W2 = S_W1 + 2048;   // Wr2 [64][64]          LBO 1024
 constexpr int S_W3 = S_W2 + 8192;   // Wr3 [64][64]
 constexpr int S_WO = S_W3 + 8192;   // Wor [16][64] (rows 0,1 used), LBO 256
 constexpr int kWBytes = S_WO + 2048;  // 20480
-constexpr int S_PAR = kWBytes;      // fp32 biases and omegas
-constexpr int S_BAR = S_PAR + 1024;
-constexpr int S_TMEM = S_BAR + 16;
-constexpr int S_RED = S_TMEM + 16;  // 24 floats: omega-gradient partials of 8 warps
-constexpr int S_X = S_RED + 128;    // 6 groups: x (4), ones, zeros
-constexpr int S_H = S_X + 6 * GRP;  // 18 groups: h2 (8), h1 (8), ones, zeros
-constexpr int S_H3 = S_H + 18 * GRP;  // 10 groups: h3 (8), ones, zeros
-constexpr int S_GY = S_H3 + 10 * GRP;  // 2 groups: (G_yr, G_yi, 0, ...), zeros
-constexpr int S_GZ1 = S_GY + 2 * GRP;  // 4 groups: G_z1
-constexpr int S_GZ = S_GZ1 + 4 * GRP;  // 16 groups: G_z3 (8), G_z2 (8)
-constexpr int S_ACT_END = S_GZ + 16 * GRP;
-// FP32 h2, h3 of the tile (backward only): [layer][re, im][32 units][128 rows],
-// kept from the forward recompute for the layer-3 and layer-2 gradients
-constexpr int S_HF = S_ACT_END;
-// BF16 residuals h - bf16(h) of the input of layer 2, 3 or the output layer (8
-// groups, rewritten layer by layer): each of those MMAs runs once on bf16(h) and
-// once on the residual into the same accumulator, so the hidden activations
-// reach the tensor core with about 16 significant bits instead of 8
-constexpr int S_LO_BWD = int(pty_align_up_c(S_HF + 2 * 2 * 32 * 128 * 4, 1024));
-constexpr int kSmemBwd = S_LO_BWD + 8 * GRP;  // 219136 bytes: one CTA per SM
-constexpr int S_LO_FWD = S_GY;                // the forward needs x, h, h3 and the residual plane only
-constexpr int kSmemFwd = S_LO_FWD + 8 * GRP;  // 107648 bytes: two CTAs per SM
-static_assert(kSmemBwd <= 232448 && 2 * (kSmemFwd + 1024) <= 233472, "shared-memory budget");
-
-// every MMA footprint used below stays inside [0, S_ACT_END)
-static_assert(S_GY + 16 * GRP <= S_ACT_END, "output-grad A footprint");
-static_assert(S_GZ1 + 16 * GRP <= S_ACT_END, "layer-1 grad A footprint");
 
 // ---- fp32 parameter block (floats) ------------------------------------------
 constexpr int P_B1 = 0, P_B2R = 32, P_B2I = 64, P_B3R = 96, P_B3I = 128, P_BOR = 160, P_BOI = 161,
               P_W1 = 162, P_W2 = 163, P_W3 = 164, kParFloats = 168;
 constexpr int kPackedBytes = kWBytes + kParFloats * 4;  // 21152
-
-// ---- TMEM columns -------------------------------------------------------------
-constexpr uint32_t T_D1 = 0, T_D2 = 32, T_D3 = 96, T_DO = 160, T_ACC = 224, T_ACC1 = 368, T_ACCO = 416;
-constexpr uint32_t kColsBwd = 512, kColsFwd = 256;
+// the kernels' copy of it: the parameters, then Re and Im of the BF16 output weights
+constexpr int P_WOR = kParFloats, P_WOI = P_WOR + 32, kParSmem = P_WOI + 32;
 
 // ---- raw per-CTA gradient partials (floats) ----------------------------------
 constexpr int R_W3 = 0, R_B3 = 4096, R_W2 = 4160, R_B2 = 8256, R_W1 = 8320, R_B1 = 9344, R_WO = 9376,
@@ -106,35 +92,85 @@ PTY_DEVI uint32_t pack_bf16x2(float a, float b) {
   __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
 }
-// store 8 consecutive features [f0, f0+8) of row c (f0 % 8 == 0)
-PTY_DEVI void st8(unsigned char* base, int c, int f0, const float* v) {
-  uint4 q;
-  q.x = pack_bf16x2(v[0], v[1]);
-  q.y = pack_bf16x2(v[2], v[3]);
-  q.z = pack_bf16x2(v[4], v[5]);
-  q.w = pack_bf16x2(v[6], v[7]);
-  *reinterpret_cast<uint4*>(base + cm_off(c, f0)) = q;
+// Two floats in one 64-bit register pair: add, multiply and fused multiply-add of
+// both in one issue slot (same results as the scalar instructions)
+typedef unsigned long long u64;
+PTY_DEVI u64 pk(float a, float b) {
+  u64 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+  return d;
 }
-// the same 8 values as bf16(v) at feature f0 of `hi` and as bf16(v - bf16(v))
-// at feature f_lo of `lo`
-PTY_DEVI void st8_split(unsigned char* hi, int f0, unsigned char* lo, int f_lo, int c, const float* v) {
-  float h[8], r[8];
+PTY_DEVI u64 pk(float a) { return pk(a, a); }
+PTY_DEVI void upk(u64 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+PTY_DEVI u64 add2(u64 a, u64 b) {
+  u64 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+PTY_DEVI u64 mul2(u64 a, u64 b) {
+  u64 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+PTY_DEVI u64 fma2(u64 a, u64 b, u64 c) {
+  u64 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+// a - b (the product with -1 is exact)
+PTY_DEVI u64 sub2(u64 a, u64 b) { return fma2(b, pk(-1.f), a); }
+
+// store 8 consecutive features [f0, f0+8) of row c (f0 % 8 == 0)
+PTY_DEVI void st8(unsigned char* base, int c, int f0, const u64 (&v)[4]) {
+  uint32_t q[4];
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    h[k] = __bfloat162float(__float2bfloat16_rn(v[k]));
-    r[k] = v[k] - h[k];
+  for (int j = 0; j < 4; ++j) {
+    float a, b;
+    upk(v[j], a, b);
+    q[j] = pack_bf16x2(a, b);
   }
-  st8(hi, c, f0, h);
-  st8(lo, c, f_lo, r);
+  *reinterpret_cast<uint4*>(base + cm_off(c, f0)) = make_uint4(q[0], q[1], q[2], q[3]);
+}
+// the same 8 values as bf16(v) at feature f of `hi` and, at the same place of
+// `lo`, as bf16(v - bf16(v)); conversions in pairs (a single one runs at 16 a
+// clock on the unit of sin, cos and exp, a pair at 64)
+PTY_DEVI void st8_split(unsigned char* hi, int f, unsigned char* lo, int f_lo, int c, const u64 (&v)[4]) {
+  uint32_t q[4], r[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float a, b;
+    upk(v[j], a, b);
+    q[j] = pack_bf16x2(a, b);
+    upk(sub2(v[j], pk(__uint_as_float(q[j] << 16), __uint_as_float(q[j] & 0xffff0000u))), a, b);
+    r[j] = pack_bf16x2(a, b);
+  }
+  *reinterpret_cast<uint4*>(hi + cm_off(c, f)) = make_uint4(q[0], q[1], q[2], q[3]);
+  *reinterpret_cast<uint4*>(lo + cm_off(c, f_lo)) = make_uint4(r[0], r[1], r[2], r[3]);
 }
 
-// sin and cos of a after Cody-Waite reduction by 2 pi (two-constant split of
-// 2 pi: the float nearest 2 pi plus its residual), then the SFU on [-pi, pi]
-PTY_DEVI void sincos_rr(float a, float* s, float* c) {
-  const float k = rintf(a * 0.159154943091895336f);
-  float r = fmaf(-k, 6.28318548202514648f, a);
-  r = fmaf(-k, -1.74845553e-7f, r);
-  __sincosf(r, s, c);
+// sin and cos of a pair after Cody-Waite reduction by 2 pi (two-constant split of
+// 2 pi: the float nearest 2 pi plus its residual), then the SFU on [-pi, pi].
+// The nearest integer comes from adding and taking off 1.5 2^23 (exact below
+// 2^22): rintf runs at 16 a clock on the unit that sin, cos and exp need.
+PTY_DEVI void sincos_rr(u64 a, u64* s, u64* c) {
+  const u64 k = add2(add2(mul2(a, pk(0.159154943091895336f)), pk(12582912.f)), pk(-12582912.f));
+  u64 r = fma2(k, pk(-6.28318548202514648f), a);
+  r = fma2(k, pk(1.74845553e-7f), r);
+  float r0, r1, s0, s1, c0, c1;
+  upk(r, r0, r1);
+  __sincosf(r0, &s0, &c0);
+  __sincosf(r1, &s1, &c1);
+  *s = pk(s0, s1);
+  *c = pk(c0, c1);
+}
+
+// exp(x) = 2^(x log2 e) of a pair; results below the normal range flush to zero
+PTY_DEVI u64 exp_fast(u64 x) {
+  float a, b, ya, yb;
+  upk(mul2(x, pk(1.44269504088896341f)), a, b);
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(ya) : "f"(a));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(yb) : "f"(b));
+  return pk(ya, yb);
 }
 
 // ---- GEMM issue helpers (single thread) --------------------------------------
@@ -174,404 +210,619 @@ struct Args {
   int x_planar;      // x feature-major: feature f of row c at x[f * N + c]
 };
 
-template <bool BWD>
-__global__ void __launch_bounds__(kThreads, BWD ? 1 : 2) k_cmlp(const Args a) {
-  extern __shared__ __align__(1024) unsigned char sm[];
-  const int t = threadIdx.x, w = t >> 5;
-  const int quarter = w & 3;                // TMEM lane quarter of this warp
-  const int hh = w >> 2;                    // half of each layer's units handled here
-  const int row = 32 * quarter + (t & 31);  // tile row (TMEM lane) of this thread
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + S_BAR);
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + S_TMEM);
-  float* par = reinterpret_cast<float*>(sm + S_PAR);
-  float* red = reinterpret_cast<float*>(sm + S_RED);
-  float* hf = reinterpret_cast<float*>(sm + S_HF);  // valid in the backward only
-  constexpr int S_LO = BWD ? S_LO_BWD : S_LO_FWD;
-  auto hfi = [&](int layer, int part, int unit) { return ((layer * 2 + part) * 32 + unit) * 128 + row; };
-  constexpr uint32_t NCOLS = BWD ? kColsBwd : kColsFwd;
-  const uint32_t sbase = tc::smem_addr(sm);
+constexpr int kTileThreads = 256;  // threads of one tile in flight
 
-  // -- set-up: zero activations, copy weights and parameters, ones columns ----
-  constexpr int kActEnd = BWD ? S_ACT_END : S_GY;
-  for (int i = t; i < (kActEnd - S_X) / 16; i += kThreads)
-    reinterpret_cast<uint4*>(sm + S_X)[i] = make_uint4(0u, 0u, 0u, 0u);
-  for (int i = t; i < kWBytes / 16; i += kThreads)
-    reinterpret_cast<uint4*>(sm)[i] = __ldg(reinterpret_cast<const uint4*>(a.packed) + i);
-  for (int i = t; i < kParFloats; i += kThreads)
-    par[i] = __ldg(reinterpret_cast<const float*>(a.packed + kWBytes) + i);
-  __syncthreads();
-  if (hh == 0) {
-    const __nv_bfloat16 one = __float2bfloat16(1.0f);
-    *reinterpret_cast<__nv_bfloat16*>(sm + S_X + cm_off(row, 32)) = one;
-    *reinterpret_cast<__nv_bfloat16*>(sm + S_H + cm_off(row, 128)) = one;
-    *reinterpret_cast<__nv_bfloat16*>(sm + S_H3 + cm_off(row, 64)) = one;
+// the tile row, half of the units and TMEM lane offset of thread st (0 .. 255) of a tile
+struct Place {
+  int row, hh;
+  uint32_t lanes;
+};
+PTY_DEVI Place place(int st) {
+  const int w = st >> 5, quarter = w & 3;
+  return {32 * quarter + (st & 31), w >> 2, uint32_t(quarter * 32) << 16};
+}
+
+// weights, parameters and the output weights as floats into shared memory
+PTY_DEVI void load_packed(const Args& a, unsigned char* w, float* par, int t, int nt) {
+  for (int i = t; i < kWBytes / 16; i += nt)
+    reinterpret_cast<uint4*>(w)[i] = __ldg(reinterpret_cast<const uint4*>(a.packed) + i);
+  for (int i = t; i < kParFloats; i += nt) par[i] = __ldg(reinterpret_cast<const float*>(a.packed + kWBytes) + i);
+  for (int i = t; i < 64; i += nt) {  // Re Wo_k at (row 0, k), Im Wo_k at (row 1, k)
+    const __nv_bfloat16* wo = reinterpret_cast<const __nv_bfloat16*>(a.packed + S_WO);
+    par[P_WOR + i] = __bfloat162float(wo[wm_off(i >> 5, i & 31, 16) / 2]);
   }
+}
+
+// this half's 16 of row c's 32 input features
+PTY_DEVI void load_x(const Args& a, int c, int hh, u64 (&lo)[4], u64 (&hi)[4]) {
+  const bool ok = c < a.N;
+  if (a.x_planar) {  // per feature, a warp reads 32 consecutive rows
+    const float* xp = a.x + size_t(16 * hh) * a.N + c;
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = ok ? __ldg(xp + size_t(i) * a.N) : 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      lo[j] = pk(v[2 * j], v[2 * j + 1]);
+      hi[j] = pk(v[8 + 2 * j], v[9 + 2 * j]);
+    }
+  } else {
+    const float4* xp = reinterpret_cast<const float4*>(a.x + size_t(ok ? c : 0) * 32 + 16 * hh);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const float4 u = ok ? __ldg(xp + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 v = ok ? __ldg(xp + 2 + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+      lo[2 * q] = pk(u.x, u.y);
+      lo[2 * q + 1] = pk(u.z, u.w);
+      hi[2 * q] = pk(v.x, v.y);
+      hi[2 * q + 1] = pk(v.z, v.w);
+    }
+  }
+}
+
+// bring tile nt's features towards L2: a tile's loads are the first link of its chain
+PTY_DEVI void prefetch_x(const Args& a, int nt, int ntiles, int st) {
+  if (nt >= ntiles) return;
+  if (a.x_planar) {  // 32 features x 512 bytes: one 64-byte piece per thread
+    const int f = st >> 3, r0 = nt * 128 + (st & 7) * 16;
+    if (r0 < a.N) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.x + size_t(f) * a.N + r0));
+  } else {  // 128 rows x 128 bytes: 16 KB, one 64-byte piece per thread
+    const size_t off = size_t(nt) * 128 * 32 + size_t(st) * 16;
+    if (off < size_t(a.N) * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.x + off));
+  }
+}
+
+// h1 = exp(i w1 zz) of eight units
+PTY_DEVI void h_layer1(const u64 (&zz)[4], float w1, u64 (&hr)[4], u64 (&hi)[4]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) sincos_rr(mul2(zz[j], pk(w1)), &hi[j], &hr[j]);
+}
+// h = exp(i w (r + i i)) of eight units
+PTY_DEVI void h_complex(const u64 (&r)[4], const u64 (&i)[4], float w, u64 (&hr)[4], u64 (&hi)[4]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const u64 amp = exp_fast(mul2(i[j], pk(-w)));
+    u64 s, co;
+    sincos_rr(mul2(r[j], pk(w)), &s, &co);
+    hr[j] = mul2(amp, co);
+    hi[j] = mul2(amp, s);
+  }
+}
+// eight columns at taddr, plus the eight floats at b
+PTY_DEVI void ld8_bias(uint32_t taddr, const float* b, u64 (&v)[4]) {
+  float z[8];
+  tc::ld8(taddr, z);
+  const ulonglong2 p = reinterpret_cast<const ulonglong2*>(b)[0], q = reinterpret_cast<const ulonglong2*>(b)[1];
+  v[0] = add2(pk(z[0], z[1]), p.x);
+  v[1] = add2(pk(z[2], z[3]), p.y);
+  v[2] = add2(pk(z[4], z[5]), q.x);
+  v[3] = add2(pk(z[6], z[7]), q.y);
+}
+PTY_DEVI void ld8x2(uint32_t ta, u64 (&va)[4], uint32_t tb, u64 (&vb)[4]) {
+  float x[8], y[8];
+  tc::ld8x2(ta, x, tb, y);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    va[j] = pk(x[2 * j], x[2 * j + 1]);
+    vb[j] = pk(y[2 * j], y[2 * j + 1]);
+  }
+}
+PTY_DEVI void bias8(u64 (&v)[4], const float* b) {
+  const ulonglong2 p = reinterpret_cast<const ulonglong2*>(b)[0], q = reinterpret_cast<const ulonglong2*>(b)[1];
+  v[0] = add2(v[0], p.x);
+  v[1] = add2(v[1], p.y);
+  v[2] = add2(v[2], q.x);
+  v[3] = add2(v[3], q.y);
+}
+// back through h = exp(i w z): om += Re(conj(G_h) i z h), r + i i <- conj(i w h) G_h
+PTY_DEVI void grad_z(u64 (&r)[4], u64 (&i)[4], const u64 (&hr)[4], const u64 (&hi)[4], const u64 (&gr)[4],
+                     const u64 (&gi)[4], float w, u64& om) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const u64 nhi = mul2(hi[j], pk(-1.f));
+    const u64 p = fma2(i[j], nhi, mul2(r[j], hr[j])), q = fma2(i[j], hr[j], mul2(r[j], hi[j]));
+    om = add2(om, sub2(mul2(gi[j], p), mul2(gr[j], q)));
+    r[j] = mul2(fma2(hr[j], gi[j], mul2(nhi, gr[j])), pk(w));
+    i[j] = mul2(fma2(hr[j], gr[j], mul2(hi[j], gi[j])), pk(-w));
+  }
+}
+
+// barrier of one slot's threads that also agrees on `bad`
+PTY_DEVI bool slot_barrier_or(int slot, bool bad) {
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 q, %2, 0;\n\t"
+      "barrier.cta.red.or.pred p, %1, %3, q;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(any)
+      : "r"(1 + slot), "r"(uint32_t(bad)), "n"(kTileThreads)
+      : "memory");
+  return any != 0;
+}
+
+// ---- forward ---------------------------------------------------------------------
+constexpr int kFwdSlots = 4;  // tiles in flight: 4 x 256 threads, one CTA per SM
+constexpr int F_HI = 0;              // bf16(h) of the running layer: 8 groups
+constexpr int F_LO = F_HI + 8 * GRP;  // h - bf16(h): 8 groups
+constexpr int F_X = F_LO + 8 * GRP;   // x of the next tile: 4 groups
+constexpr int kFwdSlotBytes = F_X + 4 * GRP;
+constexpr int F_W = kFwdSlots * kFwdSlotBytes;
+constexpr int F_PAR = F_W + kWBytes;
+constexpr int F_BAR = F_PAR + kParSmem * 4;  // one per slot
+constexpr int F_NEXT = F_BAR + kFwdSlots * 8;  // tile counter, then each slot's next tile
+constexpr int F_TMEM = F_NEXT + 4 * (kFwdSlots + 1);
+constexpr int F_SMEM = int(pty_align_up_c(F_TMEM + 8, 128));
+static_assert(P_B1 % 4 == 0 && P_B2R % 4 == 0 && F_PAR % 16 == 0 && F_BAR % 8 == 0, "alignment");
+static_assert(F_SMEM <= 232448, "shared-memory budget");
+// TMEM columns per slot: z1, z2, z3 in turn (64), the output (16)
+constexpr uint32_t kColsFwd = 512, kColsFwdSlot = 128, T_OUT = 64;
+
+__global__ void __launch_bounds__(kFwdSlots* kTileThreads, 1) k_cmlp_fwd(const Args a) {
+  extern __shared__ __align__(1024) unsigned char sm[];
+  const int t = threadIdx.x, slot = t / kTileThreads, st = t % kTileThreads;
+  const Place pl = place(st);
+  const int row = pl.row, hh = pl.hh;
+  unsigned char* sl = sm + slot * kFwdSlotBytes;
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + F_BAR) + slot;
+  int* counter = reinterpret_cast<int*>(sm + F_NEXT);
+  volatile int* next = reinterpret_cast<int*>(sm + F_NEXT) + 1 + slot;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + F_TMEM);
+  float* par = reinterpret_cast<float*>(sm + F_PAR);
+  const uint32_t sb = tc::smem_addr(sl), wb = tc::smem_addr(sm) + F_W;
+  load_packed(a, sm + F_W, par, t, kFwdSlots * kTileThreads);
   if (t == 0) {
-    mbar_init(bar, 1);
+    for (int i = 0; i < kFwdSlots; ++i) mbar_init(reinterpret_cast<uint64_t*>(sm + F_BAR) + i, 1);
     fence_mbar_init();
+    *counter = kFwdSlots;
   }
-  if (w == 0) {
-    tc::tmem_alloc(tslot, NCOLS);
+  if (t < 32) {
+    tc::tmem_alloc(tslot, kColsFwd);
     tc::tmem_relinquish();
   }
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
-  const uint32_t tm = *tslot;
-  const uint32_t lo = uint32_t(quarter * 32) << 16;  // this warp's TMEM lane quarter
+  const uint32_t tm = *tslot, tz = tm + slot * kColsFwdSlot, lz = tz + pl.lanes;
   const float w1 = par[P_W1], w2 = par[P_W2], w3 = par[P_W3];
   uint32_t phase = 0;
-  bool abort = false;
+  bool bad = false, abort = false;
 
-  // barrier + fences, then thread 0 issues `issue`, commits, everybody waits
+  // operands written -> the slot's first thread issues `issue` -> its threads wait
+  // for the result; a wait that ran out is agreed on at the next step's barrier
   auto step = [&](auto issue) {
     tc::fence_smem_async();
     tc::fence_before();
-    __syncthreads();
+    abort = slot_barrier_or(slot, bad);
+    if (abort) return;
     tc::fence_after();
-    if (t == 0) {
+    if (st == 0) {
       issue();
       tc::commit(bar);
     }
-    const bool ok = mbar_wait_bounded(bar, phase);
-    if (__syncthreads_or(!ok)) abort = true;  // phase stays at the unfinished one
-    else phase ^= 1u;
+    bad = bad || !mbar_wait_bounded(bar, phase);
+    phase ^= 1u;
     tc::fence_after();
   };
-
-  float om1 = 0.f, om2 = 0.f, om3 = 0.f;
-  bool first = true;
-  const int ntiles = (a.N + 127) / 128;
-  // this half's 16 of row c's 32 input features (and, backward, G_y of row c)
-  auto load_inputs = [&](int cc, float (&xv)[16], float2& g) {
-    const bool ok = cc < a.N;
-    if (a.x_planar) {  // per feature, a warp reads 32 consecutive rows
-#pragma unroll
-      for (int i = 0; i < 16; ++i) xv[i] = ok ? __ldg(a.x + size_t(16 * hh + i) * a.N + cc) : 0.f;
-    } else {
-      const float4* xp = reinterpret_cast<const float4*>(a.x + size_t(ok ? cc : 0) * 32 + 16 * hh);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float4 v = ok ? __ldg(xp + q) : make_float4(0.f, 0.f, 0.f, 0.f);
-        xv[4 * q] = v.x;
-        xv[4 * q + 1] = v.y;
-        xv[4 * q + 2] = v.z;
-        xv[4 * q + 3] = v.w;
-      }
-    }
-    if constexpr (BWD) g = (ok && hh == 0) ? __ldg(a.gy + cc) : make_float2(0.f, 0.f);
+  auto output = [&] {
+    gemm_act_w(tz + T_OUT, sb + F_HI, wb + S_WO, 16, 16, 64, false);
+    gemm_act_w(tz + T_OUT, sb + F_LO, wb + S_WO, 16, 16, 64, true);
   };
-  // The tile loop is a chain of dependent MMA / elementwise steps, so a tile's
-  // input loads would stall it: the backward (registers to spare) loads the
-  // next tile's inputs while this tile computes; the forward (at its register
-  // cap) has them prefetched into L2.
-  auto prefetch_l2 = [&](int nt) {
-    if (nt < ntiles) {
-      if (a.x_planar) {  // 32 features x 512 bytes: one 64-byte piece per thread
-        const int f = t >> 3, piece = t & 7;
-        const int r0 = nt * 128 + piece * 16;
-        if (r0 < a.N) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.x + size_t(f) * a.N + r0));
-      } else {  // 128 rows x 128 bytes: 16 KB, one 64-byte piece per thread
-        const size_t off = size_t(nt) * 128 * 32 + size_t(t) * 16;
-        if (off < size_t(a.N) * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.x + off));
-      }
-    }
-  };
-  float xnext[16];
-  float2 gnext = make_float2(0.f, 0.f);
-  if constexpr (BWD) load_inputs(blockIdx.x * 128 + row, xnext, gnext);
-  for (int tile = blockIdx.x; tile < ntiles && !abort; tile += gridDim.x) {
-    const int c = tile * 128 + row;
-    const bool valid = c < a.N;
-    // -- inputs ------------------------------------------------------------------
-    {
-      float xv[16];
-      float2 g;
-      if constexpr (BWD) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) xv[i] = xnext[i];
-        g = gnext;
-        load_inputs((tile + gridDim.x) * 128 + row, xnext, gnext);  // lands during this tile
-      } else {
-        load_inputs(c, xv, g);
-        prefetch_l2(tile + gridDim.x);
-      }
-      st8(sm + S_X, row, 16 * hh, xv);
-      st8(sm + S_X, row, 16 * hh + 8, xv + 8);
-      if constexpr (BWD) {
-        if (hh == 0) {
-          const float v8[8] = {g.x, g.y, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-          st8(sm + S_GY, row, 0, v8);
-        }
-      }
-    }
-    // -- layer 1 ---------------------------------------------------------------
-    step([&] { gemm_act_w(tm + T_D1, sbase + S_X, sbase + S_W1, 32, 32, 32, false); });
-    if (abort) break;
-    {
-      const int h = hh;
-      float d[16], hr[16], hi[16];
-      tc::ld16(tm + lo + T_D1 + 16 * h, d);
-#pragma unroll
-      for (int k = 0; k < 16; ++k) sincos_rr(w1 * (d[k] + par[P_B1 + 16 * h + k]), &hi[k], &hr[k]);
-      st8_split(sm + S_H, 64 + 16 * h, sm + S_LO, 16 * h, row, hr);
-      st8_split(sm + S_H, 72 + 16 * h, sm + S_LO, 8 + 16 * h, row, hr + 8);
-      st8_split(sm + S_H, 96 + 16 * h, sm + S_LO, 32 + 16 * h, row, hi);
-      st8_split(sm + S_H, 104 + 16 * h, sm + S_LO, 40 + 16 * h, row, hi + 8);
-    }
-    // -- complex layers 2 and 3 ------------------------------------------------
-    step([&] {
-      gemm_act_w(tm + T_D2, sbase + S_H + 8 * GRP, sbase + S_W2, 64, 64, 64, false);
-      gemm_act_w(tm + T_D2, sbase + S_LO, sbase + S_W2, 64, 64, 64, true);
-    });
-    if (abort) break;
-    {
-      const int h = hh;
-      float zr[16], zi[16], hr[16], hi[16];
-      tc::ld16(tm + lo + T_D2 + 16 * h, zr);
-      tc::ld16(tm + lo + T_D2 + 32 + 16 * h, zi);
-#pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        const float r = zr[k] + par[P_B2R + 16 * h + k], i = zi[k] + par[P_B2I + 16 * h + k];
-        const float amp = __expf(-w2 * i);
-        float s, co;
-        sincos_rr(w2 * r, &s, &co);
-        hr[k] = amp * co;
-        hi[k] = amp * s;
-        if constexpr (BWD) {
-          hf[hfi(0, 0, 16 * h + k)] = hr[k];
-          hf[hfi(0, 1, 16 * h + k)] = hi[k];
-        }
-      }
-      st8_split(sm + S_H, 16 * h, sm + S_LO, 16 * h, row, hr);
-      st8_split(sm + S_H, 8 + 16 * h, sm + S_LO, 8 + 16 * h, row, hr + 8);
-      st8_split(sm + S_H, 32 + 16 * h, sm + S_LO, 32 + 16 * h, row, hi);
-      st8_split(sm + S_H, 40 + 16 * h, sm + S_LO, 40 + 16 * h, row, hi + 8);
-    }
-    step([&] {
-      gemm_act_w(tm + T_D3, sbase + S_H, sbase + S_W3, 64, 64, 64, false);
-      gemm_act_w(tm + T_D3, sbase + S_LO, sbase + S_W3, 64, 64, 64, true);
-    });
-    if (abort) break;
-    {
-      const int h = hh;
-      float zr[16], zi[16], hr[16], hi[16];
-      tc::ld16(tm + lo + T_D3 + 16 * h, zr);
-      tc::ld16(tm + lo + T_D3 + 32 + 16 * h, zi);
-#pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        const float r = zr[k] + par[P_B3R + 16 * h + k], i = zi[k] + par[P_B3I + 16 * h + k];
-        const float amp = __expf(-w3 * i);
-        float s, co;
-        sincos_rr(w3 * r, &s, &co);
-        hr[k] = amp * co;
-        hi[k] = amp * s;
-        if constexpr (BWD) {
-          hf[hfi(1, 0, 16 * h + k)] = hr[k];
-          hf[hfi(1, 1, 16 * h + k)] = hi[k];
-        }
-      }
-      st8_split(sm + S_H3, 16 * h, sm + S_LO, 16 * h, row, hr);
-      st8_split(sm + S_H3, 8 + 16 * h, sm + S_LO, 8 + 16 * h, row, hr + 8);
-      st8_split(sm + S_H3, 32 + 16 * h, sm + S_LO, 32 + 16 * h, row, hi);
-      st8_split(sm + S_H3, 40 + 16 * h, sm + S_LO, 40 + 16 * h, row, hi + 8);
-    }
-    // -- output layer ----------------------------------------------------------
-    step([&] {
-      gemm_act_w(tm + T_DO, sbase + S_H3, sbase + S_WO, 16, 16, 64, false);
-      gemm_act_w(tm + T_DO, sbase + S_LO, sbase + S_WO, 16, 16, 64, true);
-    });
-    if (abort) break;
+  auto store_y = [&](int tile) {
     if (hh == 0) {  // warp-uniform
-      float d[16];
-      tc::ld16(tm + lo + T_DO, d);
-      if (a.y && valid) a.y[c] = make_float2(d[0] + par[P_BOR], d[1] + par[P_BOI]);
+      float d[8];
+      tc::ld8(lz + T_OUT, d);
+      const int c = tile * 128 + row;
+      if (c < a.N) a.y[c] = make_float2(d[0] + par[P_BOR], d[1] + par[P_BOI]);
     }
-    if constexpr (BWD) {
-      // G_h3 = Wo_r^T G_y ; output-layer gradient accumulation
+  };
+
+  // The CTA's tiles are blockIdx + i gridDim; its slots take i from a shared
+  // counter (the scheduler favours some warps, and equal shares left the SM with
+  // 3 tiles in flight on average)
+  const int ntiles = (a.N + 127) / 128;
+  auto tile_of = [&](int i) { return int(blockIdx.x) + i * int(gridDim.x); };
+  int tile = tile_of(slot), last = -1;
+  u64 xa[4], xb[4];
+  if (tile < ntiles) {
+    load_x(a, tile * 128 + row, hh, xa, xb);
+    st8(sl + F_X, row, 16 * hh, xa);
+    st8(sl + F_X, row, 16 * hh + 8, xb);
+  }
+  while (tile < ntiles) {
+    if (st == 0) *next = tile_of(atomicAdd(counter, 1));  // published by the next two barriers
+    step([&] {
+      gemm_act_w(tz, sb + F_X, wb + S_W1, 32, 32, 32, false);
+      if (last >= 0) output();  // of the tile before, whose h3 is in place
+    });
+    if (abort) break;
+    if (last >= 0) store_y(last);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int u = 16 * hh + 8 * q;
+      u64 z[4], hr[4], hi[4];
+      ld8_bias(lz + u, par + P_B1 + u, z);
+      h_layer1(z, w1, hr, hi);
+      st8_split(sl + F_HI, u, sl + F_LO, u, row, hr);
+      st8_split(sl + F_HI, 32 + u, sl + F_LO, 32 + u, row, hi);
+    }
+    step([&] {
+      gemm_act_w(tz, sb + F_HI, wb + S_W2, 64, 64, 64, false);
+      gemm_act_w(tz, sb + F_LO, wb + S_W2, 64, 64, 64, true);
+    });
+    if (abort) break;
+    last = tile;
+    tile = *next;
+    prefetch_x(a, tile, ntiles, st);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int u = 16 * hh + 8 * q;
+      u64 r[4], i[4], hr[4], hi[4];
+      ld8x2(lz + u, r, lz + 32 + u, i);
+      bias8(r, par + P_B2R + u);
+      bias8(i, par + P_B2I + u);
+      h_complex(r, i, w2, hr, hi);
+      st8_split(sl + F_HI, u, sl + F_LO, u, row, hr);
+      st8_split(sl + F_HI, 32 + u, sl + F_LO, 32 + u, row, hi);
+    }
+    if (tile < ntiles) load_x(a, tile * 128 + row, hh, xa, xb);  // lands while z3 is formed
+    step([&] {
+      gemm_act_w(tz, sb + F_HI, wb + S_W3, 64, 64, 64, false);
+      gemm_act_w(tz, sb + F_LO, wb + S_W3, 64, 64, 64, true);
+    });
+    if (abort) break;
+    if (tile < ntiles) {
+      st8(sl + F_X, row, 16 * hh, xa);
+      st8(sl + F_X, row, 16 * hh + 8, xb);
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int u = 16 * hh + 8 * q;
+      u64 r[4], i[4], hr[4], hi[4];
+      ld8x2(lz + u, r, lz + 32 + u, i);
+      bias8(r, par + P_B3R + u);
+      bias8(i, par + P_B3I + u);
+      h_complex(r, i, w3, hr, hi);
+      st8_split(sl + F_HI, u, sl + F_LO, u, row, hr);
+      st8_split(sl + F_HI, 32 + u, sl + F_LO, 32 + u, row, hi);
+    }
+  }
+  if (!abort && last >= 0) {
+    step(output);
+    if (!abort) store_y(last);
+  }
+  if (abort || bad) mbar_wait_bounded(bar, phase ^ 1u);  // let the slot's last MMAs drain
+  tc::fence_before();
+  if (__syncthreads_or(bad) && t == 0) pty_raise(a.status, PTYCHO_ERR_TIMEOUT);
+  if (t < 32) tc::tmem_free(tm, kColsFwd);
+}
+
+// ---- backward --------------------------------------------------------------------
+constexpr int kSlots = 2;                                 // tiles in flight per CTA
+constexpr int kBwdThreads = kSlots * kTileThreads;
+// per tile: every MMA reads 16-group A footprints (unused accumulator rows take
+// whatever follows an operand), all inside the tile's own buffers
+constexpr int B_GZ1 = 0;               // G_z1: 4 groups
+constexpr int B_GY = B_GZ1 + 4 * GRP;  // (G_yr, G_yi, 0 ...): 2 groups, rows 32, 33 of the G_z1 accumulator
+constexpr int B_GZ = B_GY + 2 * GRP;   // G_z3 (8), G_z2 (8)
+constexpr int B_LO = B_GZ;             // h - bf16(h) of layers 1, 2: dead before G_z3 is written
+constexpr int B_H3 = B_GZ + 8 * GRP;   // bf16(h3): its MMA completes before G_z2 is written
+constexpr int B_H = B_GZ + 16 * GRP;   // bf16(h2) (8), bf16(h1) (8), ones (1)
+constexpr int B_X = B_H + 17 * GRP;    // x (4), ones (1): two buffers, tiles alternate
+constexpr int kXBytes = 5 * GRP;
+constexpr int kSlotBytes = B_X + 2 * kXBytes + GRP;  // and a group of padding
+static_assert(B_GZ1 + 16 * GRP <= kSlotBytes && B_H + 18 * GRP <= kSlotBytes, "MMA footprints");
+constexpr int B_W = kSlots * kSlotBytes;
+constexpr int B_PAR = B_W + kWBytes;
+constexpr int B_Y = B_PAR + kParSmem * 4;            // output partials: [slot][128] float2
+constexpr int B_RED = B_Y + kSlots * 128 * 8;        // 3 sums of 16 warps
+constexpr int B_BAR = B_RED + 3 * 16 * 4;            // per slot: chain, both accumulations done
+constexpr int B_TMEM = B_BAR + kSlots * 3 * 8;
+constexpr int B_SMEM = int(pty_align_up_c(B_TMEM + 8, 128));
+static_assert(B_PAR % 16 == 0 && B_Y % 8 == 0 && B_BAR % 8 == 0 && B_SMEM <= 232448, "shared-memory budget");
+// TMEM columns: the accumulators, then per slot z1 / z3 / G_h2 / G_h1 (64) and z2 / G_h3 / G_x (64)
+constexpr uint32_t T_ACC = 0, T_ACC1 = 144, T_ACCO = 192, T_SLOT = 256, kColsBwd = 512;
+
+__global__ void __launch_bounds__(kBwdThreads, 1) k_cmlp_bwd(const Args a) {
+  extern __shared__ __align__(1024) unsigned char sm[];
+  const int t = threadIdx.x, w = t >> 5;
+  const int slot = t / kTileThreads;
+  const int st = t % kTileThreads;
+  const Place pl = place(st);
+  const int row = pl.row, hh = pl.hh;
+  unsigned char* sl = sm + slot * kSlotBytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + B_BAR);
+  uint64_t *chain = bars, *done_o = bars + kSlots, *done_a = bars + 2 * kSlots;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + B_TMEM);
+  float* par = reinterpret_cast<float*>(sm + B_PAR);
+  float* red = reinterpret_cast<float*>(sm + B_RED);
+  const uint32_t sbase = tc::smem_addr(sm);
+
+  load_packed(a, sm + B_W, par, t, kBwdThreads);
+  if (hh == 1) {  // the second feature group of G_y stays zero
+    const u64 zero[4] = {0, 0, 0, 0};
+    st8(sl + B_GY, row, 8, zero);
+  } else {  // ones columns; the other features of those groups are not used
+    const __nv_bfloat16 one = __float2bfloat16(1.0f);
+    *reinterpret_cast<__nv_bfloat16*>(sl + B_H + cm_off(row, 128)) = one;
+    *reinterpret_cast<__nv_bfloat16*>(sl + B_X + cm_off(row, 32)) = one;
+    *reinterpret_cast<__nv_bfloat16*>(sl + B_X + kXBytes + cm_off(row, 32)) = one;
+  }
+  if (t == 0) {
+    for (int i = 0; i < 3 * kSlots; ++i) mbar_init(bars + i, 1);
+    fence_mbar_init();
+  }
+  if (w == 0) {
+    tc::tmem_alloc(tslot, kColsBwd);
+    tc::tmem_relinquish();
+  }
+  tc::fence_smem_async();
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  const uint32_t tm = *tslot;
+  const int ntiles = (a.N + 127) / 128;
+  // the CTA's tiles in order: q = 0 .. nq-1 is tile q gridDim + blockIdx, on slot q % kSlots
+  const int nq = (ntiles - int(blockIdx.x) + int(gridDim.x) - 1) / int(gridDim.x);
+  bool bad = false;
+  u64 om1 = 0, om2 = 0, om3 = 0;  // pairs of partial sums
+
+  {
+    const float w1 = par[P_W1], w2 = par[P_W2], w3 = par[P_W3];
+    const uint32_t ta = tm + T_SLOT + 128 * slot, tb = ta + 64;  // the slot's columns
+    const uint32_t la = ta + pl.lanes, lb = tb + pl.lanes;
+    const uint32_t sb = sbase + slot * kSlotBytes, wb = sbase + B_W;
+    float2* ybuf = reinterpret_cast<float2*>(sm + B_Y) + slot * 128;
+    uint32_t phase = 0;
+    bool abort = false;
+    // operands written -> the slot's first thread issues `issue` and, behind it,
+    // `accumulate` -> its threads wait for the result of `issue`
+    auto step = [&](auto issue, auto accumulate) {
+      tc::fence_smem_async();
+      tc::fence_before();
+      abort = slot_barrier_or(slot, bad);
+      if (abort) return;
+      tc::fence_after();
+      if (st == 0) {
+        issue();
+        tc::commit(chain + slot);
+        accumulate();
+      }
+      bad = bad || !mbar_wait_bounded(chain + slot, phase);
+      phase ^= 1u;
+      tc::fence_after();
+    };
+    auto nothing = [] {};
+    // the two slots add into the same columns: tile q after tile q - 1 has been added
+    auto after_previous = [&](uint64_t* done, int q) {
+      if (q > 0) bad = bad || !mbar_wait_bounded(done + (q - 1) % kSlots, ((q - 1) / kSlots) & 1);
+      tc::fence_after();
+    };
+    u64 xa[4], xb[4];
+    float2 gn = make_float2(0.f, 0.f);
+    auto load_in = [&](int tile) {
+      const int c = tile * 128 + row;
+      load_x(a, c, hh, xa, xb);
+      gn = c < a.N ? __ldg(a.gy + c) : make_float2(0.f, 0.f);
+    };
+    if (slot < nq) load_in(slot * gridDim.x + blockIdx.x);
+    for (int q = slot; q < nq; q += kSlots) {
+      const int tile = q * gridDim.x + blockIdx.x;
+      const int c = tile * 128 + row;
+      const bool valid = c < a.N;
+      const uint32_t par_q = (q / kSlots) & 1;
+      // -- inputs ------------------------------------------------------------------------
+      const int bx = B_X + int(par_q) * kXBytes;
+      st8(sl + bx, row, 16 * hh, xa);
+      st8(sl + bx, row, 16 * hh + 8, xb);
+      prefetch_x(a, tile + kSlots * gridDim.x, ntiles, st);
+      step([&] { gemm_act_w(ta, sb + bx, wb + S_W1, 32, 32, 32, false); }, nothing);
+      if (abort) break;
+      // the tile before: its accumulation has read every buffer written from here on
+      if (q >= kSlots) bad = bad || !mbar_wait_bounded(done_a + slot, par_q ^ 1u);
+      if (hh == 0) {
+        const u64 v[4] = {pk(gn.x, gn.y), 0, 0, 0};
+        st8(sl + B_GY, row, 0, v);
+      }
+      // -- layer 1 (zz = z1 + b1 is kept for its gradient) -------------------------------
+      u64 zz[2][4];
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        const int u = 16 * hh + 8 * p;
+        u64 hr[4], hi[4];
+        ld8_bias(la + u, par + P_B1 + u, zz[p]);
+        h_layer1(zz[p], w1, hr, hi);
+        st8_split(sl + B_H, 64 + u, sl + B_LO, u, row, hr);
+        st8_split(sl + B_H, 96 + u, sl + B_LO, 32 + u, row, hi);
+      }
       step([&] {
-        gemm_act_wT(tm + T_DO, sbase + S_GY, sbase + S_WO, 16, 64, 16);
-        gemm_outer(tm + T_ACCO, sbase + S_GY, sbase + S_H3, 80, !first);
-      });
+        gemm_act_w(tb, sb + B_H + 8 * GRP, wb + S_W2, 64, 64, 64, false);
+        gemm_act_w(tb, sb + B_LO, wb + S_W2, 64, 64, 64, true);
+      }, nothing);
       if (abort) break;
-      // G_z3 = conj(i w3 h3) G_h3 (h3 recomputed from z3 in TMEM)
-      {
-        const int h = hh;
-        float gr[16], gi[16], zr[16], zi[16];
-        tc::ld16(tm + lo + T_DO + 16 * h, gr);
-        tc::ld16(tm + lo + T_DO + 32 + 16 * h, gi);
-        tc::ld16(tm + lo + T_D3 + 16 * h, zr);
-        tc::ld16(tm + lo + T_D3 + 32 + 16 * h, zi);
+      // -- layer 2 (z2 + b2 is kept for its gradient) -------------------------------------
+      u64 z2r[2][4], z2i[2][4];
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
-          const float r = zr[k] + par[P_B3R + 16 * h + k], i = zi[k] + par[P_B3I + 16 * h + k];
-          const float hr = hf[hfi(1, 0, 16 * h + k)], hi = hf[hfi(1, 1, 16 * h + k)];  // h3 of this tile
-          om3 += gi[k] * (r * hr - i * hi) - gr[k] * (r * hi + i * hr);
-          zr[k] = w3 * (hr * gi[k] - hi * gr[k]);
-          zi[k] = -w3 * (hr * gr[k] + hi * gi[k]);
-        }
-        st8(sm + S_GZ, row, 16 * h, zr);
-        st8(sm + S_GZ, row, 8 + 16 * h, zr + 8);
-        st8(sm + S_GZ, row, 32 + 16 * h, zi);
-        st8(sm + S_GZ, row, 40 + 16 * h, zi + 8);
+      for (int p = 0; p < 2; ++p) {
+        const int u = 16 * hh + 8 * p;
+        u64 hr[4], hi[4];
+        ld8x2(lb + u, z2r[p], lb + 32 + u, z2i[p]);
+        bias8(z2r[p], par + P_B2R + u);
+        bias8(z2i[p], par + P_B2I + u);
+        h_complex(z2r[p], z2i[p], w2, hr, hi);
+        st8_split(sl + B_H, u, sl + B_LO, u, row, hr);
+        st8_split(sl + B_H, 32 + u, sl + B_LO, 32 + u, row, hi);
       }
-      step([&] { gemm_act_wT(tm + T_D3, sbase + S_GZ, sbase + S_W3, 64, 64, 64); });
+      step([&] {  // z3, and G_h3 = Wo_r^T G_y
+        gemm_act_w(ta, sb + B_H, wb + S_W3, 64, 64, 64, false);
+        gemm_act_w(ta, sb + B_LO, wb + S_W3, 64, 64, 64, true);
+        gemm_act_wT(tb, sb + B_GY, wb + S_WO, 16, 64, 16);
+      }, nothing);
       if (abort) break;
-      // G_z2
-      {
-        const int h = hh;
-        float gr[16], gi[16], zr[16], zi[16];
-        tc::ld16(tm + lo + T_D3 + 16 * h, gr);
-        tc::ld16(tm + lo + T_D3 + 32 + 16 * h, gi);
-        tc::ld16(tm + lo + T_D2 + 16 * h, zr);
-        tc::ld16(tm + lo + T_D2 + 32 + 16 * h, zi);
+      // -- layer 3, the output, and G_z3 = conj(i w3 h3) G_h3 ------------------------------
+      float2 yp = make_float2(0.f, 0.f);
+#pragma unroll 1
+      for (int p = 0; p < 2; ++p) {
+        const int u = 16 * hh + 8 * p;
+        u64 r[4], i[4], hr[4], hi[4], gr[4], gi[4];
+        ld8x2(la + u, r, la + 32 + u, i);
+        bias8(r, par + P_B3R + u);
+        bias8(i, par + P_B3I + u);
+        h_complex(r, i, w3, hr, hi);
+        ld8x2(lb + u, gr, lb + 32 + u, gi);
+        st8(sl + B_H3, row, u, hr);
+        st8(sl + B_H3, row, 32 + u, hi);
+        if (a.y) {
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
-          const float r = zr[k] + par[P_B2R + 16 * h + k], i = zi[k] + par[P_B2I + 16 * h + k];
-          const float hr = hf[hfi(0, 0, 16 * h + k)], hi = hf[hfi(0, 1, 16 * h + k)];  // h2 of this tile
-          om2 += gi[k] * (r * hr - i * hi) - gr[k] * (r * hi + i * hr);
-          zr[k] = w2 * (hr * gi[k] - hi * gr[k]);
-          zi[k] = -w2 * (hr * gr[k] + hi * gi[k]);
+          for (int j = 0; j < 4; ++j) {
+            float h0, h1, k0, k1;
+            upk(hr[j], h0, h1);
+            upk(hi[j], k0, k1);
+            const float* wr = par + P_WOR + u + 2 * j;
+            const float* wi = par + P_WOI + u + 2 * j;
+            yp.x = fmaf(wr[0], h0, fmaf(-wi[0], k0, fmaf(wr[1], h1, fmaf(-wi[1], k1, yp.x))));
+            yp.y = fmaf(wr[0], k0, fmaf(wi[0], h0, fmaf(wr[1], k1, fmaf(wi[1], h1, yp.y))));
+          }
         }
-        st8(sm + S_GZ, row, 64 + 16 * h, zr);
-        st8(sm + S_GZ, row, 72 + 16 * h, zr + 8);
-        st8(sm + S_GZ, row, 96 + 16 * h, zi);
-        st8(sm + S_GZ, row, 104 + 16 * h, zi + 8);
+        grad_z(r, i, hr, hi, gr, gi, w3, om3);
+        st8(sl + B_GZ, row, u, r);
+        st8(sl + B_GZ, row, 32 + u, i);
       }
-      step([&] { gemm_act_wT(tm + T_D2, sbase + S_GZ + 8 * GRP, sbase + S_W2, 64, 64, 64); });
+      if (a.y && hh == 1) ybuf[row] = yp;
+      step([&] { gemm_act_wT(ta, sb + B_GZ, wb + S_W3, 64, 64, 64); },
+           [&] {
+             after_previous(done_o, q);
+             gemm_outer(tm + T_ACCO, sb + B_GY, sb + B_H3, 64, q > 0);
+             tc::commit(done_o + slot);
+           });
       if (abort) break;
-      // G_z1 = Re(conj(G_h1) i w1 h1)
-      {
-        const int h = hh;
-        float gr[16], gi[16], z[16];
-        tc::ld16(tm + lo + T_D2 + 16 * h, gr);
-        tc::ld16(tm + lo + T_D2 + 32 + 16 * h, gi);
-        tc::ld16(tm + lo + T_D1 + 16 * h, z);
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-          const float zz = z[k] + par[P_B1 + 16 * h + k];
-          float s, co;
-          sincos_rr(w1 * zz, &s, &co);
-          const float q = co * gi[k] - s * gr[k];
-          om1 += zz * q;
-          z[k] = w1 * q;
-        }
-        st8(sm + S_GZ1, row, 16 * h, z);
-        st8(sm + S_GZ1, row, 8 + 16 * h, z + 8);
+      if (a.y && hh == 0 && valid) {
+        const float2 o = ybuf[row];
+        a.y[c] = make_float2(yp.x + o.x + par[P_BOR], yp.y + o.y + par[P_BOI]);
       }
-      // G_x = W1^T G_z1 ; hidden / layer-1 weight-gradient accumulation
-      step([&] {
-        gemm_act_wT(tm + T_D1, sbase + S_GZ1, sbase + S_W1, 32, 32, 32);
-        gemm_outer(tm + T_ACC, sbase + S_GZ, sbase + S_H, 144, !first);
-        gemm_outer(tm + T_ACC1, sbase + S_GZ1, sbase + S_X, 48, !first);
-      });
+      // -- G_z2 = conj(i w2 h2) G_h2 (written over h3: wait for its accumulation) ---------------
+      bad = bad || !mbar_wait_bounded(done_o + slot, par_q);
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        const int u = 16 * hh + 8 * p;
+        u64 gr[4], gi[4], hr[4], hi[4];
+        ld8x2(la + u, gr, la + 32 + u, gi);
+        h_complex(z2r[p], z2i[p], w2, hr, hi);  // again: 32 registers less than keeping it
+        grad_z(z2r[p], z2i[p], hr, hi, gr, gi, w2, om2);
+        st8(sl + B_GZ, row, 64 + u, z2r[p]);
+        st8(sl + B_GZ, row, 96 + u, z2i[p]);
+      }
+      step([&] { gemm_act_wT(ta, sb + B_GZ + 8 * GRP, wb + S_W2, 64, 64, 64); }, nothing);
+      if (abort) break;
+      // -- G_z1 = Re(conj(G_h1) i w1 h1) ----------------------------------------------------
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        const int u = 16 * hh + 8 * p;
+        u64 gr[4], gi[4];
+        ld8x2(la + u, gr, la + 32 + u, gi);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          u64 sn, co;
+          sincos_rr(mul2(zz[p][j], pk(w1)), &sn, &co);
+          const u64 v = fma2(co, gi[j], mul2(mul2(sn, pk(-1.f)), gr[j]));
+          om1 = fma2(zz[p][j], v, om1);
+          gr[j] = mul2(v, pk(w1));
+        }
+        st8(sl + B_GZ1, row, u, gr);
+      }
+      if (q + kSlots < nq) load_in(tile + kSlots * gridDim.x);  // lands while G_x is formed
+      step([&] { gemm_act_wT(tb, sb + B_GZ1, wb + S_W1, 32, 32, 32); },
+           [&] {
+             after_previous(done_a, q);
+             gemm_outer(tm + T_ACC, sb + B_GZ, sb + B_H, 144, q > 0);
+             gemm_outer(tm + T_ACC1, sb + B_GZ1, sb + bx, 48, q > 0);
+             tc::commit(done_a + slot);
+           });
       if (abort) break;
       if (a.gx) {
-        {
-          const int h = hh;
-          float d[16];
-          tc::ld16(tm + lo + T_D1 + 16 * h, d);
-          if (valid) {
-            if (a.gx_planar) {  // per feature, a warp stores 32 consecutive rows
+        float d[16];
+        tc::ld16(lb + 16 * hh, d);
+        if (valid) {
+          if (a.gx_planar) {  // per feature, a warp stores 32 consecutive rows
 #pragma unroll
-              for (int i = 0; i < 16; ++i) a.gx[size_t(16 * h + i) * a.N + c] = d[i];
-            } else {
-              float4* gp = reinterpret_cast<float4*>(a.gx + size_t(c) * 32 + 16 * h);
+            for (int i = 0; i < 16; ++i) a.gx[size_t(16 * hh + i) * a.N + c] = d[i];
+          } else {
+            float4* gp = reinterpret_cast<float4*>(a.gx + size_t(c) * 32 + 16 * hh);
 #pragma unroll
-              for (int q = 0; q < 4; ++q) gp[q] = make_float4(d[4 * q], d[4 * q + 1], d[4 * q + 2], d[4 * q + 3]);
-            }
+            for (int i = 0; i < 4; ++i) gp[i] = make_float4(d[4 * i], d[4 * i + 1], d[4 * i + 2], d[4 * i + 3]);
           }
         }
       }
-      first = false;
+      // the last tile's accumulation is read below
+      if (q + kSlots >= nq) bad = bad || !mbar_wait_bounded(done_a + slot, par_q);
     }
+    if (abort || bad) mbar_wait_bounded(chain + slot, phase ^ 1u);  // let the slot's last MMAs drain
   }
 
-  if (abort) {  // bounded wait gave up: report, let the tensor core drain, free TMEM
-    if (t == 0) pty_raise(a.status, PTYCHO_ERR_TIMEOUT);
-    mbar_wait_bounded(bar, phase);
-  }
-  if constexpr (BWD) {
-    if (!abort) {
-      // -- raw accumulators -> this CTA's partial --------------------------------
-      float* P = a.part + size_t(blockIdx.x) * kPartFloats;
-      auto rd = [&](uint32_t col, float (&d)[16]) {
-        if (first) {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) d[i] = 0.f;
-        } else {
-          tc::ld16(tm + lo + col, d);
-        }
-      };
+  tc::fence_before();
+  const bool abort = __syncthreads_or(bad);
+  tc::fence_after();
+  if (abort && t == 0) pty_raise(a.status, PTYCHO_ERR_TIMEOUT);
+  if (!abort) {
+    // -- raw accumulators -> this CTA's partial: warp w reads lane quarter w & 3,
+    //    16-column chunk w >> 2 of each accumulator -------------------------------------
+    float* P = a.part + size_t(blockIdx.x) * kPartFloats;
+    {
+      const int chunk = w >> 2;
+      const uint32_t lo = tm + pl.lanes;
       float d[16];
-      if (hh == 1) {
-        // the raw accumulators are read by warps 0..3 (one per lane quarter)
-      } else if (quarter < 2) {  // rows 0..63: W3 real form and b3
+      const bool top = row < 64;  // rows 0..63: W3 real form and b3; rows 64..127: W2 real form and b2
+      tc::ld16(lo + T_ACC + (top ? 0 : 64) + 16 * chunk, d);
+      float* pw = P + (top ? R_W3 + row * 64 : R_W2 + (row - 64) * 64) + 16 * chunk;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          rd(T_ACC + 16 * q, d);
-#pragma unroll
-          for (int i = 0; i < 16; ++i) P[R_W3 + row * 64 + 16 * q + i] = d[i];
-        }
-        rd(T_ACC + 128, d);
-        P[R_B3 + row] = d[0];
-      } else {  // rows 64..127: W2 real form and b2
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          rd(T_ACC + 64 + 16 * q, d);
-#pragma unroll
-          for (int i = 0; i < 16; ++i) P[R_W2 + (row - 64) * 64 + 16 * q + i] = d[i];
-        }
-        rd(T_ACC + 128, d);
-        P[R_B2 + row - 64] = d[0];
+      for (int i = 0; i < 16; ++i) pw[i] = d[i];
+      if (chunk == 0) {
+        tc::ld16(lo + T_ACC + 128, d);
+        P[top ? R_B3 + row : R_B2 + row - 64] = d[0];
       }
-      if (w == 0) {  // rows 0..31: W1, b1 ; rows 0,1: Wo real form, bo
+      if ((w & 3) == 0) {  // rows 0..31: W1, b1 ; rows 0,1: Wo real form
+        if (chunk < 2) {
+          tc::ld16(lo + T_ACC1 + 16 * chunk, d);
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          rd(T_ACC1 + 16 * q, d);
-#pragma unroll
-          for (int i = 0; i < 16; ++i) P[R_W1 + row * 32 + 16 * q + i] = d[i];
+          for (int i = 0; i < 16; ++i) P[R_W1 + row * 32 + 16 * chunk + i] = d[i];
         }
-        rd(T_ACC1 + 32, d);
-        P[R_B1 + row] = d[0];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          rd(T_ACCO + 16 * q, d);
-          if (row < 2) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) P[R_WO + row * 64 + 16 * q + i] = d[i];
-          }
+        if (chunk == 2) {
+          tc::ld16(lo + T_ACC1 + 32, d);
+          P[R_B1 + row] = d[0];
         }
-        rd(T_ACCO + 64, d);
-        if (row < 2) P[R_BO + row] = d[0];
+        tc::ld16(lo + T_ACCO + 16 * chunk, d);
+        if (row < 2) {
+#pragma unroll
+          for (int i = 0; i < 16; ++i) P[R_WO + row * 64 + 16 * chunk + i] = d[i];
+        }
+      }
+      if (w == 1) {  // rows 32, 33 of the G_z1 accumulator: G_y against the ones column
+        tc::ld16(lo + T_ACC1 + 32, d);
+        if (row < 34) P[R_BO + row - 32] = d[0];
       }
       // omega gradients: fixed shuffle tree, then warps in order
+      const u64 om[3] = {om1, om2, om3};
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        om1 += __shfl_xor_sync(0xffffffffu, om1, o);
-        om2 += __shfl_xor_sync(0xffffffffu, om2, o);
-        om3 += __shfl_xor_sync(0xffffffffu, om3, o);
-      }
-      if ((t & 31) == 0) {
-        red[w] = om1;
-        red[8 + w] = om2;
-        red[16 + w] = om3;
-      }
-      __syncthreads();
-      if (t == 0) {
+      for (int l = 0; l < 3; ++l) {
+        float x, y;
+        upk(om[l], x, y);
+        x += y;
 #pragma unroll
-        for (int l = 0; l < 3; ++l) {
-          float s = 0.f;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) s += red[8 * l + i];  // warps in order
-          P[R_OM + l] = s;
-        }
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if ((t & 31) == 0) red[16 * l + w] = x;
       }
+    }
+    __syncthreads();
+    if (t < 3) {
+      float s = 0.f;
+#pragma unroll
+      for (int i = 0; i < 16; ++i) s += red[16 * t + i];  // warps in order
+      P[R_OM + t] = s;
     }
   }
   tc::fence_before();
   __syncthreads();
-  if (w == 0) tc::tmem_free(tm, NCOLS);
+  if (w == 0) tc::tmem_free(tm, kColsBwd);
 }
 
 // sum the CTA partials in a fixed order and fold the real-form blocks
@@ -709,21 +960,18 @@ __global__ void __launch_bounds__(256) k_cmlp_pack(const PackArgs p) {
   }
 }
 
-template <bool BWD>
-static int launch(const Args& a, cudaStream_t s, int* grid_out) {
-  auto kern = k_cmlp<BWD>;
-  constexpr int smem = BWD ? kSmemBwd : kSmemFwd;
+template <typename K>
+static int launch(K kern, int threads, int smem, const Args& a, cudaStream_t s, int* grid_out) {
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return PTYCHO_ERR_LAUNCH;
   int dev = 0, nsm = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const int ntiles = (a.N + 127) / 128;
-  const int per_sm = BWD ? 1 : 2;  // TMEM: 512 columns (backward) or 2 x 256 (forward) per SM
-  const int grid = ntiles < nsm * per_sm ? ntiles : nsm * per_sm;
+  const int grid = ntiles < nsm ? ntiles : nsm;  // one CTA per SM: each allocates all of TMEM
   if (grid_out) *grid_out = grid;
   if (grid == 0) return PTYCHO_OK;
-  kern<<<grid, kThreads, smem, s>>>(a);
+  kern<<<grid, threads, smem, s>>>(a);
   return cudaGetLastError() == cudaSuccess ? PTYCHO_OK : PTYCHO_ERR_LAUNCH;
 }
 
@@ -757,7 +1005,8 @@ static int cmlp_forward(int planar, const void* packed, const float* x, int N, f
     return PTYCHO_ERR_MISALIGNED;
   cm::Args a{static_cast<const unsigned char*>(packed), x, nullptr, N, reinterpret_cast<float2*>(y), nullptr,
              nullptr, status_out, 0, planar};
-  return cm::launch<false>(a, reinterpret_cast<cudaStream_t>(stream), nullptr);
+  return cm::launch(cm::k_cmlp_fwd, cm::kFwdSlots * cm::kTileThreads, cm::F_SMEM, a,
+                    reinterpret_cast<cudaStream_t>(stream), nullptr);
 }
 
 int ptycho_cmlp_forward(const void* packed, const float* x, int N, float* y, int32_t* status_out,
@@ -801,7 +1050,7 @@ static int cmlp_backward(int planar, const void* packed, const float* x, const f
   cm::Args a{static_cast<const unsigned char*>(packed), x, reinterpret_cast<const float2*>(gy), N,
              reinterpret_cast<float2*>(y), gx, static_cast<float*>(workspace), status_out, planar, planar};
   int grid = 0;
-  int st = cm::launch<true>(a, s, &grid);
+  int st = cm::launch(cm::k_cmlp_bwd, cm::kBwdThreads, cm::B_SMEM, a, s, &grid);
   if (st) return st;
   cm::k_cmlp_reduce<<<(cm::kGradFloats + 31) / 32, 256, 0, s>>>(static_cast<const float*>(workspace), grid,
                                                                   grad);
