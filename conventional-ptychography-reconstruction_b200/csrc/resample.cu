@@ -14,8 +14,9 @@
 //   row pass    -- lines are rows (contiguous), written as rows;
 //   column pass -- lines are LINES adjacent columns (32-byte or wider
 //                  segments per row), written the same way.
-// Upsampling: row pass x -> t [h][w s], column pass t -> y.  Adjoint: row pass
-// g -> t [h s][w], column pass t -> x-gradient.
+// Upsampling: column pass x -> t [h s][w], row pass t -> y.  Adjoint: row pass
+// g -> t [h s][w], column pass t -> x-gradient.  Both column passes move the
+// narrow side, in pieces of a few columns; the wide side moves as whole rows.
 //
 // Each CTA loads LINES lines into two shared-memory planes (re, im; one float
 // of padding every 32), runs radix-8 or radix-16 Stockham passes (8- or
@@ -222,33 +223,253 @@ int launch(const float2* in, float2* out, int nlines, long long ld_in, long long
   return cudaGetLastError() == cudaSuccess ? PTYCHO_OK : PTYCHO_ERR_LAUNCH;
 }
 
-// dispatch over line lengths 2^6 .. 2^12 with L2 / L1 in {1/4, 1/2, 1, 2, 4}
+// short power-of-two lines: 64 and 128 points, s = 2 or 4
 template <bool COL>
 int dispatch(int l1, int l2, const float2* in, float2* out, int nlines, long long ld_in, long long ld_out,
              cudaStream_t s) {
-#define PTY_RS(A, B) \
-  if (l1 == A && l2 == B) return launch<A, B, COL>(in, out, nlines, ld_in, ld_out, s);
-#define PTY_RS_ROW(A) PTY_RS(A, A) PTY_RS(A, 2 * A) PTY_RS(2 * A, A) PTY_RS(A, 4 * A) PTY_RS(4 * A, A)
-  PTY_RS_ROW(64)
-  PTY_RS_ROW(128)
-  PTY_RS_ROW(256)
-  PTY_RS_ROW(512)
-  PTY_RS_ROW(1024)
-  PTY_RS(2048, 2048) PTY_RS(2048, 4096) PTY_RS(4096, 2048)
-  PTY_RS(4096, 4096)
-#undef PTY_RS_ROW
+#define PTY_RS(A, B)                                                                                \
+  if (l1 == A && l2 == B) return launch<A, B, COL>(in, out, nlines, ld_in, ld_out, s);               \
+  if (l1 == B && l2 == A) return launch<B, A, COL>(in, out, nlines, ld_in, ld_out, s);
+  PTY_RS(64, 128) PTY_RS(64, 256) PTY_RS(128, 256) PTY_RS(128, 512)
 #undef PTY_RS
   return PTYCHO_ERR_UNSUPPORTED_SIZE;
 }
 
 bool supported(int n, int N) {
-  auto pow2 = [](int v) { return v >= 64 && v <= 4096 && (v & (v - 1)) == 0; };
-  if (!pow2(n) || !pow2(N)) return false;
-  const int r = n > N ? n / N : N / n;
-  return r == 1 || r == 2 || r == 4;
+  const int lo = n < N ? n : N, r = n < N ? N / n : n / N;
+  return (lo == 64 || lo == 128) && lo * r == (n < N ? N : n) && (r == 2 || r == 4);
 }
 
 }  // namespace rs
+
+namespace sh {
+
+// ---------------------------------------------------------------------------
+// Power-of-two lines of 256 to 2048 points, upsampled by s = 2 or 4.
+//
+// Interleaving the s phases of the long line, y[s m + p] is the inverse length-n
+// transform of X_k exp(2 pi i k p / N): phase 0 is x itself, and every other
+// phase is one forward and one inverse length-n transform with a diagonal
+// between -- for s = 2 a third of the arithmetic and half the shared memory of
+// padding the spectrum to length N, and a quarter of the samples are copies.  The
+// adjoint is the same with the conjugate diagonal, summed over the phases.
+//
+// n = 16 * 16 * C: a line is held by n / 16 threads, 16 values each.  Forward,
+// decimation in frequency: thread q has x[q + 16 C e]; DFT16 over e -> digit a,
+// twiddle W_n^(q a); exchange; thread (a, q0) has q = q0 + C e; DFT16 -> digit b,
+// twiddle W_16C^(q0 b); exchange; DFT_C -> digit c, frequency a + 16 b + 256 c.
+// The diagonal is applied in that order and the inverse walks back, so nothing is
+// reordered: four exchanges in all (the padded form moved the line through
+// shared memory seven times).  The diagonal of frequency a + 16 b + 256 c is a
+// product of three factors: that of c is applied where c is in registers, those of
+// a and b are part of the inverse's twiddles.  An exchange writes value (a, q) at a P + q or
+// (a, q0, b) at a P + 17 q0 + b, P = 17 C: conflict free both ways for 8-byte
+// accesses of a half-warp (P = C, 17 = 1 mod 16).
+// Measured on B200, 2048^2 to 4096^2 and back: 286 us for the four passes (49 + 77
+// up, 93 + 64 down) against 668 us by padded spectra; bound by latency (issue 35 to
+// 40 %, four to seven barriers between loads and stores), 336 MB would take 51 us.
+// Columns: COLS adjacent columns per CTA, interleaved in shared memory the same
+// way, so global accesses are pieces of 8 COLS bytes.
+// ---------------------------------------------------------------------------
+template <int N, bool COL>
+struct Cfg {
+  static constexpr int C = N / 256;           // last radix
+  static constexpr int T = N / 16;            // threads per line
+  static constexpr int COLS = COL ? (512 / T) : 1;
+  static constexpr int LINES = 512 / T;       // lines per CTA
+  static constexpr int NT = 512;
+  static constexpr int P = 17 * C;
+  static constexpr int PLANE = 16 * P;        // float2 per line
+  static constexpr size_t SMEM = size_t(LINES * PLANE + 2 * N + 32 * C + 16) * sizeof(float2);
+  static constexpr int MINB = 2;              // CTAs per SM: 64 registers
+  static_assert(C == 1 || C == 2 || C == 4 || C == 8, "line length");
+};
+
+struct Args {
+  const float2* in;
+  float2* out;
+  int nlines;
+  long long ld_in, ld_out;  // elements between rows
+  int s;
+  int vec;  // rows: the long line's pairs (s = 2) are 16-byte aligned
+};
+
+// bring the lines from l0 on towards L2 (a line's loads start its chain)
+template <int N, bool COL, bool ADJ>
+PTY_DEVI void prefetch_line(const Args& g, int l0, int t) {
+  using F = Cfg<N, COL>;
+  const int len = ADJ ? N * g.s : N;  // input length
+  if constexpr (COL) {
+    if (l0 < g.nlines)
+      for (int i = t; i < len; i += F::NT) asm volatile("prefetch.global.L2 [%0];" ::"l"(g.in + i * g.ld_in + l0));
+  } else {
+    for (int i = t * 16; i < F::LINES * len; i += F::NT * 16) {  // 128-byte pieces
+      const int l = l0 + i / len;
+      if (l < g.nlines) asm volatile("prefetch.global.L2 [%0];" ::"l"(g.in + l * g.ld_in + i % len));
+    }
+  }
+}
+
+template <int N, bool COL, bool ADJ>
+__global__ void __launch_bounds__(Cfg<N, COL>::NT, Cfg<N, COL>::MINB) k_shift(const Args g) {
+  using F = Cfg<N, COL>;
+  constexpr int C = F::C, T = F::T, P = F::P, LINES = F::LINES, ST = COL ? F::COLS : 1;
+  extern __shared__ __align__(16) unsigned char smem[];
+  float2* buf = reinterpret_cast<float2*>(smem);
+  float2* twa = buf + LINES * F::PLANE;  // W_N^(q a) at a T + q
+  float2* twi = twa + N;                 // its conjugate times the diagonal's factor of a, / N
+  float2* twb = twi + N;                 // W_16C^(q0 b) at b C + q0
+  float2* twj = twb + 16 * C;            // its conjugate times the factor of b
+  float2* dg = twj + 16 * C;             // the factor of c (C = 1: of b)
+  const int t = threadIdx.x;
+  const int line = COL ? t % LINES : t / T, q = COL ? t / LINES : t % T;
+  float2* lb = buf + (COL ? line : line * F::PLANE);  // this line's value i at lb[i * ST]
+  const int a = q / C, q0 = q % C;                    // stage B: digit a, residue q0; stage C: b = q0 + C g
+  const int s = g.s;
+  const int unit = 4096 / (s * N);  // exp(2 pi i j / (s N)) is the conjugate of entry j unit
+  for (int i = t; i < N; i += F::NT) twa[i] = __ldg(&kTw4096[((i / T) * (i % T) * s * unit) & 4095]);
+  for (int i = t; i < 16 * C; i += F::NT) twb[i] = __ldg(&kTw4096[((i / C) * (i % C) * (256 / C)) & 4095]);
+  for (int p = 1; p < s; ++p) {
+    const int sp = ADJ ? -p : p;  // the adjoint's diagonal is the conjugate
+    if (p > 1) __syncthreads();   // the last phase's tables are no longer read
+    for (int i = t; i < N; i += F::NT) {
+      const float2 w = __ldg(&kTw4096[(-(i / T) * ((i % T) * s + sp) * unit) & 4095]);
+      twi[i] = make_float2(w.x * (1.0f / float(N)), w.y * (1.0f / float(N)));
+    }
+    for (int i = t; i < 16 * C; i += F::NT)
+      twj[i] = __ldg(&kTw4096[(-16 * (i / C) * ((i % C) * s + sp) * unit) & 4095]);
+    if (t < 16) {  // frequencies from N / 2 on are negative
+      const int f = C > 1 ? 256 * (t < C / 2 ? t : t - C) : 16 * (t < 8 ? t : t - 16);
+      dg[t] = __ldg(&kTw4096[(-f * sp * unit) & 4095]);
+    }
+    for (int l0 = blockIdx.x * LINES; l0 < g.nlines; l0 += gridDim.x * LINES) {
+      const int l = l0 + line;
+      const bool ok = l < g.nlines;
+      // element i of this line (short side: x or gx; long side: y or gy)
+      auto at = [&](auto* base, long long ld, int i) { return COL ? base + i * ld + l : base + l * ld + i; };
+      float2 v[16];
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        const int m = q + T * e;
+        v[e] = make_float2(0.f, 0.f);
+        if (ok) v[e] = ADJ ? __ldg(at(g.in, g.ld_in, s * m + p)) : __ldg(at(g.in, g.ld_in, m));
+        if (COL && !ADJ && ok && p == 1) *at(g.out, g.ld_out, s * m) = v[e];  // phase 0
+      }
+      prefetch_line<N, COL, ADJ>(g, l0 + gridDim.x * LINES, t);
+      __syncthreads();  // the tables are in place; earlier readers of the exchange are done
+      dft16<false, 1>(v);
+#pragma unroll
+      for (int k = 1; k < 16; ++k) v[k] = c_mul(v[k], twa[k * T + q]);
+#pragma unroll
+      for (int k = 0; k < 16; ++k) lb[(k * P + q) * ST] = v[k];
+      __syncthreads();
+#pragma unroll
+      for (int e = 0; e < 16; ++e) v[e] = lb[(a * P + q0 + C * e) * ST];
+      dft16<false, 1>(v);
+      if constexpr (C > 1) {
+#pragma unroll
+        for (int b = 1; b < 16; ++b) v[b] = c_mul(v[b], twb[b * C + q0]);
+        __syncthreads();
+#pragma unroll
+        for (int b = 0; b < 16; ++b) lb[(a * P + 17 * q0 + b) * ST] = v[b];
+        __syncthreads();
+#pragma unroll
+        for (int gg = 0; gg < 16 / C; ++gg)
+#pragma unroll
+          for (int k = 0; k < C; ++k) v[gg * C + k] = lb[(a * P + 17 * k + q0 + C * gg) * ST];
+#pragma unroll
+        for (int gg = 0; gg < 16 / C; ++gg) dft<C, false, 1>(v + gg * C);
+      }
+#pragma unroll
+      for (int j = 1; j < 16; ++j)
+        if (C == 1 || j % C > 0) v[j] = c_mul(v[j], dg[C > 1 ? j % C : j]);
+      if constexpr (C > 1) {
+#pragma unroll
+        for (int gg = 0; gg < 16 / C; ++gg) dft<C, true, 1>(v + gg * C);
+        __syncthreads();
+#pragma unroll
+        for (int gg = 0; gg < 16 / C; ++gg)
+#pragma unroll
+          for (int k = 0; k < C; ++k) lb[(a * P + 17 * k + q0 + C * gg) * ST] = v[gg * C + k];
+        __syncthreads();
+#pragma unroll
+        for (int b = 0; b < 16; ++b) v[b] = lb[(a * P + 17 * q0 + b) * ST];
+#pragma unroll
+        for (int b = 1; b < 16; ++b) v[b] = c_mul(v[b], twj[b * C + q0]);
+      }
+      dft16<true, 1>(v);
+      __syncthreads();
+#pragma unroll
+      for (int e = 0; e < 16; ++e) lb[(a * P + q0 + C * e) * ST] = v[e];
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < 16; ++k) v[k] = lb[(k * P + q) * ST];
+      v[0] = c_scale(v[0], 1.0f / float(N));
+#pragma unroll
+      for (int k = 1; k < 16; ++k) v[k] = c_mul(v[k], twi[k * T + q]);
+      dft16<true, 1>(v);
+      if (!ok) continue;
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        const int m = q + T * e;
+        if constexpr (ADJ) {
+          float2* o = at(g.out, g.ld_out, m);
+          *o = c_add(p == 1 ? __ldg(at(g.in, g.ld_in, s * m)) : *o, v[e]);
+        } else if (!COL && s == 2 && g.vec) {
+          const float2 x = __ldg(at(g.in, g.ld_in, m));
+          *reinterpret_cast<float4*>(at(g.out, g.ld_out, 2 * m)) = make_float4(x.x, x.y, v[e].x, v[e].y);
+        } else {
+          if (!COL && p == 1) *at(g.out, g.ld_out, s * m) = __ldg(at(g.in, g.ld_in, m));
+          *at(g.out, g.ld_out, s * m + p) = v[e];
+        }
+      }
+    }
+  }
+}
+
+template <int N, bool COL, bool ADJ>
+static int launch(const Args& g, cudaStream_t st) {
+  using F = Cfg<N, COL>;
+  auto kern = k_shift<N, COL, ADJ>;
+  static PtyDevCache slots_cache;  // resident CTAs, with the shared-memory attribute set
+  int dev = 0;
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    int slots = slots_cache.get(&dev);
+    if (dev < 0) return PTYCHO_ERR_LAUNCH;
+    if (slots == 0) {
+      int nsm = 148, per_sm = 1;
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(F::SMEM)) != cudaSuccess)
+        return PTYCHO_ERR_LAUNCH;
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, F::NT, F::SMEM) != cudaSuccess || per_sm < 1)
+        per_sm = 1;
+      slots = nsm * per_sm;
+      slots_cache.put(dev, slots);
+    }
+    const int need = (g.nlines + F::LINES - 1) / F::LINES;
+    kern<<<need < slots ? need : slots, F::NT, F::SMEM, st>>>(g);
+    if (cudaGetLastError() == cudaSuccess) return PTYCHO_OK;
+    slots_cache.put(dev, 0);
+  }
+  return PTYCHO_ERR_LAUNCH;
+}
+
+static bool supported(int n, int s) {
+  return (n == 256 || n == 512 || n == 1024 || n == 2048) && (s == 2 || s == 4) && n * s <= 4096;
+}
+
+// one axis of the upsampling (ADJ: of its adjoint) on every line of a pass
+template <bool COL, bool ADJ>
+static int dispatch(int n, const Args& g, cudaStream_t st) {
+  switch (n) {
+    case 256: return launch<256, COL, ADJ>(g, st);
+    case 512: return launch<512, COL, ADJ>(g, st);
+    case 1024: return launch<1024, COL, ADJ>(g, st);
+    default: return launch<2048, COL, ADJ>(g, st);
+  }
+}
+
+}  // namespace sh
 
 // ---------------------------------------------------------------------------
 // Any line length (the canvases Recovery.py builds are multiples of 6, so
@@ -431,13 +652,25 @@ using namespace pty;
 
 namespace {
 
-// power-of-two pairs keep the compile-time kernels; every other pair runs the
-// run-time-planned one
-template <bool COL>
-int line_pass(int l1, int l2, const float2* in, float2* out, int nlines, long long ld_in, long long ld_out,
-              cudaStream_t s) {
-  if (rs::supported(l1, l2)) return rs::dispatch<COL>(l1, l2, in, out, nlines, ld_in, ld_out, s);
-  return rsg::launch<COL>(l1, l2, in, out, nlines, ld_in, ld_out, s);
+// one axis of the upsampling by s (ADJ: of its adjoint) on every line of a pass:
+// n is the short side
+template <bool COL, bool ADJ>
+int axis_pass(int n, int s, const float2* in, float2* out, int nlines, long long ld_in, long long ld_out,
+              cudaStream_t st) {
+  if (sh::supported(n, s)) {
+    sh::Args g{in, out, nlines, ld_in, ld_out, s, pty_aligned(ADJ ? in : out, 16) ? 1 : 0};
+    return sh::dispatch<COL, ADJ>(n, g, st);
+  }
+  const int l1 = ADJ ? n * s : n, l2 = ADJ ? n : n * s;
+  if (rs::supported(l1, l2)) return rs::dispatch<COL>(l1, l2, in, out, nlines, ld_in, ld_out, st);
+  return rsg::launch<COL>(l1, l2, in, out, nlines, ld_in, ld_out, st);
+}
+
+// s = 1: the operator is the identity
+int copy_plane(const float* in, float* out, size_t n, cudaStream_t st) {
+  return cudaMemcpyAsync(out, in, n * sizeof(float2), cudaMemcpyDeviceToDevice, st) == cudaSuccess
+             ? PTYCHO_OK
+             : PTYCHO_ERR_LAUNCH;
 }
 
 bool supported_upsample(int h, int w, int s) {
@@ -464,10 +697,11 @@ int ptycho_fourier_upsample(const float* x, int h, int w, int s, float* y, void*
   if (!pty_aligned(x, 8) || !pty_aligned(y, 8) || !pty_aligned(workspace, 8)) return PTYCHO_ERR_MISALIGNED;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int W = w * s, H = h * s;
-  float2* tmp = static_cast<float2*>(workspace);
-  int rc = line_pass<false>(w, W, reinterpret_cast<const float2*>(x), tmp, h, w, W, st);  // rows
+  if (s == 1) return copy_plane(x, y, size_t(h) * w, st);
+  float2* tmp = static_cast<float2*>(workspace);  // [H][w]: the column pass moves the narrow side
+  int rc = axis_pass<true, false>(h, s, reinterpret_cast<const float2*>(x), tmp, w, w, w, st);  // columns
   if (rc) return rc;
-  return line_pass<true>(h, H, tmp, reinterpret_cast<float2*>(y), W, W, W, st);           // columns
+  return axis_pass<false, false>(w, s, tmp, reinterpret_cast<float2*>(y), H, w, W, st);          // rows
 }
 
 int ptycho_fourier_upsample_adjoint(const float* gy, int h, int w, int s, float* gx, void* workspace,
@@ -479,10 +713,11 @@ int ptycho_fourier_upsample_adjoint(const float* gy, int h, int w, int s, float*
   if (!pty_aligned(gy, 8) || !pty_aligned(gx, 8) || !pty_aligned(workspace, 8)) return PTYCHO_ERR_MISALIGNED;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int W = w * s, H = h * s;
+  if (s == 1) return copy_plane(gy, gx, size_t(h) * w, st);
   float2* tmp = static_cast<float2*>(workspace);  // [H][w]
-  int rc = line_pass<false>(W, w, reinterpret_cast<const float2*>(gy), tmp, H, W, w, st);  // rows
+  int rc = axis_pass<false, true>(w, s, reinterpret_cast<const float2*>(gy), tmp, H, W, w, st);  // rows
   if (rc) return rc;
-  return line_pass<true>(H, h, tmp, reinterpret_cast<float2*>(gx), w, w, w, st);           // columns
+  return axis_pass<true, true>(h, s, tmp, reinterpret_cast<float2*>(gx), w, w, w, st);            // columns
 }
 
 }  // extern "C"
