@@ -8,240 +8,24 @@
 // unnormalised DFT and P places frequency f in [-n/2, n/2) of the length-n
 // spectrum at f mod N of the length-N one (for even n and N this is what the
 // shift / centred pad / inverse shift of the reference does).  Its adjoint is
-// (s / N) F_n^-1 P^T F_N.  Both are "forward FFT of length L1, spectrum remap,
-// inverse FFT of length L2, scale 1 / min(L1, L2)", so one kernel does all
-// four line transforms:
+// (s / N) F_n^-1 P^T F_N.  Neither forms the long spectrum: the s interleaved
+// phases of the long line are length-n transforms (below).
 //   row pass    -- lines are rows (contiguous), written as rows;
-//   column pass -- lines are LINES adjacent columns (32-byte or wider
-//                  segments per row), written the same way.
+//   column pass -- lines are a few adjacent columns.
 // Upsampling: column pass x -> t [h s][w], row pass t -> y.  Adjoint: row pass
 // g -> t [h s][w], column pass t -> x-gradient.  Both column passes move the
 // narrow side, in pieces of a few columns; the wide side moves as whole rows.
-//
-// Each CTA loads LINES lines into two shared-memory planes (re, im; one float
-// of padding every 32), runs radix-8 or radix-16 Stockham passes (8- or
-// 16-value register slots; lines up to 1024 points use 8 for more threads) --
-// natural order in and out, each thread holding one or two slots in
-// registers, in place between barriers -- remaps the spectrum, runs the
-// inverse passes and writes the lines back.  Twiddles come from the
-// correctly rounded build-time table kTw4096 (twiddle4096.cuh, read through
-// the L1 cache with stride 4096 / L), so no CTA spends time building one.
+// Twiddles of the power-of-two kernels come from the correctly rounded build-time
+// table kTw4096 (twiddle4096.cuh).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "common.cuh"
 #include "dft_regs.cuh"
-#include "line_fft.cuh"
+#include "lines.cuh"
 #include "twiddle4096.cuh"
 
 namespace pty {
-namespace rs {
-
-constexpr int cmax(int a, int b) { return a > b ? a : b; }
-constexpr int cmin(int a, int b) { return a < b ? a : b; }
-
-template <int L1, int L2, bool COL>
-struct Cfg {
-  static constexpr int LMAX = cmax(L1, L2);
-  // row pass: 2048 values per CTA (>= 1 line); column pass: >= 4 lines
-  // (32-byte segments) and 4096 values per CTA when lines are short (2 lines
-  // of 4096, which would fit three CTAs per SM, ran slower: 16-byte pieces)
-  static constexpr int LINES = COL ? cmax(4, 4096 / LMAX) : cmax(1, 2048 / LMAX);
-  static constexpr int N = LINES * LMAX;            // values held by the CTA
-  // values per register slot: 8 (radix-8 passes) for lines up to 1024 points,
-  // which doubles the threads of these small, latency-bound transforms
-  static constexpr int VPT = LMAX <= 1024 ? 8 : 16;
-  static constexpr int NT = cmin(512, N / VPT);     // threads: one slot each, or two
-  static constexpr int SPT = N / VPT / NT;          // slots per thread (1 or 2)
-  static constexpr int PLANE = N + N / 32;          // padded plane length (floats)
-  static constexpr size_t SMEM = size_t(2) * PLANE * 4;
-  static_assert(SPT == 1 || SPT == 2, "slot count");
-  static_assert(L1 >= 64 && L2 >= 64 && LMAX <= 4096, "supported line lengths");
-};
-
-PTY_DEVI int pad(int i) { return i + (i >> 5); }
-
-// One Stockham pass of radix R over every line of length L: butterfly j of a
-// line reads j + r L/R, applies exp(-+2 pi i (j mod NS) r / (NS R)) and the
-// radix-R DFT, and writes (j / NS) NS R + (j mod NS) + r NS.  Twiddles are
-// read from the 4096-entry table kTw4096 (global memory, L1-cached).
-template <int L, int R, int NS, bool INV, int LINES, int NT, int SPT, int LMAX, int VPT>
-PTY_DEVI void stockham(float* re, float* im, int t) {
-  constexpr int BPL = L / R;              // butterflies per line
-  constexpr int NB = LINES * BPL;         // butterflies in the CTA
-  constexpr int PER = VPT / R;            // butterflies per VPT-value slot
-  constexpr int NSLOT = NB / PER;         // slots in use (<= SPT * NT)
-  constexpr int TWS = 4096 / (NS * R);    // twiddle table stride
-  float2 v[SPT][VPT];
-  int jj[SPT][PER], base[SPT][PER];
-#pragma unroll
-  for (int q = 0; q < SPT; ++q) {
-    const int s = t + q * NT;
-#pragma unroll
-    for (int p = 0; p < PER; ++p) {
-      const int b = s + p * NSLOT;  // consecutive lanes -> consecutive j
-      const int line = b / BPL, j = b - line * BPL;
-      jj[q][p] = j;
-      base[q][p] = line * LMAX;
-      if (s < NSLOT) {
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int i = pad(base[q][p] + j + r * BPL);
-          v[q][p * R + r] = make_float2(re[i], im[i]);
-        }
-      }
-    }
-  }
-  __syncthreads();  // every value is read before any is overwritten
-#pragma unroll
-  for (int q = 0; q < SPT; ++q) {
-    const int s = t + q * NT;
-    if (s < NSLOT) {
-#pragma unroll
-      for (int p = 0; p < PER; ++p) {
-        const int j = jj[q][p];
-        const int k = j % NS;
-        if constexpr (NS > 1) {
-#pragma unroll
-          for (int r = 1; r < R; ++r) {
-            float2 w = __ldg(&kTw4096[k * r * TWS]);
-            if constexpr (INV) w.y = -w.y;
-            v[q][p * R + r] = c_mul(v[q][p * R + r], w);
-          }
-        }
-        dft<R, INV, 1>(&v[q][p * R]);
-        const int o = base[q][p] + (j / NS) * NS * R + k;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const int i = pad(o + r * NS);
-          re[i] = v[q][p * R + r].x;
-          im[i] = v[q][p * R + r].y;
-        }
-      }
-    }
-  }
-  __syncthreads();
-}
-
-// all passes of a length-L transform: radix VPT while it divides the rest, then smaller
-template <int L, bool INV, int LINES, int NT, int SPT, int LMAX, int VPT, int NS = 1>
-PTY_DEVI void fft_lines(float* re, float* im, int t) {
-  if constexpr (NS < L) {
-    constexpr int REST = L / NS;
-    constexpr int R = REST >= VPT ? VPT : REST;
-    stockham<L, R, NS, INV, LINES, NT, SPT, LMAX, VPT>(re, im, t);
-    fft_lines<L, INV, LINES, NT, SPT, LMAX, VPT, NS * R>(re, im, t);
-  }
-}
-
-template <int L1, int L2, bool COL>
-__global__ void __launch_bounds__(Cfg<L1, L2, COL>::NT) k_resample(const float2* __restrict__ in,
-                                                                   float2* __restrict__ out, int nlines,
-                                                                   long long ld_in, long long ld_out,
-                                                                   float scale) {
-  using C = Cfg<L1, L2, COL>;
-  constexpr int LINES = C::LINES, NT = C::NT, LMAX = C::LMAX;
-  extern __shared__ __align__(16) unsigned char smem[];
-  float* re = reinterpret_cast<float*>(smem);
-  float* im = re + C::PLANE;
-  const int t = threadIdx.x;
-  const int l0 = blockIdx.x * LINES;
-  // load LINES lines of length L1 (lines past the end read as zero)
-  for (int idx = t; idx < LINES * L1; idx += NT) {
-    int l, k;
-    if constexpr (COL) {
-      l = idx % LINES;
-      k = idx / LINES;
-    } else {
-      l = idx / L1;
-      k = idx - l * L1;
-    }
-    float2 x = make_float2(0.f, 0.f);
-    if (l0 + l < nlines)
-      x = COL ? __ldg(in + k * ld_in + (l0 + l)) : __ldg(in + (l0 + l) * ld_in + k);
-    const int i = pad(l * LMAX + k);
-    re[i] = x.x;
-    im[i] = x.y;
-  }
-  __syncthreads();
-  fft_lines<L1, false, LINES, NT, C::SPT, LMAX, C::VPT>(re, im, t);
-  // spectrum remap: frequency f in [-n/2, n/2), n = min(L1, L2), from f mod L1 to f mod L2
-  if constexpr (L2 > L1) {
-    for (int idx = t; idx < LINES * (L1 / 2); idx += NT) {  // negative frequencies move up
-      const int l = idx / (L1 / 2), k = L1 / 2 + (idx - l * (L1 / 2));
-      const int a = pad(l * LMAX + k), b = pad(l * LMAX + k + (L2 - L1));
-      re[b] = re[a];
-      im[b] = im[a];
-    }
-    __syncthreads();
-    for (int idx = t; idx < LINES * (L2 - L1); idx += NT) {  // the new band is empty
-      const int l = idx / (L2 - L1), k = L1 / 2 + (idx - l * (L2 - L1));
-      const int a = pad(l * LMAX + k);
-      re[a] = 0.f;
-      im[a] = 0.f;
-    }
-    __syncthreads();
-  } else if constexpr (L2 < L1) {
-    for (int idx = t; idx < LINES * (L2 / 2); idx += NT) {  // negative frequencies move down
-      const int l = idx / (L2 / 2), k = L2 / 2 + (idx - l * (L2 / 2));
-      const int a = pad(l * LMAX + k + (L1 - L2)), b = pad(l * LMAX + k);
-      re[b] = re[a];
-      im[b] = im[a];
-    }
-    __syncthreads();
-  }
-  fft_lines<L2, true, LINES, NT, C::SPT, LMAX, C::VPT>(re, im, t);
-  for (int idx = t; idx < LINES * L2; idx += NT) {
-    int l, k;
-    if constexpr (COL) {
-      l = idx % LINES;
-      k = idx / LINES;
-    } else {
-      l = idx / L2;
-      k = idx - l * L2;
-    }
-    if (l0 + l < nlines) {
-      const int i = pad(l * LMAX + k);
-      const float2 y = make_float2(re[i] * scale, im[i] * scale);
-      if constexpr (COL)
-        out[k * ld_out + (l0 + l)] = y;
-      else
-        out[(l0 + l) * ld_out + k] = y;
-    }
-  }
-}
-
-template <int L1, int L2, bool COL>
-int launch(const float2* in, float2* out, int nlines, long long ld_in, long long ld_out, cudaStream_t s) {
-  using C = Cfg<L1, L2, COL>;
-  auto kern = k_resample<L1, L2, COL>;
-  if (C::SMEM > 48 * 1024 &&
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(C::SMEM)) != cudaSuccess)
-    return PTYCHO_ERR_LAUNCH;
-  const int grid = (nlines + C::LINES - 1) / C::LINES;
-  kern<<<grid, C::NT, C::SMEM, s>>>(in, out, nlines, ld_in, ld_out, 1.0f / float(L1 < L2 ? L1 : L2));
-  return cudaGetLastError() == cudaSuccess ? PTYCHO_OK : PTYCHO_ERR_LAUNCH;
-}
-
-// short power-of-two lines: 64 and 128 points, s = 2 or 4
-template <bool COL>
-int dispatch(int l1, int l2, const float2* in, float2* out, int nlines, long long ld_in, long long ld_out,
-             cudaStream_t s) {
-#define PTY_RS(A, B)                                                                                \
-  if (l1 == A && l2 == B) return launch<A, B, COL>(in, out, nlines, ld_in, ld_out, s);               \
-  if (l1 == B && l2 == A) return launch<B, A, COL>(in, out, nlines, ld_in, ld_out, s);
-  PTY_RS(64, 128) PTY_RS(64, 256) PTY_RS(128, 256) PTY_RS(128, 512)
-#undef PTY_RS
-  return PTYCHO_ERR_UNSUPPORTED_SIZE;
-}
-
-bool supported(int n, int N) {
-  const int lo = n < N ? n : N, r = n < N ? N / n : n / N;
-  return (lo == 64 || lo == 128) && lo * r == (n < N ? N : n) && (r == 2 || r == 4);
-}
-
-}  // namespace rs
-
 namespace sh {
 
 // ---------------------------------------------------------------------------
@@ -329,9 +113,11 @@ __global__ void __launch_bounds__(Cfg<N, COL>::NT, Cfg<N, COL>::MINB) k_shift(co
   const int unit = 4096 / (s * N);  // exp(2 pi i j / (s N)) is the conjugate of entry j unit
   for (int i = t; i < N; i += F::NT) twa[i] = __ldg(&kTw4096[((i / T) * (i % T) * s * unit) & 4095]);
   for (int i = t; i < 16 * C; i += F::NT) twb[i] = __ldg(&kTw4096[((i / C) * (i % C) * (256 / C)) & 4095]);
-  for (int p = 1; p < s; ++p) {
+  // upsampling: a CTA has one phase; adjoint: it sums over all of them
+  const int p0 = ADJ ? 1 : blockIdx.y + 1, p1 = ADJ ? s : p0 + 1;
+  for (int p = p0; p < p1; ++p) {
     const int sp = ADJ ? -p : p;  // the adjoint's diagonal is the conjugate
-    if (p > 1) __syncthreads();   // the last phase's tables are no longer read
+    if (p > p0) __syncthreads();  // the last phase's tables are no longer read
     for (int i = t; i < N; i += F::NT) {
       const float2 w = __ldg(&kTw4096[(-(i / T) * ((i % T) * s + sp) * unit) & 4095]);
       twi[i] = make_float2(w.x * (1.0f / float(N)), w.y * (1.0f / float(N)));
@@ -447,7 +233,7 @@ static int launch(const Args& g, cudaStream_t st) {
       slots_cache.put(dev, slots);
     }
     const int need = (g.nlines + F::LINES - 1) / F::LINES;
-    kern<<<need < slots ? need : slots, F::NT, F::SMEM, st>>>(g);
+    kern<<<dim3(need < slots ? need : slots, ADJ ? 1 : g.s - 1), F::NT, F::SMEM, st>>>(g);
     if (cudaGetLastError() == cudaSuccess) return PTYCHO_OK;
     slots_cache.put(dev, 0);
   }
@@ -472,177 +258,204 @@ static int dispatch(int n, const Args& g, cudaStream_t st) {
 }  // namespace sh
 
 // ---------------------------------------------------------------------------
-// Any line length (the canvases Recovery.py builds are multiples of 6, so
+// Any other line length (the canvases Recovery.py builds are multiples of 6, so
 // object grids are multiples of 3 and can hold large prime factors: 498 =
-// 2 * 3 * 83).  Per line: forward DFT of length L1, band remap, inverse DFT
-// of length L2, scale -- the same per-axis operator as above, with the remap
-// written for odd lengths too.  With n = min(L1, L2), N = max(L1, L2) and the
-// band k in [lo, lo + n), lo = -floor(n/2), the reference's fftshift /
-// centred pad / ifftshift puts bin k of the length-n spectrum at bin
-// (k + d) mod N of the length-N one, d = floor(n/2) + floor((N-n)/2) -
-// floor(N/2): d = 0 for even n, or odd n and odd N; d = -1 for odd n and even
-// N (the reference's half-bin asymmetry, kept).  The adjoint gathers back.
-//
-// Transforms are Stockham passes with a run-time plan: radix 16, 8, 4, 2, 3,
-// 5, 7 as register butterflies (dft_regs.cuh), any other prime factor p as a
-// direct p-term sum per output with table twiddles.  Passes ping-pong between
-// two shared-memory buffers of float2 (one float2 of padding every 16 breaks
-// the stride-2^k bank conflicts of the first passes).  Twiddles:
-// exp(-2 pi i j / LMAX), LMAX = max(L1, L2) = s * min(L1, L2), rounded from
-// double-precision sincospi; a length-L pass reads it with stride LMAX / L.
+// 2 * 3 * 83) and any scale, by the same phases on the transforms of lines.cuh.
+// For odd n the reference's fftshift / centred pad / ifftshift puts the band's bin k
+// at (k + d) mod N, d = floor(n/2) + floor((N-n)/2) - floor(N/2): d = 0 for even n,
+// or odd n and odd N; d = -1 for odd n and even N (the reference's half-bin
+// asymmetry, kept): every sample j of the long line is turned by exp(2 pi i d j / N).
+// Measured on B200: 1500^2 to 3000^2 71 + 118 us against 213 + 141 by padded spectra
+// with run-time radix loops; 498^2 to 996^2 and back 160 against 675 us (factor 83).
 // ---------------------------------------------------------------------------
 namespace rsg {
 
-using lfft::LinePlan;
-using lfft::make_plan;
-using lfft::kMaxLen;
-using lfft::pad16;
-using lfft::transform;
-constexpr int kNT = lfft::kLineNT;
-constexpr size_t kSmemCap = 200 * 1024;
+using ln::Plan;
 
 struct Args {
   const float2* in;
   float2* out;
   int nlines;
   long long ld_in, ld_out;
-  LinePlan f1, f2;  // forward transform (length L1), inverse transform (length L2)
-  int lmax;         // max(L1, L2): twiddle table length
-  int lines;        // lines per CTA
-  int ls;           // padded line stride in float2
-  int d, lo;        // band remap offset and lowest band frequency
-  float scale;
+  int s, d;     // scale; band offset (0 or -1)
+  int lines;    // lines per CTA
+  int tables;   // tables of n values: the diagonals, and the turns when d != 0
+  int acc;      // keeps a sum of spectra (adjoint, s > 2)
+  int ngroups;
+  int vec;      // rows: the long line's pairs (s = 2) are 16-byte aligned
+  Plan plan;    // length n, the short side
 };
 
-template <bool COL>
-__global__ void __launch_bounds__(kNT) k_resample_any(const Args g) {
+// LINES = 0: rows; else LINES adjacent columns per CTA
+template <int LINES, int NT, bool ADJ>
+__global__ void __launch_bounds__(NT, LINES == 16 || LINES == 0 ? 4 : 1) k_resample_any(const Args g) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int lines = g.lines, ls = g.ls, lmax = g.lmax;
-  float2* bufA = reinterpret_cast<float2*>(smem);
-  float2* bufB = bufA + size_t(lines) * ls;
-  float2* tw = bufB + size_t(lines) * ls;
-  const int t = threadIdx.x;
-  const int l0 = blockIdx.x * lines;
-  const int L1 = g.f1.L, L2 = g.f2.L;
-  for (int k = t; k < lmax; k += kNT) {
-    double sn, cs;
-    sincospi(-2.0 * double(k) / double(lmax), &sn, &cs);
-    tw[k] = make_float2(float(cs), float(sn));
+  constexpr bool COL = LINES > 0;
+  const int t = threadIdx.x, n = g.plan.n, N = n * g.s, s = g.s;
+  ln::Lines<LINES, NT> ln;
+  float2* ph = ln.init(g.plan, reinterpret_cast<float2*>(smem), COL ? LINES : g.lines, t);
+  auto at = [&](auto* base, long long ld, int l, int i) { return COL ? base + i * ld + l : base + l * ld + i; };
+  // upsampling: a CTA has one phase, whose diagonal is ph; adjoint: it sums all phases'
+  // spectra (s > 2: in acc) before the one inverse transform, with a diagonal each
+  const int p0 = ADJ ? 1 : blockIdx.y + 1, p1 = ADJ ? s : p0 + 1;
+  // odd n, even N: sample s k + p of the long line is turned into (ADJ: out of) the
+  // band's place by exp(-2 pi i (s k + p) / N)
+  const bool turned = g.d != 0;
+  float2* turn_k = ph + (p1 - p0) * n;
+  float2* acc = turn_k + (turned ? n : 0);
+  for (int e = t; e < (p1 - p0) * n; e += NT) {
+    const int p = p0 + e / n, k = e % n;
+    const int f = k < (n + 1) / 2 ? k : k - n;  // signed frequency
+    int j = int((long long)(ADJ ? f : -f) * p % N);
+    if (j < 0) j += N;
+    ph[e] = c_scale(ln::cis_ratio(j, N), 1.0f / float(n));
   }
-  for (int idx = t; idx < lines * L1; idx += kNT) {
-    int l, k;
-    if (COL) {
-      l = idx % lines;
-      k = idx / lines;
-    } else {
-      l = idx / L1;
-      k = idx - l * L1;
-    }
-    float2 x = make_float2(0.f, 0.f);
-    if (l0 + l < g.nlines) x = COL ? __ldg(g.in + k * g.ld_in + (l0 + l)) : __ldg(g.in + (l0 + l) * g.ld_in + k);
-    bufA[l * ls + pad16(k)] = x;
-  }
+  if (turned)
+    for (int k = t; k < n; k += NT) turn_k[k] = ln::cis_ratio(s * k, N);
   __syncthreads();
-  float2* spec = transform<false>(g.f1, bufA, bufB, tw, lines, ls, lmax, t);
-  float2* rem = spec == bufA ? bufB : bufA;
-  // band remap into the other buffer
-  const int n = L1 < L2 ? L1 : L2;
-  for (int idx = t; idx < lines * L2; idx += kNT) {
-    const int l = idx / L2, j = idx - l * L2;
-    float2 v = make_float2(0.f, 0.f);
-    if (L2 >= L1) {  // pad: bin j of the long spectrum holds band frequency k, or nothing
-      int k = (j - g.d - g.lo) % L2;
-      if (k < 0) k += L2;
-      k += g.lo;
-      if (k < g.lo + n) {
-        int src = k % L1;
-        if (src < 0) src += L1;
-        v = spec[l * ls + pad16(src)];
+  auto turn = [&](float2 v, int k, float2 wp) {
+    if (!turned) return v;
+    const float2 w = c_mul(turn_k[k], wp);
+    return ADJ ? c_mulc(v, w) : c_mul(v, w);
+  };
+  const float2 one = make_float2(1.f, 0.f);
+  // element e of a group -> its line and place
+  auto split = [&](int e, int& l, int& k) {
+    if constexpr (COL) {
+      l = e % LINES;
+      k = e / LINES;
+    } else {
+      l = ln::fdiv(e, g.plan.m_n);
+      k = e - l * n;
+    }
+  };
+  const int per = (COL ? LINES : g.lines) * n;
+  for (int grp = blockIdx.x; grp < g.ngroups; grp += gridDim.x) {
+    const int l0 = grp * (COL ? LINES : g.lines);
+    int l, k;
+    for (int p = p0; p < p1; ++p) {
+      const float2 wp = turned ? ln::cis_ratio(p, N) : one;
+      const float2* d = ph + (p - p0) * n;
+#pragma unroll 4
+      for (int e = t; e < per; e += NT) {
+        split(e, l, k);
+        float2 v = make_float2(0.f, 0.f);
+        if (l0 + l < g.nlines)
+          v = ADJ ? turn(__ldg(at(g.in, g.ld_in, l0 + l, s * k + p)), k, wp) : __ldg(at(g.in, g.ld_in, l0 + l, k));
+        ln.put(g.plan, l, k, v);
       }
-    } else {  // crop: bin j of the short spectrum is band frequency k of the long one
-      int k = (j - g.lo) % n;
-      if (k < 0) k += n;
-      k += g.lo;
-      int src = (k + g.d) % L1;
-      if (src < 0) src += L1;
-      v = spec[l * ls + pad16(src)];
+      ln.pad(g.plan);
+      ln.run(g.plan);
+      for (int e = t; e < per; e += NT) {
+        split(e, l, k);
+        float2 v = c_mul(ln.get(g.plan, l, k), d[k]);
+        if (ADJ && s > 2) {  // this thread's own place of acc
+          if (p > 1) v = c_add(acc[e], v);
+          if (p + 1 < s) {
+            acc[e] = v;
+            continue;
+          }
+        }
+        ln.put(g.plan, l, k, c_conj(v));
+      }
+      if (p + 1 < p1) __syncthreads();  // the spectrum is read before the next phase's line overwrites it
     }
-    rem[l * ls + pad16(j)] = v;
+    ln.pad(g.plan);
+    ln.run(g.plan);
+    const float2 wp = turned ? ln::cis_ratio(p0, N) : one;
+#pragma unroll 4
+    for (int e = t; e < per; e += NT) {
+      split(e, l, k);
+      if (l0 + l >= g.nlines) continue;
+      const float2 v = c_conj(ln.get(g.plan, l, k));
+      if constexpr (ADJ) {
+        *at(g.out, g.ld_out, l0 + l, k) = c_add(turn(__ldg(at(g.in, g.ld_in, l0 + l, s * k)), k, one), v);
+      } else {
+        const float2 z = turn(v, k, wp);
+        float2 x = make_float2(0.f, 0.f);
+        if (p0 == 1) x = turn(__ldg(at(g.in, g.ld_in, l0 + l, k)), k, one);
+        if (!COL && s == 2 && g.vec) {
+          *reinterpret_cast<float4*>(at(g.out, g.ld_out, l0 + l, 2 * k)) = make_float4(x.x, x.y, z.x, z.y);
+        } else {
+          if (p0 == 1) *at(g.out, g.ld_out, l0 + l, s * k) = x;
+          *at(g.out, g.ld_out, l0 + l, s * k + p0) = z;
+        }
+      }
+    }
+    __syncthreads();  // the buffers are free for the next group
   }
-  __syncthreads();
-  float2* other = rem == bufA ? bufB : bufA;
-  float2* res = transform<true>(g.f2, rem, other, tw, lines, ls, lmax, t);
-  for (int idx = t; idx < lines * L2; idx += kNT) {
-    int l, k;
-    if (COL) {
-      l = idx % lines;
-      k = idx / lines;
-    } else {
-      l = idx / L2;
-      k = idx - l * L2;
+}
+
+static size_t smem_of(const Args& g, int lines) {
+  return ln::smem_bytes(g.plan, lines, g.tables + (g.acc ? lines : 0));
+}
+
+template <int LINES, int NT, bool ADJ>
+static int launch_k(const Args& g, cudaStream_t st) {
+  auto kern = k_resample_any<LINES, NT, ADJ>;
+  const size_t smem = smem_of(g, LINES > 0 ? LINES : g.lines);
+  static PtyDevCache attr;
+  int dev = 0;
+  for (int attempt = 0; attempt < 2; ++attempt) {
+    int nsm = attr.get(&dev);
+    if (dev < 0) return PTYCHO_ERR_LAUNCH;
+    if (!nsm) {
+      nsm = 148;
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ln::kSmemCap)) != cudaSuccess)
+        return PTYCHO_ERR_LAUNCH;
+      attr.put(dev, nsm);
     }
-    if (l0 + l < g.nlines) {
-      const float2 y = res[l * ls + pad16(k)];
-      const float2 o = make_float2(y.x * g.scale, y.y * g.scale);
-      if (COL)
-        g.out[k * g.ld_out + (l0 + l)] = o;
-      else
-        g.out[(l0 + l) * g.ld_out + k] = o;
-    }
+    const int per_sm = int(233472 / (smem + 1024));
+    const int slots = nsm * (per_sm < 1 ? 1 : (per_sm > 4 ? 4 : per_sm));
+    kern<<<dim3(g.ngroups < slots ? g.ngroups : slots, ADJ ? 1 : g.s - 1), NT, smem, st>>>(g);
+    if (cudaGetLastError() == cudaSuccess) return PTYCHO_OK;
+    attr.put(dev, 0);
   }
+  return PTYCHO_ERR_LAUNCH;
 }
 
-static size_t smem_bytes(int lines, int ls, int lmax) {
-  return (size_t(2) * lines * ls + size_t(lmax)) * sizeof(float2);
-}
-
-// true when the pair of line lengths is handled (one a whole multiple of the other)
-static bool supported_pair(int l1, int l2) {
-  if (l1 < 1 || l2 < 1 || l1 > kMaxLen || l2 > kMaxLen) return false;
-  const int lo = l1 < l2 ? l1 : l2, hi = l1 < l2 ? l2 : l1;
-  return hi % lo == 0;
-}
-
-// lines of length l1 -> lines of length l2: forward DFT, band remap, inverse DFT, scale 1 / min(l1, l2)
-template <bool COL>
-static int launch(int l1, int l2, const float2* in, float2* out, int nlines, long long ld_in, long long ld_out,
-                  cudaStream_t s) {
-  if (!supported_pair(l1, l2)) return PTYCHO_ERR_UNSUPPORTED_SIZE;
+// one axis of length n upsampled by s (ADJ: its adjoint) on every line of a pass
+template <bool COL, bool ADJ>
+static int launch(int n, int s, const float2* in, float2* out, int nlines, long long ld_in, long long ld_out,
+                  cudaStream_t st) {
   Args g{};
-  if (!make_plan(l1, &g.f1) || !make_plan(l2, &g.f2)) return PTYCHO_ERR_UNSUPPORTED_SIZE;
+  const int N = n * s;
+  g.d = n / 2 + (N - n) / 2 - N / 2;
+  g.acc = ADJ && s > 2;
+  g.tables = (ADJ ? s - 1 : 1) + (g.d ? 1 : 0);
+  if (!ln::make_plan(n, g.tables + g.acc, &g.plan)) return PTYCHO_ERR_UNSUPPORTED_SIZE;
   g.in = in;
   g.out = out;
   g.nlines = nlines;
   g.ld_in = ld_in;
   g.ld_out = ld_out;
-  const int n = l1 < l2 ? l1 : l2, N = l1 < l2 ? l2 : l1;
-  g.lmax = N;
-  g.lo = -(n / 2);
-  g.d = n / 2 + (N - n) / 2 - N / 2;
-  g.scale = 1.0f / float(n);
-  g.ls = pad16(N - 1) + 1;
-  // lines per CTA: ~8192 values, at least 4 adjacent columns (32-byte
-  // segments) in the column pass, within the shared-memory cap
-  int lines = N >= 8192 ? 1 : 8192 / N;
-  if (COL && lines < 4) lines = 4;
-  while (lines > 1 && smem_bytes(lines, g.ls, N) > kSmemCap) --lines;
-  g.lines = lines;
-  const size_t smem = smem_bytes(lines, g.ls, N);
-  auto kern = k_resample_any<COL>;
-  static PtyDevCache attr_set;
-  int dev = 0;
-  for (int attempt = 0; attempt < 2; ++attempt) {
-    if (!attr_set.get(&dev)) {
-      if (dev < 0) return PTYCHO_ERR_LAUNCH;
-      if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemCap)) != cudaSuccess)
-        return PTYCHO_ERR_LAUNCH;
-      attr_set.put(dev, 1);
+  g.s = s;
+  g.vec = ld_out % 2 == 0 && pty_aligned(out, 16) ? 1 : 0;
+  auto groups = [&](int lines) {
+    g.lines = lines;
+    g.ngroups = (nlines + lines - 1) / lines;
+  };
+  if constexpr (COL) {
+    // 16 adjacent columns (128-byte pieces) while two CTAs fit an SM, else 4 or 1
+    if (smem_of(g, 16) <= 112 * 1024) {
+      groups(16);
+      return launch_k<16, 256, ADJ>(g, st);
     }
-    kern<<<(nlines + lines - 1) / lines, kNT, smem, s>>>(g);
-    if (cudaGetLastError() == cudaSuccess) return PTYCHO_OK;
-    attr_set.put(dev, 0);
+    if (smem_of(g, 4) <= ln::kSmemCap) {
+      groups(4);
+      return launch_k<4, 512, ADJ>(g, st);
+    }
+    groups(1);
+    return launch_k<1, 512, ADJ>(g, st);
+  } else {
+    // about 3072 values per CTA
+    int lines = 3072 / g.plan.m;
+    lines = lines < 1 ? 1 : lines;
+    while (lines > 1 && smem_of(g, lines) > ln::kSmemCap) --lines;
+    groups(lines);
+    return launch_k<0, 256, ADJ>(g, st);
   }
-  return PTYCHO_ERR_LAUNCH;
 }
 
 }  // namespace rsg
@@ -661,9 +474,7 @@ int axis_pass(int n, int s, const float2* in, float2* out, int nlines, long long
     sh::Args g{in, out, nlines, ld_in, ld_out, s, pty_aligned(ADJ ? in : out, 16) ? 1 : 0};
     return sh::dispatch<COL, ADJ>(n, g, st);
   }
-  const int l1 = ADJ ? n * s : n, l2 = ADJ ? n : n * s;
-  if (rs::supported(l1, l2)) return rs::dispatch<COL>(l1, l2, in, out, nlines, ld_in, ld_out, st);
-  return rsg::launch<COL>(l1, l2, in, out, nlines, ld_in, ld_out, st);
+  return rsg::launch<COL, ADJ>(n, s, in, out, nlines, ld_in, ld_out, st);
 }
 
 // s = 1: the operator is the identity
@@ -675,7 +486,7 @@ int copy_plane(const float* in, float* out, size_t n, cudaStream_t st) {
 
 bool supported_upsample(int h, int w, int s) {
   if (h <= 0 || w <= 0 || s <= 0) return false;
-  if (h > rsg::kMaxLen / s || w > rsg::kMaxLen / s) return false;
+  if (h > ln::kMaxLen / s || w > ln::kMaxLen / s) return false;
   return true;
 }
 
