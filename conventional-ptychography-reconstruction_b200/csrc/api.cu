@@ -114,7 +114,8 @@ int ptycho_forward_intensity(const float* O, int H, int W, const float* P, int M
 
 size_t ptycho_forward_intensity_workspace_size(int M, int N, int B) {
   if (B < 0 || !supported_probe(M, N)) return 0;
-  if (fused_probe(M, N)) return 256;  // the fused kernels need none
+  if (M == 256 && N == 256) return split256_intensity_scratch(B);  // 256 bytes will do: the cluster kernel
+  if (fused_probe(M, N)) return 256;                               // the fused kernels need none
   return pty_align_up(size_t(B) * M * N * sizeof(float2), 256);
 }
 
@@ -126,8 +127,14 @@ int ptycho_forward_intensity_ws(const float* O, int H, int W, const float* P, in
   if (st) return st;
   if (B == 0) return PTYCHO_OK;
   if (!I_out) return PTYCHO_ERR_INVALID_ARG;
-  if (fused_probe(M, N))
+  if (fused_probe(M, N)) {
+    if (M == 256 && workspace && workspace_bytes >= split256_intensity_scratch(B) && pty_aligned(workspace, 256)) {
+      FusedArgs a = make_args(O, H, W, P, tl, nullptr, F, batch, B, status_out);
+      a.I_out = I_out;
+      return split256_intensity(a, workspace, reinterpret_cast<cudaStream_t>(stream));
+    }
     return ptycho_forward_intensity(O, H, W, P, M, N, tl, F, batch, B, I_out, status_out, stream);
+  }
   if (!workspace || workspace_bytes < ptycho_forward_intensity_workspace_size(M, N, B)) return PTYCHO_ERR_WORKSPACE;
   if (!pty_aligned(workspace, 256)) return PTYCHO_ERR_MISALIGNED;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);

@@ -53,14 +53,17 @@ PTY_DEVI void dft2(float2* a) {
   a[S] = c_sub(t, a[S]);
 }
 
-template <bool INV, int S>
+// PK: packed adds (fewer issue slots; the rotated sums swap parts and stay scalar)
+template <bool INV, int S, bool PK = false>
 PTY_DEVI void dft4(float2* a) {
-  float2 t0 = c_add(a[0], a[2 * S]);
-  float2 t1 = c_sub(a[0], a[2 * S]);
-  float2 t2 = c_add(a[S], a[3 * S]);
-  float2 t3 = mul_mi<INV>(c_sub(a[S], a[3 * S]));
-  a[0] = c_add(t0, t2);
-  a[2 * S] = c_sub(t0, t2);
+  auto add = [](float2 x, float2 y) { return PK ? c_add_pk(x, y) : c_add(x, y); };
+  auto sub = [](float2 x, float2 y) { return PK ? c_sub_pk(x, y) : c_sub(x, y); };
+  const float2 t0 = add(a[0], a[2 * S]);
+  const float2 t1 = sub(a[0], a[2 * S]);
+  const float2 t2 = add(a[S], a[3 * S]);
+  const float2 t3 = mul_mi<INV>(sub(a[S], a[3 * S]));
+  a[0] = add(t0, t2);
+  a[2 * S] = sub(t0, t2);
   a[S] = c_add(t1, t3);
   a[3 * S] = c_sub(t1, t3);
 }
@@ -85,14 +88,14 @@ PTY_DEVI void dft8(float2* a) {
   }
 }
 
-template <bool INV, int S>
+template <bool INV, int S, bool PK = false>
 PTY_DEVI void dft16(float2* a) {
   // n = 4*n1 + n2 ; k = k1 + 4*k2
   float2 t[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) t[i] = a[i * S];
 #pragma unroll
-  for (int n2 = 0; n2 < 4; ++n2) dft4<INV, 4>(t + n2);  // over n1 -> k1 at t[4*k1+n2]
+  for (int n2 = 0; n2 < 4; ++n2) dft4<INV, 4, PK>(t + n2);  // over n1 -> k1 at t[4*k1+n2]
   // twiddle W16^(n2*k1)
   t[5] = w16_mul<1, INV>(t[5]);
   t[6] = w16_mul<2, INV>(t[6]);
@@ -104,7 +107,7 @@ PTY_DEVI void dft16(float2* a) {
   t[14] = w16_mul<6, INV>(t[14]);
   t[15] = w16_mul<9, INV>(t[15]);
 #pragma unroll
-  for (int k1 = 0; k1 < 4; ++k1) dft4<INV, 1>(t + 4 * k1);  // over n2 -> k2 at t[4*k1+k2]
+  for (int k1 = 0; k1 < 4; ++k1) dft4<INV, 1, PK>(t + 4 * k1);  // over n2 -> k2 at t[4*k1+k2]
 #pragma unroll
   for (int k1 = 0; k1 < 4; ++k1)
 #pragma unroll

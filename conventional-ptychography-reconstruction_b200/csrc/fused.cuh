@@ -386,4 +386,16 @@ int launch_split256(int mode, int loss, const FusedArgs& a, double* lpart, float
 int split256_dp_sum(const float2* dp_part, int B, float2* dP, bool accumulate, const double* loss_pat,
                     double* loss_total, cudaStream_t s);
 
+// M = 256 intensities by the same row kernel and a column kernel: `scratch` holds
+// split256_intensity_scratch(B) bytes, 256-byte aligned, for up to
+// kIntensityChunk patterns at a time (512 KB each).  Measured for 512 patterns:
+// chunks of 64, 128, 256, 512 took 198, 190, 169, 157 us (fuller waves win over
+// keeping a chunk in L2); the cluster kernel, which needs no scratch, 314 us.
+#ifndef PTY_S256_INTENSITY_CHUNK
+#define PTY_S256_INTENSITY_CHUNK 512
+#endif
+constexpr int kIntensityChunk = PTY_S256_INTENSITY_CHUNK;
+size_t split256_intensity_scratch(int B);
+int split256_intensity(FusedArgs a, void* scratch, cudaStream_t s);
+
 }  // namespace pty

@@ -18,7 +18,7 @@
 // Line DFT of length 256 = 16 x 16.  Rows: a half-warp per row, lane j
 // holding x[j + 16 k] in registers; a 16-point DFT over k, the twiddle
 // W256^(j p), a 16 x 16 transpose through shared memory (padded rows of 17:
-// the two half-warps of a warp hit disjoint banks), a second 16-point DFT;
+// conflict free for 8-byte accesses), a second 16-point DFT;
 // lane p then holds X[p + 16 q], the input layout, so lines chain without
 // reordering.  Columns: the same factorisation with the 16 values of a
 // column spread over 16 half-warps (a half-warp = 16 adjacent columns, so
@@ -34,13 +34,16 @@
 
 // Build-time tuning (measured on B200, c3 = 64 and c4 = 512 patterns): one
 // launch per kernel for up to 512 patterns beat chunks of 64 that keep the
-// scratch in L2 (c4 515 vs 551 us: fuller waves, fewer launches); three
-// column CTAs per SM at 85 registers beat four at 64 with a 20-byte spill.
+// scratch in L2 (c4 515 vs 551 us: fuller waves, fewer launches).  Four
+// column CTAs per SM fit 64 registers with the 8-byte transpose and packed adds
+// (c3 71.8 -> 68.6, c4 458 -> 442 us a step; three CTAs 69.0, 451).  The column
+// kernels take the patterns in descending order, so they start on the scratch that
+// the row kernel wrote last and that is still in L2 (c4 442 -> 429 us).
 #ifndef PTY_S256_CHUNK
 #define PTY_S256_CHUNK 512
 #endif
 #ifndef PTY_S256_COLS_MINB
-#define PTY_S256_COLS_MINB 3
+#define PTY_S256_COLS_MINB 4
 #endif
 #ifndef PTY_S256_ROWS_MINB
 #define PTY_S256_ROWS_MINB 4
@@ -53,17 +56,17 @@ constexpr int M = 256;
 constexpr int NT = 256;            // 16 lines x 16 lanes per CTA
 constexpr int LINES = 16;
 constexpr int TP = 17;             // padded row of a 16 x 16 transpose / tile
-constexpr int BUF = LINES * 16 * TP;  // floats per plane (re or im): 4352
+constexpr int BUF = LINES * 16 * TP;  // float2 of the transpose buffer: 4352
 constexpr int NCB = M / LINES;     // column (or row) blocks per pattern: 16
 static_assert(NCB == kSplit256Blocks, "loss partials per pattern");
 constexpr int kChunk = PTY_S256_CHUNK;
 static_assert(kChunk % kDpGroup == 0, "probe-gradient groups do not straddle chunks");
 
-// shared memory: twiddles, two transpose planes (re, im), reduction
+// shared memory: twiddles, transpose buffer (8-byte accesses: half the instructions
+// of separate planes, and both half-warps of a transpose free of conflicts), reduction
 constexpr size_t SM_TW = 0;
-constexpr size_t SM_RE = SM_TW + M * 8;
-constexpr size_t SM_IM = SM_RE + BUF * 4;
-constexpr size_t SM_RED = SM_IM + BUF * 4;
+constexpr size_t SM_BUF = SM_TW + M * 8;
+constexpr size_t SM_RED = SM_BUF + BUF * 8;
 constexpr size_t SMEM_ROWS = SM_RED;              // kernels A and C
 constexpr size_t SMEM_COLS = SM_RED + 8 * 8;      // kernel B
 
@@ -71,6 +74,7 @@ struct Args {
   FusedArgs f;
   double* lpart;  // [B][NCB] FP64 loss partial of each column block
   int b0;         // first pattern of this chunk
+  int x0;         // pattern whose scratch is slot 0 of Eout
 };
 
 // The line twiddles W256^(j p), j, p = 0..15 (forward sign), stored at
@@ -86,10 +90,10 @@ PTY_DEVI void fill_twiddles(float2* tw) {
 
 // 256-point DFT (INV: unnormalised inverse) of one line held by a half-warp.
 // In: lane j holds x[j + 16 k] in v[k].  Out: lane j holds X[j + 16 q] in v[q].
-// bre / bim: this line's private 16 x 17 transpose planes.
+// buf: this line's private 16 x 17 transpose buffer.
 template <bool INV>
-PTY_DEVI void line256(float2 (&v)[16], int j, float* bre, float* bim, const float2* tw) {
-  dft16<INV, 1>(v);  // v[p] = sum_k x[j + 16 k] W16^(k p)
+PTY_DEVI void line256(float2 (&v)[16], int j, float2* buf, const float2* tw) {
+  dft16<INV, 1, true>(v);  // v[p] = sum_k x[j + 16 k] W16^(k p)
 #pragma unroll
   for (int p = 1; p < 16; ++p) {
     const float2 w = tw[p * 16 + j];
@@ -97,14 +101,11 @@ PTY_DEVI void line256(float2 (&v)[16], int j, float* bre, float* bim, const floa
   }
   __syncwarp();
 #pragma unroll
-  for (int p = 0; p < 16; ++p) {
-    bre[p * TP + j] = v[p].x;
-    bim[p * TP + j] = v[p].y;
-  }
+  for (int p = 0; p < 16; ++p) buf[p * TP + j] = v[p];
   __syncwarp();
 #pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = make_float2(bre[j * TP + i], bim[j * TP + i]);
-  dft16<INV, 1>(v);  // v[q] = X[j + 16 q]
+  for (int i = 0; i < 16; ++i) v[i] = buf[j * TP + i];
+  dft16<INV, 1, true>(v);  // v[q] = X[j + 16 q]
 }
 
 PTY_DEVI bool window_ok(const FusedArgs& a, int b, int& f, int2& w) {
@@ -123,8 +124,7 @@ PTY_DEVI bool window_ok(const FusedArgs& a, int b, int& f, int2& w) {
 __global__ void __launch_bounds__(NT, PTY_S256_ROWS_MINB) k_rows_fwd(const Args g) {
   extern __shared__ __align__(16) unsigned char smem[];
   float2* tw = reinterpret_cast<float2*>(smem + SM_TW);
-  float* pre = reinterpret_cast<float*>(smem + SM_RE);
-  float* pim = reinterpret_cast<float*>(smem + SM_IM);
+  float2* buf = reinterpret_cast<float2*>(smem + SM_BUF);
   const FusedArgs& a = g.f;
   const int t = threadIdx.x, r = t >> 4, j = t & 15;
   const int b = g.b0 + blockIdx.y;
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(NT, PTY_S256_ROWS_MINB) k_rows_fwd(const Args 
   int2 w;
   const bool ok = window_ok(a, b, f, w);
   if (blockIdx.x == 0 && t == 0) {
-    a.tlb[b] = ok ? w : make_int2(-1, -1);
+    a.tlb[b - g.x0] = ok ? w : make_int2(-1, -1);
     if (!ok) pty_raise(a.status, PTYCHO_ERR_WINDOW);
   }
   if (!ok) return;  // uniform over the CTA
@@ -154,8 +154,8 @@ __global__ void __launch_bounds__(NT, PTY_S256_ROWS_MINB) k_rows_fwd(const Args 
     }
   }
   __syncthreads();  // twiddles ready
-  line256<false>(v, j, pre + r * 16 * TP, pim + r * 16 * TP, tw);
-  float2* Xr = a.Eout + size_t(b) * M * M + size_t(y) * M + j;
+  line256<false>(v, j, buf + r * 16 * TP, tw);
+  float2* Xr = a.Eout + size_t(b - g.x0) * M * M + size_t(y) * M + j;
 #pragma unroll
   for (int q = 0; q < 16; ++q) Xr[16 * q] = v[q];
 }
@@ -166,8 +166,7 @@ __global__ void __launch_bounds__(NT, PTY_S256_ROWS_MINB) k_rows_fwd(const Args 
 __global__ void __launch_bounds__(NT, PTY_S256_ROWS_MINB) k_rows_inv(const Args g) {
   extern __shared__ __align__(16) unsigned char smem[];
   float2* tw = reinterpret_cast<float2*>(smem + SM_TW);
-  float* pre = reinterpret_cast<float*>(smem + SM_RE);
-  float* pim = reinterpret_cast<float*>(smem + SM_IM);
+  float2* buf = reinterpret_cast<float2*>(smem + SM_BUF);
   const FusedArgs& a = g.f;
   const int t = threadIdx.x, r = t >> 4, j = t & 15;
   const int b = g.b0 + blockIdx.y;
@@ -185,7 +184,7 @@ __global__ void __launch_bounds__(NT, PTY_S256_ROWS_MINB) k_rows_inv(const Args 
 #pragma unroll
   for (int k = 0; k < 16; ++k) v[k] = Xr[16 * k];
   __syncthreads();
-  line256<true>(v, j, pre + r * 16 * TP, pim + r * 16 * TP, tw);
+  line256<true>(v, j, buf + r * 16 * TP, tw);
 #pragma unroll
   for (int q = 0; q < 16; ++q) Xr[16 * q] = v[q];
 }
@@ -200,8 +199,7 @@ __global__ void __launch_bounds__(NT, PTY_S256_ROWS_MINB) k_rows_inv(const Args 
 __global__ void __launch_bounds__(NT, 2) k_rows_inv_dp(const Args g, float2* __restrict__ part) {
   extern __shared__ __align__(16) unsigned char smem[];
   float2* tw = reinterpret_cast<float2*>(smem + SM_TW);
-  float* pre = reinterpret_cast<float*>(smem + SM_RE);
-  float* pim = reinterpret_cast<float*>(smem + SM_IM);
+  float2* buf = reinterpret_cast<float2*>(smem + SM_BUF);
   const FusedArgs& a = g.f;
   const int t = threadIdx.x, r = t >> 4, j = t & 15;
   const int y = blockIdx.x * LINES + r;
@@ -225,7 +223,7 @@ __global__ void __launch_bounds__(NT, 2) k_rows_inv_dp(const Args g, float2* __r
     float2 v[16];
 #pragma unroll
     for (int k = 0; k < 16; ++k) v[k] = Xr[16 * k];
-    line256<true>(v, j, pre + r * 16 * TP, pim + r * 16 * TP, tw);
+    line256<true>(v, j, buf + r * 16 * TP, tw);
     const float2* Or = a.O + size_t(w.x + y) * a.W + w.y + j;
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
@@ -289,15 +287,15 @@ __global__ void __launch_bounds__(256) k_dp_sum(const float2* __restrict__ part,
 // 256-point DFT of one column per thread slot, spread over the CTA: thread
 // (j, c) = (t >> 4, t & 15) holds x[j + 16 k] of column c in v[k]; a 16-point
 // DFT over k, the twiddle W256^(j p), a transpose across warps through the
-// planes (row p of the transpose at p * CT, so the two half-warps of a warp
-// hit disjoint banks when writing and when reading), a second 16-point DFT.
+// buffer (row p of the transpose at p * CT; a half-warp is 16 adjacent columns, so
+// its 8-byte accesses are one contiguous piece), a second 16-point DFT.
 // Thread (p, c) then holds X[p + 16 q] in v[q] -- the input layout again.
 // Contains two barriers: every thread of the CTA calls it, with the twiddle
 // table already published by a barrier.
-constexpr int CT = 16 * 16 + 16;  // floats per transpose row p (16 j x 16 c + pad)
+constexpr int CT = 16 * 16;  // float2 per transpose row p (16 j x 16 c)
 template <bool INV>
-PTY_DEVI void col256(float2 (&v)[16], int j, int c, float* bre, float* bim, const float2* tw) {
-  dft16<INV, 1>(v);
+PTY_DEVI void col256(float2 (&v)[16], int j, int c, float2* buf, const float2* tw) {
+  dft16<INV, 1, true>(v);
 #pragma unroll
   for (int p = 1; p < 16; ++p) {
     const float2 w = tw[p * 16 + j];
@@ -305,16 +303,13 @@ PTY_DEVI void col256(float2 (&v)[16], int j, int c, float* bre, float* bim, cons
   }
   __syncthreads();  // earlier readers of the planes are done
 #pragma unroll
-  for (int p = 0; p < 16; ++p) {
-    bre[p * CT + j * 16 + c] = v[p].x;
-    bim[p * CT + j * 16 + c] = v[p].y;
-  }
+  for (int p = 0; p < 16; ++p) buf[p * CT + j * 16 + c] = v[p];
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = make_float2(bre[j * CT + i * 16 + c], bim[j * CT + i * 16 + c]);
-  dft16<INV, 1>(v);
+  for (int i = 0; i < 16; ++i) v[i] = buf[j * CT + i * 16 + c];
+  dft16<INV, 1, true>(v);
 }
-static_assert(16 * CT <= BUF, "column transpose planes fit the plane size");
+static_assert(16 * CT <= BUF, "column transpose fits the buffer");
 
 // B: column DFTs, loss, and (GRAD) the gradient's inverse column DFTs.
 // grid (NCB, chunk): CTA (cb, b - b0) owns columns 16 cb .. 16 cb + 15 of
@@ -325,12 +320,11 @@ template <int LOSS, bool GRAD>
 __global__ void __launch_bounds__(NT, PTY_S256_COLS_MINB) k_cols(const Args g) {
   extern __shared__ __align__(16) unsigned char smem[];
   float2* tw = reinterpret_cast<float2*>(smem + SM_TW);
-  float* bre = reinterpret_cast<float*>(smem + SM_RE);
-  float* bim = reinterpret_cast<float*>(smem + SM_IM);
+  float2* buf = reinterpret_cast<float2*>(smem + SM_BUF);
   double* red = reinterpret_cast<double*>(smem + SM_RED);
   const FusedArgs& a = g.f;
   const int t = threadIdx.x, j = t >> 4, c = t & 15;
-  const int b = g.b0 + blockIdx.y;
+  const int b = g.b0 + gridDim.y - 1 - blockIdx.y;
   const int fx0 = blockIdx.x * LINES;
   if (__ldg(&a.tlb[b].x) < 0) return;  // skipped window (uniform)
   const int f = a.batch ? __ldg(a.batch + b) : b;
@@ -343,7 +337,7 @@ __global__ void __launch_bounds__(NT, PTY_S256_COLS_MINB) k_cols(const Args g) {
 #pragma unroll
   for (int k = 0; k < 16; ++k) v[k] = Xc[size_t(j + 16 * k) * M];
   __syncthreads();  // twiddles ready
-  col256<false>(v, j, c, bre, bim, tw);  // v[q] = F[j + 16 q][fx0 + c]
+  col256<false>(v, j, c, buf, tw);  // v[q] = F[j + 16 q][fx0 + c]
 
   constexpr float inv_mn = 1.0f / float(M * M);
   float part[16];
@@ -376,10 +370,36 @@ __global__ void __launch_bounds__(NT, PTY_S256_COLS_MINB) k_cols(const Args g) {
   const double tot = block_sum<NT>((double)part[0], red);
   if (t == 0) g.lpart[size_t(b) * NCB + blockIdx.x] = tot;
   if constexpr (GRAD) {
-    col256<true>(v, j, c, bre, bim, tw);  // v[q] = X2[j + 16 q][fx0 + c]
+    col256<true>(v, j, c, buf, tw);  // v[q] = X2[j + 16 q][fx0 + c]
 #pragma unroll
     for (int q = 0; q < 16; ++q) Xc[size_t(j + 16 * q) * M] = v[q];
   }
+}
+
+// B for MODE_INTENSITY: column DFTs and |F|^2 (NaN for a skipped window)
+__global__ void __launch_bounds__(NT, PTY_S256_ROWS_MINB) k_cols_intensity(const Args g) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  float2* tw = reinterpret_cast<float2*>(smem + SM_TW);
+  float2* buf = reinterpret_cast<float2*>(smem + SM_BUF);
+  const FusedArgs& a = g.f;
+  const int t = threadIdx.x, j = t >> 4, c = t & 15;
+  const int b = g.b0 + gridDim.y - 1 - blockIdx.y;
+  const int fx0 = blockIdx.x * LINES;
+  float* Ic = a.I_out + size_t(b) * M * M + fx0 + c;
+  if (__ldg(&a.tlb[b - g.x0].x) < 0) {  // uniform
+#pragma unroll
+    for (int q = 0; q < 16; ++q) Ic[size_t(j + 16 * q) * M] = __int_as_float(0x7fc00000);
+    return;
+  }
+  const float2* Xc = a.Eout + size_t(b - g.x0) * M * M + fx0 + c;
+  fill_twiddles(tw);
+  float2 v[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) v[k] = Xc[size_t(j + 16 * k) * M];
+  __syncthreads();  // twiddles ready
+  col256<false>(v, j, c, buf, tw);
+#pragma unroll
+  for (int q = 0; q < 16; ++q) Ic[size_t(j + 16 * q) * M] = fmaf(v[q].x, v[q].x, v[q].y * v[q].y);
 }
 
 // MODE_LOSS: per-pattern losses from the column-block partials (fixed order)
@@ -413,7 +433,7 @@ static int launch_t(bool adj, const FusedArgs& fa, double* lpart, float2* dp_par
   if (!set_smem(k_rows_fwd, SMEM_ROWS, c_rows_fwd) || !set_smem(k_rows_inv, SMEM_ROWS, c_rows_inv) ||
       !set_smem(k_rows_inv_dp, SMEM_ROWS, c_rows_inv_dp) || !set_smem(kcols, SMEM_COLS, c_cols))
     return PTYCHO_ERR_LAUNCH;
-  Args g{fa, lpart, 0};
+  Args g{fa, lpart, 0, 0};
   for (int b0 = 0; b0 < fa.B; b0 += kChunk) {
     const int n = fa.B - b0 < kChunk ? fa.B - b0 : kChunk;
     g.b0 = b0;
@@ -429,6 +449,26 @@ static int launch_t(bool adj, const FusedArgs& fa, double* lpart, float2* dp_par
   if (cudaGetLastError() == cudaSuccess) return PTYCHO_OK;
   int dev;
   for (PtyDevCache* c : {&c_rows_fwd, &c_rows_inv, &c_rows_inv_dp, &c_cols})
+    if (c->get(&dev)) c->put(dev, 0);
+  return PTYCHO_ERR_LAUNCH;
+}
+
+// Intensities over chunks of kIntensityChunk patterns, each a row and a column
+// launch over the same scratch
+static int launch_intensity(const FusedArgs& fa, cudaStream_t s) {
+  static PtyDevCache c_rows, c_cols;
+  if (!set_smem(k_rows_fwd, SMEM_ROWS, c_rows) || !set_smem(k_cols_intensity, SMEM_ROWS, c_cols))
+    return PTYCHO_ERR_LAUNCH;
+  Args g{fa, nullptr, 0, 0};
+  for (int b0 = 0; b0 < fa.B; b0 += kIntensityChunk) {
+    const int n = fa.B - b0 < kIntensityChunk ? fa.B - b0 : kIntensityChunk;
+    g.b0 = g.x0 = b0;
+    k_rows_fwd<<<dim3(NCB, n), NT, SMEM_ROWS, s>>>(g);
+    k_cols_intensity<<<dim3(NCB, n), NT, SMEM_ROWS, s>>>(g);
+  }
+  if (cudaGetLastError() == cudaSuccess) return PTYCHO_OK;
+  int dev;
+  for (PtyDevCache* c : {&c_rows, &c_cols})
     if (c->get(&dev)) c->put(dev, 0);
   return PTYCHO_ERR_LAUNCH;
 }
@@ -454,6 +494,19 @@ int launch_split256(int mode, int loss, const FusedArgs& a, double* lpart, float
     case PTYCHO_LOSS_POISSON: return launch_t<PTYCHO_LOSS_POISSON>(adj, a, lpart, dp_part, s);
     default: return launch_t<PTYCHO_LOSS_INTENSITY_GRAD>(adj, a, lpart, dp_part, s);
   }
+}
+
+size_t split256_intensity_scratch(int B) {
+  const size_t n = size_t(B < kIntensityChunk ? B : kIntensityChunk);
+  return pty_align_up(n * s256::M * s256::M * sizeof(float2), 256) + pty_align_up(n * sizeof(int2), 256);
+}
+
+int split256_intensity(FusedArgs a, void* scratch, cudaStream_t s) {
+  const size_t n = size_t(a.B < kIntensityChunk ? a.B : kIntensityChunk);
+  a.Eout = static_cast<float2*>(scratch);
+  a.tlb = reinterpret_cast<int2*>(static_cast<char*>(scratch) +
+                                  pty_align_up(n * s256::M * s256::M * sizeof(float2), 256));
+  return s256::launch_intensity(a, s);
 }
 
 int split256_dp_sum(const float2* dp_part, int B, float2* dP, bool accumulate, const double* loss_pat,

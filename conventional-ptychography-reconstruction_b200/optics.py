@@ -186,7 +186,7 @@ def forward_intensity(O: torch.Tensor, P: torch.Tensor, tl: torch.Tensor, batch=
     st = device_status(O.device)
     L = _lib.lib()
     bp = bt.data_ptr() if bt is not None else None
-    if M == N and M in FUSED_PROBE_SIZES:
+    if M == N and M in (64, 128):  # no scratch
         _lib.check(L.ptycho_forward_intensity(O.data_ptr(), H, W, P.data_ptr(), M, N, tl.data_ptr(), F, bp, B,
                                               out.data_ptr(), st.data_ptr(), _stream_handle(O.device)),
                    "ptycho_forward_intensity")

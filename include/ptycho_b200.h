@@ -87,7 +87,8 @@ int ptycho_version(void);
  * accepts any probe shape, Recovery.py:290): shapes the fused kernels do not
  * cover run as gather, mixed-radix row and column DFTs and an intensity
  * pass over a workspace of ptycho_forward_intensity_workspace_size(M, N, B)
- * bytes (256-byte aligned; the fused shapes need none).
+ * bytes (256-byte aligned).  64 and 128 need none; 256 runs row and column
+ * kernels over it, or with a smaller (or no) workspace the cluster kernel.
  * ---------------------------------------------------------------------- */
 int ptycho_forward_intensity(const float* O, int H, int W, const float* P, int M, int N,
                              const int32_t* tl, int F, const int32_t* batch, int B,
