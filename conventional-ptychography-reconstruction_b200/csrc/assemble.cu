@@ -25,8 +25,10 @@
 
 namespace pty {
 
-PTY_DEVI float2 c_xor_sign(float2 a, unsigned m) {
-  return make_float2(__uint_as_float(__float_as_uint(a.x) ^ m), __uint_as_float(__float_as_uint(a.y) ^ m));
+// acc -= a * conj(b)
+PTY_DEVI void c_fnma_conj(float2& acc, float2 a, float2 b) {
+  acc.x = fmaf(-a.x, b.x, fmaf(-a.y, b.y, acc.x));
+  acc.y = fmaf(-a.y, b.x, fmaf(a.x, b.y, acc.y));
 }
 
 __global__ void __launch_bounds__(256) k_loss_total(const double* __restrict__ loss_pat, int B,
@@ -53,11 +55,11 @@ struct AsmArgs {
 
 // dP role: block (p, g), PAIR = 2 adjacent probe pixels per thread (16-byte
 // E' loads; N even) or 1, four patterns' loads in flight
-template <bool SIGNED, int PAIR>
+template <bool SIGNED, int PAIR, int NC>
 PTY_DEVI void dp_block(const AsmArgs& a, int p, int g) {
   __shared__ int last;
-  const int N = a.N;
-  const size_t MN = size_t(a.M) * N;
+  const int N = NC ? NC : a.N;
+  const size_t MN = size_t(NC ? NC : a.M) * N;
   const int idx = PAIR * (p * kPixBlock + threadIdx.x);  // PAIR 2: (x, x + 1) share a row
   const bool in = idx < int(MN);
   const int y = idx / N, x = idx - (idx / N) * N;
@@ -125,15 +127,17 @@ PTY_DEVI void dp_block(const AsmArgs& a, int p, int g) {
   }
 }
 
+// e and p of a partial hit are set under the same tests that guard their use
+#pragma nv_diag_suppress 549
 // dO role: one TW x kTile canvas tile; lane + 32 h = column, warp w = rows w + 8 j
-template <bool SIGNED, int TW>
+template <bool SIGNED, int TW, int NC>
 PTY_DEVI void do_block(const AsmArgs& a, int tile) {
   __shared__ int lb[256];
   __shared__ int2 lc[256];
   __shared__ int wcnt[8];
   static_assert(TW % 32 == 0, "dO tile width");
   constexpr int CH = TW / 32;  // columns per thread
-  const int M = a.M, N = a.N;
+  const int M = NC ? NC : a.M, N = NC ? NC : a.N;
   const size_t MN = size_t(M) * N;
   const int ty0 = (tile / a.ntx) * kTile, tx0 = (tile % a.ntx) * TW;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -171,38 +175,59 @@ PTY_DEVI void do_block(const AsmArgs& a, int tile) {
     for (int i = 0; i < n; ++i) {
       const int bb = lb[i];
       const int2 cc = lc[i];
-      const unsigned sg = SIGNED ? unsigned((cc.x + cc.y) & 1) << 31 : 0u;  // (-1)^(tlY + tlX) of the pattern
+      const bool neg = SIGNED && ((cc.x + cc.y) & 1);  // (-1)^(tlY + tlX) of the pattern
       const int lx = X - cc.y;
       const int ly0 = Y0 - cc.x;
       const float2* Eg = a.Eb + size_t(bb) * MN;
       float2 e[R][CH], p[R][CH];
+      const float2 *eb = Eg + ly0 * N + lx, *pb = a.P + ly0 * N + lx;
       const bool full = cc.x <= ty0 && cc.x + M >= ty0 + kTile && cc.y <= tx0 && cc.y + N >= tx0 + TW;
+      auto add = [&](int j, int h) {
+        if (neg) c_fnma_conj(acc[j][h], e[j][h], p[j][h]);  // uniform
+        else c_fma_conj(acc[j][h], e[j][h], p[j][h]);
+      };
       if (full) {  // uniform: the window covers the whole tile
 #pragma unroll
         for (int j = 0; j < R; ++j)
 #pragma unroll
           for (int h = 0; h < CH; ++h) {
-            const int o = (ly0 + 8 * j) * N + lx + 32 * h;
-            e[j][h] = __ldg(Eg + o);
-            p[j][h] = __ldg(a.P + o);
+            e[j][h] = __ldg(eb + 8 * j * N + 32 * h);
+            p[j][h] = __ldg(pb + 8 * j * N + 32 * h);
           }
-      } else {
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+#pragma unroll
+          for (int h = 0; h < CH; ++h) add(j, h);
+      } else if constexpr (CH == 1) {
+        // a row is in or out for a whole warp, a column for all of a lane's rows:
+        // loads and sums under those two tests (two thirds of the hits of a
+        // 128-wide window cover a 32 x 32 tile only in part)
+        const bool col = unsigned(lx) < unsigned(N);
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+          if (unsigned(ly0 + 8 * j) < unsigned(M) && col) {
+            e[j][0] = __ldg(eb + 8 * j * N);
+            p[j][0] = __ldg(pb + 8 * j * N);
+          }
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+          if (unsigned(ly0 + 8 * j) < unsigned(M) && col) add(j, 0);
+      } else {  // 64-column tiles: zeros outside (tests per column cost 14 registers and a block per SM)
 #pragma unroll
         for (int j = 0; j < R; ++j)
 #pragma unroll
           for (int h = 0; h < CH; ++h) {
-            const int ly = ly0 + 8 * j, lxh = lx + 32 * h;
             e[j][h] = p[j][h] = make_float2(0.f, 0.f);
-            if (lxh >= 0 && lxh < N && ly >= 0 && ly < M) {
-              e[j][h] = __ldg(Eg + ly * N + lxh);
-              p[j][h] = __ldg(a.P + ly * N + lxh);
+            if (unsigned(lx + 32 * h) < unsigned(N) && unsigned(ly0 + 8 * j) < unsigned(M)) {
+              e[j][h] = __ldg(eb + 8 * j * N + 32 * h);
+              p[j][h] = __ldg(pb + 8 * j * N + 32 * h);
             }
           }
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+#pragma unroll
+          for (int h = 0; h < CH; ++h) add(j, h);
       }
-#pragma unroll
-      for (int j = 0; j < R; ++j)
-#pragma unroll
-        for (int h = 0; h < CH; ++h) c_fma_conj(acc[j][h], c_xor_sign(e[j][h], sg), p[j][h]);
     }
     __syncthreads();
   }
@@ -219,20 +244,22 @@ PTY_DEVI void do_block(const AsmArgs& a, int tile) {
     }
 }
 
-// blocks [0, np * ng): dP role; the rest: dO tiles
-template <bool SIGNED, int PAIR, int TW>
-__global__ void __launch_bounds__(256) k_assemble(const AsmArgs a) {
+// blocks [0, np * ng): dP role; the rest: dO tiles.  NC: the window's side when it
+// is known at compile time (the fused sizes), so row offsets are immediates; 0:
+// from the arguments.
+template <bool SIGNED, int PAIR, int TW, int NC>
+__global__ void __launch_bounds__(256, 4) k_assemble(const AsmArgs a) {
   const int bid = blockIdx.x;
   const int ndp = a.np * a.ng;
   if (bid < ndp) {
     const int p = bid % a.np, g = bid / a.np;
-    dp_block<SIGNED, PAIR>(a, p, g);
+    dp_block<SIGNED, PAIR, NC>(a, p, g);
     if (p == 0 && g == 0 && a.loss_total) {
       __syncthreads();
       loss_sum_block(a.loss_pat, a.B, a.loss_total);
     }
   } else {
-    do_block<SIGNED, TW>(a, bid - ndp);
+    do_block<SIGNED, TW, NC>(a, bid - ndp);
   }
 }
 
@@ -265,26 +292,31 @@ int launch_assemble(const float2* Eb, const float2* O, const float2* P, const in
   a.ng = dP ? (B + kGroup - 1) / kGroup : 0;
   // dO tiles 64 columns wide for windows of 256 columns or more (fewer
   // blocks scanning the batch, more pixels per hit: c3 +3 %, c4 +6 %), 32
-  // below (c1: 64 measured 1 % slower)
+  // below (c1: 64 measured 1 % slower).  Compile-time row lengths and signs and
+  // row tests taken out of the inner sums: c1 66.7 -> 63.0, c3 70.1 -> 67.5, c4 429
+  // -> 423 us a step
   const int tw = N >= 256 ? 64 : 32;
   a.ntx = (W + tw - 1) / tw;
   const int ntiles = dO ? a.ntx * ((H + kTile - 1) / kTile) : 0;
   const int grid = a.np * a.ng + ntiles;
   if (!dP && loss_total) k_loss_total<<<1, 256, 0, s>>>(loss_pat, B, loss_total);
-  if (tw == 64) {
-    if (fftshift_sign)
-      k_assemble<true, 2, 64><<<grid, 256, 0, s>>>(a);  // fused path: M = N even
-    else if (pair == 2)
-      k_assemble<false, 2, 64><<<grid, 256, 0, s>>>(a);
+  if (fftshift_sign) {  // fused path: M = N even, 64, 128 or 256
+    if (N == 64)
+      k_assemble<true, 2, 32, 64><<<grid, 256, 0, s>>>(a);
+    else if (N == 128)
+      k_assemble<true, 2, 32, 128><<<grid, 256, 0, s>>>(a);
     else
-      k_assemble<false, 1, 64><<<grid, 256, 0, s>>>(a);
+      k_assemble<true, 2, 64, 256><<<grid, 256, 0, s>>>(a);
+  } else if (tw == 64) {
+    if (pair == 2)
+      k_assemble<false, 2, 64, 0><<<grid, 256, 0, s>>>(a);
+    else
+      k_assemble<false, 1, 64, 0><<<grid, 256, 0, s>>>(a);
   } else {
-    if (fftshift_sign)
-      k_assemble<true, 2, 32><<<grid, 256, 0, s>>>(a);
-    else if (pair == 2)
-      k_assemble<false, 2, 32><<<grid, 256, 0, s>>>(a);
+    if (pair == 2)
+      k_assemble<false, 2, 32, 0><<<grid, 256, 0, s>>>(a);
     else
-      k_assemble<false, 1, 32><<<grid, 256, 0, s>>>(a);
+      k_assemble<false, 1, 32, 0><<<grid, 256, 0, s>>>(a);
   }
   return cudaGetLastError() == cudaSuccess ? PTYCHO_OK : PTYCHO_ERR_LAUNCH;
 }
