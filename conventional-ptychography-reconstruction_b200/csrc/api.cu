@@ -54,10 +54,11 @@ static int check_common(const float* O, int H, int W, const float* P, int M, int
   return PTYCHO_OK;
 }
 
+// the kernels that need no scratch beyond E': M = 64 and 128 in one SM, or a cluster
+// per pattern (small batches; M = 256)
 static int launch_fused(int M, int mode, int loss, const FusedArgs& a, cudaStream_t s) {
-  if (M == 64) return launch_fused_64(mode, loss, a, s);
-  if (M == 128) return launch_fused_128(mode, loss, a, s);
-  return launch_fused_256(mode, loss, a, s);
+  if (M == 256 || a.B <= small_batch_max(M, mode, loss)) return launch_small(M, mode, loss, a, s);
+  return M == 64 ? launch_fused_64(mode, loss, a, s) : launch_fused_128(mode, loss, a, s);
 }
 
 static FusedArgs make_args(const float* O, int H, int W, const float* P, const int32_t* tl,
@@ -114,8 +115,9 @@ int ptycho_forward_intensity(const float* O, int H, int W, const float* P, int M
 
 size_t ptycho_forward_intensity_workspace_size(int M, int N, int B) {
   if (B < 0 || !supported_probe(M, N)) return 0;
-  if (M == 256 && N == 256) return split256_intensity_scratch(B);  // 256 bytes will do: the cluster kernel
-  if (fused_probe(M, N)) return 256;                               // the fused kernels need none
+  if (M == 256 && N == 256 && B > small_batch_max(M, MODE_INTENSITY, 0))
+    return split256_intensity_scratch(B);  // with less, the cluster kernel
+  if (fused_probe(M, N)) return 256;       // the fused kernels need none
   return pty_align_up(size_t(B) * M * N * sizeof(float2), 256);
 }
 
@@ -128,7 +130,8 @@ int ptycho_forward_intensity_ws(const float* O, int H, int W, const float* P, in
   if (B == 0) return PTYCHO_OK;
   if (!I_out) return PTYCHO_ERR_INVALID_ARG;
   if (fused_probe(M, N)) {
-    if (M == 256 && workspace && workspace_bytes >= split256_intensity_scratch(B) && pty_aligned(workspace, 256)) {
+    if (M == 256 && B > small_batch_max(M, MODE_INTENSITY, 0) && workspace &&
+        workspace_bytes >= split256_intensity_scratch(B) && pty_aligned(workspace, 256)) {
       FusedArgs a = make_args(O, H, W, P, tl, nullptr, F, batch, B, status_out);
       a.I_out = I_out;
       return split256_intensity(a, workspace, reinterpret_cast<cudaStream_t>(stream));
@@ -184,7 +187,7 @@ int ptycho_fwd_adj(const float* O, int H, int W, const float* P, int M, int N, c
   const bool adj = dO || dP;
   const bool fused = fused_probe(M, N);
   const int mode = adj ? MODE_ADJ : MODE_LOSS;
-  if (fused && M == 256 && split256_supported(mode, loss_type)) {
+  if (fused && M == 256 && split256_supported(mode, loss_type) && B > small_batch_max(M, mode, loss_type)) {
     // the line-DFT kernels use E' as their scratch in both modes; on large
     // batches the probe gradient comes out of the inverse-row kernel
     a.Eout = Ews;

@@ -363,10 +363,9 @@ int launch_fused_m(int mode, int loss, const FusedArgs& a, cudaStream_t s) {
   }
 }
 
-// defined in fused_m64.cu / fused_m128.cu / fused256.cu (4-CTA cluster per pattern)
+// defined in fused_m64.cu / fused_m128.cu
 int launch_fused_64(int mode, int loss, const FusedArgs& a, cudaStream_t s);
 int launch_fused_128(int mode, int loss, const FusedArgs& a, cudaStream_t s);
-int launch_fused_256(int mode, int loss, const FusedArgs& a, cudaStream_t s);
 
 // split256.cu: M = 256 as three line-DFT kernels (smooth-L1, Poisson and the
 // intensity-gradient losses in MODE_LOSS / MODE_ADJ); a.Eout is the scratch,
@@ -390,12 +389,30 @@ int split256_dp_sum(const float2* dp_part, int B, float2* dP, bool accumulate, c
 // split256_intensity_scratch(B) bytes, 256-byte aligned, for up to
 // kIntensityChunk patterns at a time (512 KB each).  Measured for 512 patterns:
 // chunks of 64, 128, 256, 512 took 198, 190, 169, 157 us (fuller waves win over
-// keeping a chunk in L2); the cluster kernel, which needs no scratch, 314 us.
+// keeping a chunk in L2); the cluster kernel without scratch 250 us.
 #ifndef PTY_S256_INTENSITY_CHUNK
 #define PTY_S256_INTENSITY_CHUNK 512
 #endif
 constexpr int kIntensityChunk = PTY_S256_INTENSITY_CHUNK;
 size_t split256_intensity_scratch(int B);
 int split256_intensity(FusedArgs a, void* scratch, cudaStream_t s);
+
+// cluster_small.cu: a pattern per cluster of M / 16 CTAs, any mode and loss
+int launch_small(int M, int mode, int loss, const FusedArgs& a, cudaStream_t s);
+
+// Largest batch that the cluster kernel takes: where a pattern per SM (or, at M =
+// 256, the line kernels' three launches) leaves SMs idle.  Measured, us a step on a
+// 1024^2 object, cluster kernel against the other: M = 64, 10 patterns 19.0 : 22.9,
+// 12 to 30 equal, 37 22.9 : 21.5; M = 128, 10 23.0 : 33.2, 64 29.1 : 34.7, 80
+// 36.0 : 35.3; M = 256, 4 23.2 : 24.9, 5 equal, 16 37.3 : 31.2.  FD loss: M = 64 never
+// better (10 25.0 : 24.6), M = 128 10 27.1 : 49.8, 100 50.0 : 53.8, 148 64.6 : 57.9,
+// M = 256 always (10 33.5 : 78.4, 200 347 : 532 for a 4-CTA cluster kernel).
+// M = 256 intensities: 20 16.2 : 18.7, 64 37.3 : 24.0.
+inline int small_batch_max(int M, int mode, int loss) {
+  const bool fd = mode != MODE_INTENSITY && loss == PTYCHO_LOSS_FD;
+  if (M == 64) return fd ? 0 : 16;
+  if (M == 128) return fd ? 96 : 64;
+  return fd ? 0x7fffffff : (mode == MODE_INTENSITY ? 24 : 4);
+}
 
 }  // namespace pty
