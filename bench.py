@@ -268,7 +268,7 @@ def side_workload(pkg, key, dev, steps=30, warmup=5, n_check=8):
                                                              / np.abs(ref["loss"]))),
                 "dO_rel_err": rn(dO.cpu().numpy(), ref["dO"]),
                 "dP_rel_err": rn(dP.cpu().numpy(), ref["dP"])},
-            "note": "one CUDA-graph launch per minibatch (k_fused256 + k_assemble), L2 flushed before "
+            "note": "one CUDA-graph launch per minibatch (row, column and inverse-row kernels + k_assemble), L2 flushed before "
                     "each step; clocks not sampled for these steps"}
 
 

@@ -1,7 +1,8 @@
 // split256.cu -- forward / loss / adjoint for 256 x 256 probes as three
 // line-DFT kernels over the E' workspace (smooth-L1, Poisson and the
-// intensity-gradient losses; the FD loss and MODE_INTENSITY keep the
-// cluster kernel of fused256.cu).
+// intensity-gradient losses), and intensities over a scratch of their own.  The FD
+// loss, small batches and intensities without scratch run the cluster kernel of
+// cluster_small.cu.
 //
 // Same contract as the fused kernels (fused.cuh): per pattern b of the batch,
 //   A  rows:     X_b[y][.] = DFT_x( (-1)^(x+y) P[y][x] O[tlY+y][tlX+x] )

@@ -80,9 +80,8 @@ int ptycho_version(void);
  * batched: for b < B, with f = batch[b],
  *   I_out[b] = | fftshift( fft2( P * O[tlY_f : tlY_f+M, tlX_f : tlX_f+N] ) ) |^2
  * O [H][W] complex64, P [M][N] complex64, I_out [B][M][N] float32.
- * ptycho_forward_intensity takes M == N in {64, 128, 256} (the fused
- * kernels; 256: one 4-CTA thread-block cluster per pattern) and needs no
- * scratch memory; other shapes return PTYCHO_ERR_UNSUPPORTED_SIZE.
+ * ptycho_forward_intensity takes M == N in {64, 128, 256} (a pattern per SM,
+ * or per thread-block cluster of M / 16 CTAs) and needs no scratch memory; other shapes return PTYCHO_ERR_UNSUPPORTED_SIZE.
  * ptycho_forward_intensity_ws takes any 1 <= M, N <= 4096 (the reference
  * accepts any probe shape, Recovery.py:290): shapes the fused kernels do not
  * cover run as gather, mixed-radix row and column DFTs and an intensity
@@ -119,10 +118,12 @@ int ptycho_forward_intensity_ws(const float* O, int H, int W, const float* P, in
  * Probes: M == N in {64, 128} run the fused kernels; M == N == 256 runs
  * three line-DFT kernels over the workspace (smooth-L1, Poisson and the
  * intensity-gradient code; batches of 192 or more also take dP from the
- * inverse-row kernel) or, for the FD loss, one 4-CTA cluster per pattern;
- * any other 1 <= M, N <= 4096 (non-square, odd, 96, 192, ...) runs the
- * general path: the same losses and gradients through workspace passes
- * (gather, row and column DFTs of any length, loss, inverse DFTs), then the
+ * inverse-row kernel); small batches of the three, and the FD loss at 256, run
+ * one thread-block cluster of M / 16 CTAs per pattern; any other
+ * 1 <= M, N <= 4096 (non-square, odd, 96, 192, ...) runs the general path: the
+ * same losses and gradients through three workspace passes (gather and row
+ * DFTs of any length, column DFTs with the loss and their inverse, inverse
+ * row DFTs), then the
  * same assembly.
  * ---------------------------------------------------------------------- */
 size_t ptycho_fwd_adj_workspace_size(int H, int W, int M, int N, int B);
