@@ -127,8 +127,8 @@ _torchext_tried = False
 
 
 def torchext():
-    """The fused loss's C++ autograd node (csrc/torch_ext.cpp) bound to this
-    process's library, or None when it is not built."""
+    """The C++ autograd nodes (csrc/torch_ext.cpp) bound to this process's
+    library, or None when they are not built."""
     global _torchext, _torchext_tried
     if _torchext_tried:
         return _torchext
@@ -143,6 +143,12 @@ def torchext():
                 addr = lambda f: ctypes.cast(f, ctypes.c_void_p).value  # noqa: E731
                 m.bind(addr(L.ptycho_fwd_adj), addr(L.ptycho_scale_pair), addr(L.ptycho_fwd_adj_workspace_size),
                        addr(L.ptycho_status_string))
+                m.bind_inr([addr(f) for f in (L.ptycho_cmlp_pack, L.ptycho_cmlp_forward, L.ptycho_cmlp_forward_planar,
+                                              L.ptycho_cmlp_backward, L.ptycho_cmlp_backward_planar,
+                                              L.ptycho_cmlp_backward_workspace_size, L.ptycho_fourier_upsample,
+                                              L.ptycho_fourier_upsample_adjoint,
+                                              L.ptycho_fourier_upsample_workspace_size)],
+                           int(L.ptycho_cmlp_packed_bytes()), int(L.ptycho_cmlp_grad_floats()))
             _torchext = m
             _torchext_tried = True
     return _torchext

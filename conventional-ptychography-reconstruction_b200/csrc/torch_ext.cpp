@@ -1,4 +1,5 @@
-// torch_ext.cpp -- the fused loss as a C++ torch autograd function over the C ABI.
+// torch_ext.cpp -- the fused loss, the complex MLP and the Fourier upsampling as C++
+// torch autograd functions over the C ABI.
 //
 // fused_loss (Recovery.py:288-307, backward at :316) needs an autograd node
 // whose backward scales the gradients the forward already computed.  Written
@@ -7,6 +8,9 @@
 // forward calls ptycho_fwd_adj, the backward ptycho_scale_pair, both through
 // addresses handed over by `bind` (taken from the ctypes handle of
 // libptycho_b200.so, so there is one copy of the library in the process).
+// The MLP's Python Function converted eleven parameters to views, and as many
+// gradients back, on every call: 327 us of host work for a forward and backward, the
+// time of 600,000 coordinates on the GPU, EXT_FIGURES here.
 // No computation happens here; a non-zero library status raises RuntimeError,
 // bad arguments raise ValueError / TypeError as the Python path does.
 #include <ATen/cuda/CUDAContext.h>
@@ -31,11 +35,25 @@ typedef int (*scale_pair_fn)(const float*, float*, long long, const float*, floa
                              void*);
 typedef size_t (*ws_size_fn)(int, int, int, int, int);
 typedef const char* (*status_string_fn)(int);
+typedef int (*cmlp_pack_fn)(const float*, const float*, const float*, const float*, const float*, const float*,
+                            const float*, const float*, const float*, const float*, const float*, void*, void*);
+typedef int (*cmlp_fwd_fn)(const void*, const float*, int, float*, int32_t*, void*);
+typedef int (*cmlp_bwd_fn)(const void*, const float*, const float*, int, float*, float*, float*, void*, size_t,
+                           int32_t*, void*);
+typedef int (*upsample_fn)(const float*, int, int, int, float*, void*, size_t, void*);
 
 fwd_adj_fn g_fwd_adj = nullptr;
 scale_pair_fn g_scale_pair = nullptr;
 ws_size_fn g_ws_size = nullptr;
 status_string_fn g_status_string = nullptr;
+
+cmlp_pack_fn g_cmlp_pack = nullptr;
+cmlp_fwd_fn g_cmlp_fwd[2] = {nullptr, nullptr};  // [N][32] features, feature-major
+cmlp_bwd_fn g_cmlp_bwd[2] = {nullptr, nullptr};
+size_t (*g_cmlp_bwd_ws)(int) = nullptr;
+int64_t g_cmlp_packed_bytes = 0, g_cmlp_grad_floats = 0;
+upsample_fn g_upsample[2] = {nullptr, nullptr};  // forward, adjoint
+size_t (*g_upsample_ws)(int, int, int) = nullptr;
 
 constexpr int64_t kMaxProbeDim = 4096;
 
@@ -173,6 +191,166 @@ Tensor fused_loss(const Tensor& O, const Tensor& P, const Tensor& tl_in, const T
   return loss;
 }
 
+// ---------------------------------------------------------------------------
+// Complex MLP (cmlp.py): parameters in the order omega_0, weight, bias of three
+// layers, output weight and bias.
+// ---------------------------------------------------------------------------
+constexpr int kCmlpParams = 11;
+
+// a parameter's values as contiguous float32 (complex64 as pairs); no copy when
+// that is what it is
+Tensor floats_of(const Tensor& p) {
+  Tensor t = p.detach();
+  if (t.is_complex()) t = torch::view_as_real(t.resolve_conj().contiguous());
+  return t.contiguous().to(torch::kFloat32);
+}
+
+// [N, 32] float32 view of a feature-major [32, N] buffer (the encoder's output)
+bool is_planar(const Tensor& x) {
+  return x.dim() == 2 && x.size(1) == 32 && x.size(0) > 1 && x.stride(0) == 1 && x.stride(1) == x.size(0);
+}
+
+class Cmlp : public torch::autograd::Function<Cmlp> {
+ public:
+  // x [N, 32] float32, feature-major or contiguous (checked by the caller)
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& om1, const Tensor& W1, const Tensor& b1,
+                        const Tensor& om2, const Tensor& W2, const Tensor& b2, const Tensor& om3, const Tensor& W3,
+                        const Tensor& b3, const Tensor& Wo, const Tensor& bo, const Tensor& status, int* rc) {
+    const Tensor ps[kCmlpParams] = {W1, b1, om1, W2, b2, om2, W3, b3, om3, Wo, bo};  // ptycho_cmlp_pack's order
+    Tensor f[kCmlpParams];
+    for (int i = 0; i < kCmlpParams; ++i) f[i] = floats_of(ps[i]);
+    void* s = current_stream(x);
+    const int64_t N = x.size(0);
+    Tensor packed = torch::empty({g_cmlp_packed_bytes}, x.options().dtype(torch::kUInt8));
+    Tensor y = torch::empty({N, 1}, x.options().dtype(torch::kComplexFloat));
+    const int planar = is_planar(x);
+    *rc = g_cmlp_pack(fptr<const float>(f[0]), fptr<const float>(f[1]), fptr<const float>(f[2]), fptr<const float>(f[3]),
+                      fptr<const float>(f[4]), fptr<const float>(f[5]), fptr<const float>(f[6]), fptr<const float>(f[7]),
+                      fptr<const float>(f[8]), fptr<const float>(f[9]), fptr<const float>(f[10]), packed.data_ptr(), s);
+    if (*rc == 0)
+      *rc = g_cmlp_fwd[planar](packed.data_ptr(), fptr<const float>(x), int(N), fptr<float>(y), fptr<int32_t>(status), s);
+    ctx->save_for_backward({x, packed});
+    ctx->saved_data["status"] = status;  // not a saved variable: reading it out clears it in place
+    const Tensor in[kCmlpParams] = {om1, W1, b1, om2, W2, b2, om3, W3, b3, Wo, bo};
+    std::vector<int64_t> types;
+    std::vector<c10::IValue> sizes;
+    for (const Tensor& p : in) {
+      types.push_back(int64_t(p.scalar_type()));
+      sizes.emplace_back(p.sizes().vec());
+    }
+    ctx->saved_data["types"] = types;
+    ctx->saved_data["sizes"] = c10::ivalue::Tuple::create(sizes);
+    return y;
+  }
+
+  static tensor_list backward(AutogradContext* ctx, tensor_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &packed = saved[1];
+    const Tensor status = ctx->saved_data["status"].toTensor();
+    c10::cuda::CUDAGuard guard(x.device());
+    void* s = current_stream(x);
+    const int64_t N = x.size(0);
+    const Tensor gy = grads[0].reshape({N}).to(torch::kComplexFloat).resolve_conj().contiguous();
+    const int planar = is_planar(x);
+    Tensor grad = torch::empty({g_cmlp_grad_floats}, x.options());
+    Tensor ws = torch::empty({int64_t(g_cmlp_bwd_ws(int(N)))}, x.options().dtype(torch::kUInt8));
+    // the features' gradient goes back in their own layout
+    Tensor gx;
+    if (ctx->needs_input_grad(0)) gx = planar ? torch::empty({32, N}, x.options()) : torch::empty({N, 32}, x.options());
+    check(g_cmlp_bwd[planar](packed.data_ptr(), fptr<const float>(x), fptr<const float>(gy), int(N), fptr<float>(gx),
+                             fptr<float>(grad), nullptr, ws.data_ptr(), size_t(ws.numel()), fptr<int32_t>(status), s),
+          planar ? "ptycho_cmlp_backward_planar" : "ptycho_cmlp_backward");
+    tensor_list out(1 + kCmlpParams + 2);
+    if (gx.defined()) out[0] = planar ? gx.t() : gx;
+    // offset and length of each parameter's gradient in the blob (floats), complex or not
+    struct Part {
+      int64_t off, n;
+      bool cplx;
+    };
+    static constexpr Part parts[kCmlpParams] = {{1056, 1, false},   {0, 1024, false},   {1024, 32, false}, {3170, 1, false},
+                                                {1058, 2048, true}, {3106, 64, true},   {5284, 1, false},  {3172, 2048, true},
+                                                {5220, 64, true},   {5286, 64, true},   {5350, 2, true}};
+    const auto types = ctx->saved_data["types"].toIntVector();
+    const auto sizes = ctx->saved_data["sizes"].toTuple();
+    for (int i = 0; i < kCmlpParams; ++i) {
+      if (!ctx->needs_input_grad(1 + i)) continue;
+      Tensor g = grad.narrow(0, parts[i].off, parts[i].n);
+      if (parts[i].cplx) g = torch::view_as_complex(g.view({-1, 2}));
+      out[1 + i] = g.reshape(sizes->elements()[i].toIntVector()).to(torch::ScalarType(types[i]));
+    }
+    return out;
+  }
+};
+
+// (y [N, 1] complex64, library status of the forward)
+std::pair<Tensor, int> cmlp(const Tensor& x_in, const std::vector<Tensor>& p, const Tensor& status) {
+  TORCH_CHECK(g_cmlp_pack && g_cmlp_bwd_ws, "bind_inr() was not called");
+  TORCH_CHECK_VALUE(x_in.is_cuda(), "features must be a CUDA tensor (there is no CPU path)");
+  TORCH_CHECK_VALUE(p.size() == size_t(kCmlpParams), "the MLP has eleven parameters");
+  c10::cuda::CUDAGuard guard(x_in.device());
+  Tensor x = x_in.to(torch::kFloat32);
+  if (!is_planar(x)) x = x.contiguous();
+  int rc = 0;
+  Tensor y = Cmlp::apply(x, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], p[8], p[9], p[10], status, &rc);
+  return {y, rc};
+}
+
+// ---------------------------------------------------------------------------
+// Fourier upsampling (resample.py)
+// ---------------------------------------------------------------------------
+class Upsample : public torch::autograd::Function<Upsample> {
+ public:
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, int64_t s, int* rc) {
+    const Tensor xc = x.to(torch::kComplexFloat).resolve_conj().contiguous();
+    const int64_t h = x.size(0), w = x.size(1);
+    Tensor y = torch::empty({h * s, w * s}, xc.options());
+    Tensor ws = torch::empty({int64_t(g_upsample_ws(int(h), int(w), int(s)))}, xc.options().dtype(torch::kUInt8));
+    *rc = g_upsample[0](fptr<const float>(xc), int(h), int(w), int(s), fptr<float>(y), ws.data_ptr(), size_t(ws.numel()),
+                        current_stream(xc));
+    ctx->saved_data["h"] = h;
+    ctx->saved_data["w"] = w;
+    ctx->saved_data["s"] = s;
+    return y;
+  }
+
+  static tensor_list backward(AutogradContext* ctx, tensor_list grads) {
+    const int64_t h = ctx->saved_data["h"].toInt(), w = ctx->saved_data["w"].toInt(), s = ctx->saved_data["s"].toInt();
+    const Tensor g = grads[0].to(torch::kComplexFloat).resolve_conj().contiguous();
+    c10::cuda::CUDAGuard guard(g.device());
+    Tensor gx = torch::empty({h, w}, g.options());
+    Tensor ws = torch::empty({int64_t(g_upsample_ws(int(h), int(w), int(s)))}, g.options().dtype(torch::kUInt8));
+    check(g_upsample[1](fptr<const float>(g), int(h), int(w), int(s), fptr<float>(gx), ws.data_ptr(), size_t(ws.numel()),
+                        current_stream(g)),
+          "ptycho_fourier_upsample_adjoint");
+    return {gx, Tensor(), Tensor()};
+  }
+};
+
+// (y [h s, w s] complex64, library status); the caller has checked shape and scale
+std::pair<Tensor, int> upsample(const Tensor& x, int64_t s) {
+  TORCH_CHECK(g_upsample[0] && g_upsample_ws, "bind_inr() was not called");
+  TORCH_CHECK_VALUE(x.is_cuda(), "x must be a CUDA tensor (there is no CPU path)");
+  c10::cuda::CUDAGuard guard(x.device());
+  int rc = 0;
+  Tensor y = Upsample::apply(x, s, &rc);
+  return {y, rc};
+}
+
+void bind_inr(const std::vector<int64_t>& a, int64_t packed_bytes, int64_t grad_floats) {
+  TORCH_CHECK(a.size() == 9, "bind_inr: nine addresses");
+  g_cmlp_pack = reinterpret_cast<cmlp_pack_fn>(a[0]);
+  g_cmlp_fwd[0] = reinterpret_cast<cmlp_fwd_fn>(a[1]);
+  g_cmlp_fwd[1] = reinterpret_cast<cmlp_fwd_fn>(a[2]);
+  g_cmlp_bwd[0] = reinterpret_cast<cmlp_bwd_fn>(a[3]);
+  g_cmlp_bwd[1] = reinterpret_cast<cmlp_bwd_fn>(a[4]);
+  g_cmlp_bwd_ws = reinterpret_cast<size_t (*)(int)>(a[5]);
+  g_upsample[0] = reinterpret_cast<upsample_fn>(a[6]);
+  g_upsample[1] = reinterpret_cast<upsample_fn>(a[7]);
+  g_upsample_ws = reinterpret_cast<size_t (*)(int, int, int)>(a[8]);
+  g_cmlp_packed_bytes = packed_bytes;
+  g_cmlp_grad_floats = grad_floats;
+}
+
 // the cached workspace of the current stream of `like`'s device, at least `bytes` long
 Tensor workspace(const Tensor& like, int64_t bytes) {
   TORCH_CHECK_VALUE(like.is_cuda() && bytes >= 0, "workspace needs a CUDA tensor and a size");
@@ -185,4 +363,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("bind", &bind, "bind(fwd_adj, scale_pair, workspace_size, status_string) function addresses");
   m.def("fused_loss", &fused_loss, "fused forward + loss + adjoint as one autograd node");
   m.def("workspace", &workspace, "the per-stream ptycho_fwd_adj workspace");
+  m.def("bind_inr", &bind_inr, "addresses of the MLP and upsampling entry points");
+  m.def("cmlp", &cmlp, "complex MLP as one autograd node: (y, status)");
+  m.def("upsample", &upsample, "Fourier upsampling as one autograd node: (y, status)");
 }

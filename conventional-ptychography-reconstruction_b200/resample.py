@@ -15,7 +15,7 @@ from __future__ import annotations
 
 import torch
 
-from . import _lib
+from . import _lib, optics
 
 MAX_LEN = 8192
 
@@ -36,7 +36,7 @@ class _FourierUpsample(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, s: int):
         h, w = x.shape
-        xc = x.to(torch.complex64).contiguous()
+        xc = x.to(torch.complex64).resolve_conj().contiguous()
         y = torch.empty((h * s, w * s), dtype=torch.complex64, device=x.device)
         ws, n = _workspace(h, w, s, x.device)
         _lib.check(_lib.lib().ptycho_fourier_upsample(
@@ -48,7 +48,7 @@ class _FourierUpsample(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gy):
         h, w, s = ctx.shape
-        g = gy.to(torch.complex64).contiguous()
+        g = gy.to(torch.complex64).resolve_conj().contiguous()
         gx = torch.empty((h, w), dtype=torch.complex64, device=g.device)
         ws, n = _workspace(h, w, s, g.device)
         _lib.check(_lib.lib().ptycho_fourier_upsample_adjoint(
@@ -63,4 +63,9 @@ def fourier_upsample(x: torch.Tensor, s: int) -> torch.Tensor:
         raise ValueError("x must be a CUDA tensor (there is no CPU path)")
     if x.dim() != 2 or not supported(x.shape[0], x.shape[1], s):
         raise ValueError(f"unsupported shape {tuple(x.shape)} with scale {s}")
+    ext = _lib.torchext() if optics.USE_TORCHEXT else None
+    if ext is not None:  # the C++ autograd node: the same library calls
+        y, rc = ext.upsample(x, int(s))
+        _lib.check(rc, "ptycho_fourier_upsample")
+        return y
     return _FourierUpsample.apply(x, int(s))
