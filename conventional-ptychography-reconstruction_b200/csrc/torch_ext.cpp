@@ -10,7 +10,7 @@
 // libptycho_b200.so, so there is one copy of the library in the process).
 // The MLP's Python Function converted eleven parameters to views, and as many
 // gradients back, on every call: 327 us of host work for a forward and backward, the
-// time of 600,000 coordinates on the GPU, EXT_FIGURES here.
+// time of 600,000 coordinates on the GPU; 204 us here (an upsampling 107, now 62).
 // No computation happens here; a non-zero library status raises RuntimeError,
 // bad arguments raise ValueError / TypeError as the Python path does.
 #include <ATen/cuda/CUDAContext.h>
