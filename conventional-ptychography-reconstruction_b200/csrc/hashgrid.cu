@@ -35,6 +35,8 @@ struct LevelTable {
   int dense[kMaxLevels];
   int levels;
   int total;  // total entries
+  int ndense; // levels 0 .. ndense - 1 are dense, the rest hashed (n = 2^log2_hashmap_size)
+  int whole;  // every scale is below 2^20
 };
 
 static int make_levels(int n_levels, int log2_T, int base_res, float per_level_scale, LevelTable* L) {
@@ -43,6 +45,8 @@ static int make_levels(int n_levels, int log2_T, int base_res, float per_level_s
     return PTYCHO_ERR_INVALID_ARG;
   const long long T = 1ll << log2_T;
   long long off = 0;
+  L->ndense = 0;
+  L->whole = 1;
   for (int l = 0; l < n_levels; ++l) {
     const double scale = double(base_res) * pow(double(per_level_scale), double(l)) - 1.0;
     const long long res = (long long)ceil(scale) + 1;
@@ -54,6 +58,8 @@ static int make_levels(int n_levels, int log2_T, int base_res, float per_level_s
     L->n[l] = (int)n;
     L->offset[l] = (int)off;
     L->dense[l] = dn <= T;
+    if (dn <= T) L->ndense = l + 1;  // res never falls with l
+    if (!(scale < 1048576.0)) L->whole = 0;
     off += n;
   }
   L->levels = n_levels;
@@ -77,82 +83,90 @@ PTY_DEVI int corner_entry(const LevelTable& L, int l, int cx, int cy) {
   return L.offset[l] + int(e);
 }
 
-// one thread per coordinate, all levels: adjacent threads hold adjacent
-// coordinates, so each level's corner gathers of a warp fall on neighbouring
-// cells, and a thread writes its n_levels x 2 features contiguously
+// the bilinear value from the four corners
+PTY_DEVI float2 bilinear(float2 t00, float2 t10, float2 t01, float2 t11, float fx, float fy) {
+  const float w00 = (1.f - fx) * (1.f - fy), w10 = fx * (1.f - fy), w01 = (1.f - fx) * fy, w11 = fx * fy;
+  return make_float2(fmaf(w11, t11.x, fmaf(w01, t01.x, fmaf(w10, t10.x, w00 * t00.x))),
+                     fmaf(w11, t11.y, fmaf(w01, t01.y, fmaf(w10, t10.y, w00 * t00.y))));
+}
+
+// floor and fraction of 0 <= p < 2^22 in two adds: p + 1.5 * 2^23 rounded down
+// holds floor(p) in its last bits (floorf and the conversion to int would both
+// run at a quarter of the rate)
+PTY_DEVI int cell_of(float p, float& f) {
+  const float t = __fadd_rd(p, 12582912.f);
+  f = p - (t - 12582912.f);
+  return __float_as_int(t) - 0x4B400000;
+}
+
+// Forward: one thread per coordinate, all levels, so the coordinate is read once
+// and the corner gathers of a warp (adjacent coordinates) fall on neighbouring
+// cells.  PLANAR writes features [2L][N] (every store coalesced), else [N][2L]
+// (a thread's features contiguous).  Bound by instructions: with the floors by
+// adds, the dense and hashed levels in loops of their own (one compare covers a
+// dense cell's four corners, the modulo only where the last is past the level's
+// end), 1024^2 coordinates and 16 levels take 51 us
+// (57 with floorf and corner_entry; 1.9 TB/s; two or four coordinates per thread
+// measured 3 and 15 us more).  The short loops hold for coordinates in [0, 1] and scales below 2^20; any other
+// coordinate takes the general one, bitwise the same where both apply.
+template <bool PLANAR>
 __global__ void __launch_bounds__(256) k_hash_fwd(const float2* __restrict__ coords, int N,
                                                   const float2* __restrict__ table, const LevelTable L,
-                                                  float2* __restrict__ feat) {
+                                                  float* __restrict__ feat) {
   const int n = blockIdx.x * 256 + threadIdx.x;
   if (n >= N) return;
   const float2 x = __ldg(coords + n);
-  float2* out = feat + (long long)n * L.levels;
+  float* out = PLANAR ? feat + n : feat + (size_t)n * (2 * L.levels);
+  const size_t plane = size_t(N);
+  auto put = [&](float2 o) {
+    if constexpr (PLANAR) {
+      out[0] = o.x;
+      out[plane] = o.y;
+      out += 2 * plane;
+    } else {
+      *reinterpret_cast<float2*>(out) = o;
+      out += 2;
+    }
+  };
+  if (L.whole && x.x >= 0.f && x.x <= 1.f && x.y >= 0.f && x.y <= 1.f) {
+    int l = 0;
 #pragma unroll 4
-  for (int l = 0; l < L.levels; ++l) {
-    const float s = L.scale[l];
-    const float px = fmaf(x.x, s, 0.5f), py = fmaf(x.y, s, 0.5f);
-    const float gx = floorf(px), gy = floorf(py);
-    const float fx = px - gx, fy = py - gy;
-    const int ix = int(gx), iy = int(gy);
-    const float2 t00 = __ldg(table + corner_entry(L, l, ix, iy));
-    const float2 t10 = __ldg(table + corner_entry(L, l, ix + 1, iy));
-    const float2 t01 = __ldg(table + corner_entry(L, l, ix, iy + 1));
-    const float2 t11 = __ldg(table + corner_entry(L, l, ix + 1, iy + 1));
-    const float w00 = (1.f - fx) * (1.f - fy), w10 = fx * (1.f - fy), w01 = (1.f - fx) * fy, w11 = fx * fy;
-    float2 o;
-    o.x = fmaf(w11, t11.x, fmaf(w01, t01.x, fmaf(w10, t10.x, w00 * t00.x)));
-    o.y = fmaf(w11, t11.y, fmaf(w01, t01.y, fmaf(w10, t10.y, w00 * t00.y)));
-    out[l] = o;
+    for (; l < L.ndense; ++l) {
+      const float s = L.scale[l];
+      float fx, fy;
+      const int ix = cell_of(fmaf(x.x, s, 0.5f), fx), iy = cell_of(fmaf(x.y, s, 0.5f), fy);
+      const uint32_t n_l = uint32_t(L.n[l]), r = uint32_t(L.res[l]);
+      uint32_t e00 = uint32_t(ix) + uint32_t(iy) * r, e10 = e00 + 1, e01 = e00 + r, e11 = e01 + 1;
+      if (e11 >= n_l) {
+        e00 %= n_l;
+        e10 %= n_l;
+        e01 %= n_l;
+        e11 %= n_l;
+      }
+      const float2* T = table + L.offset[l];
+      put(bilinear(__ldg(T + e00), __ldg(T + e10), __ldg(T + e01), __ldg(T + e11), fx, fy));
+    }
+#pragma unroll 4
+    for (; l < L.levels; ++l) {
+      const float s = L.scale[l];
+      float fx, fy;
+      const int ix = cell_of(fmaf(x.x, s, 0.5f), fx), iy = cell_of(fmaf(x.y, s, 0.5f), fy);
+      const uint32_t m = uint32_t(L.n[l]) - 1, h0 = uint32_t(iy) * kPrimeY, h1 = h0 + kPrimeY;
+      const uint32_t c0 = uint32_t(ix), c1 = c0 + 1;
+      const float2* T = table + L.offset[l];
+      put(bilinear(__ldg(T + ((c0 ^ h0) & m)), __ldg(T + ((c1 ^ h0) & m)), __ldg(T + ((c0 ^ h1) & m)),
+                   __ldg(T + ((c1 ^ h1) & m)), fx, fy));
+    }
+    return;
   }
-}
-
-// feature-major forward: blockIdx.y = level, one thread per coordinate; writes
-// features [2L][N] (feature 2l + c of coordinate n at (2l + c) * N + n), so
-// every store is coalesced and the grid has L times the threads
-__global__ void __launch_bounds__(256) k_hash_fwd_planar(const float2* __restrict__ coords, int N,
-                                                         const float2* __restrict__ table, const LevelTable L,
-                                                         float* __restrict__ feat) {
-  const int n = blockIdx.x * 256 + threadIdx.x;
-  const int l = blockIdx.y;
-  if (n >= N) return;
-  const float2 x = __ldg(coords + n);
-  const float s = L.scale[l];
-  const float px = fmaf(x.x, s, 0.5f), py = fmaf(x.y, s, 0.5f);
-  const float gx = floorf(px), gy = floorf(py);
-  const float fx = px - gx, fy = py - gy;
-  const int ix = int(gx), iy = int(gy);
-  const float2 t00 = __ldg(table + corner_entry(L, l, ix, iy));
-  const float2 t10 = __ldg(table + corner_entry(L, l, ix + 1, iy));
-  const float2 t01 = __ldg(table + corner_entry(L, l, ix, iy + 1));
-  const float2 t11 = __ldg(table + corner_entry(L, l, ix + 1, iy + 1));
-  const float w00 = (1.f - fx) * (1.f - fy), w10 = fx * (1.f - fy), w01 = (1.f - fx) * fy, w11 = fx * fy;
-  feat[size_t(2 * l) * N + n] = fmaf(w11, t11.x, fmaf(w01, t01.x, fmaf(w10, t10.x, w00 * t00.x)));
-  feat[size_t(2 * l + 1) * N + n] = fmaf(w11, t11.y, fmaf(w01, t01.y, fmaf(w10, t10.y, w00 * t00.y)));
-}
-
-// feature-major forward, one thread per coordinate over all levels: the
-// coordinate is read once (not once per level) and each level's two stores
-// are still coalesced across the warp
-__global__ void __launch_bounds__(256) k_hash_fwd_planar_all(const float2* __restrict__ coords, int N,
-                                                             const float2* __restrict__ table, const LevelTable L,
-                                                             float* __restrict__ feat) {
-  const int n = blockIdx.x * 256 + threadIdx.x;
-  if (n >= N) return;
-  const float2 x = __ldg(coords + n);
-#pragma unroll 4
   for (int l = 0; l < L.levels; ++l) {
     const float s = L.scale[l];
     const float px = fmaf(x.x, s, 0.5f), py = fmaf(x.y, s, 0.5f);
     const float gx = floorf(px), gy = floorf(py);
-    const float fx = px - gx, fy = py - gy;
     const int ix = int(gx), iy = int(gy);
-    const float2 t00 = __ldg(table + corner_entry(L, l, ix, iy));
-    const float2 t10 = __ldg(table + corner_entry(L, l, ix + 1, iy));
-    const float2 t01 = __ldg(table + corner_entry(L, l, ix, iy + 1));
-    const float2 t11 = __ldg(table + corner_entry(L, l, ix + 1, iy + 1));
-    const float w00 = (1.f - fx) * (1.f - fy), w10 = fx * (1.f - fy), w01 = (1.f - fx) * fy, w11 = fx * fy;
-    feat[size_t(2 * l) * N + n] = fmaf(w11, t11.x, fmaf(w01, t01.x, fmaf(w10, t10.x, w00 * t00.x)));
-    feat[size_t(2 * l + 1) * N + n] = fmaf(w11, t11.y, fmaf(w01, t01.y, fmaf(w10, t10.y, w00 * t00.y)));
+    put(bilinear(__ldg(table + corner_entry(L, l, ix, iy)), __ldg(table + corner_entry(L, l, ix + 1, iy)),
+                 __ldg(table + corner_entry(L, l, ix, iy + 1)), __ldg(table + corner_entry(L, l, ix + 1, iy + 1)),
+                 px - gx, py - gy));
   }
 }
 
@@ -326,243 +340,216 @@ struct GridArgs {
   int lo0off[kMaxLevels], lo1off[kMaxLevels];
   long long voff[kMaxLevels + 1];
   float2* G;
-  // the separable levels (k = 0 .. nsep-1): level, lanes of the row and column
-  // passes, offset of the level's rows in H, first block of each pass
+  // the coarse levels (k = 0 .. nsep-1): level, columns of a block, cells of a
+  // row slot, column blocks, lanes of the row pass, offset of the level's columns
+  // in H0 / H1, first block of each pass
   int nsep;
-  int sep_l[kMaxLevels], sep_gr[kMaxLevels], sep_gc[kMaxLevels];
-  long long sep_h[kMaxLevels], sep_rb[kMaxLevels + 1], sep_cb[kMaxLevels + 1];
-  // the tiled fine levels: level, tiles per row, first block
-  int ntile;
-  int tile_l[kMaxLevels], tile_gx[kMaxLevels];
-  long long tile_b[kMaxLevels + 1];
-  float4* H;  // (S0, S1) row sums of the separable levels
+  int sep_l[kMaxLevels], sep_cb[kMaxLevels], sep_kc[kMaxLevels], sep_nx[kMaxLevels], sep_g[kMaxLevels];
+  long long sep_h[kMaxLevels];
+  int sep_b1[kMaxLevels + 1], sep_b2[kMaxLevels + 1];
+  // the fine levels: level, vertex columns of a tile, tiles per row, first block
+  int nfine;
+  int fine_l[kMaxLevels], fine_kx[kMaxLevels], fine_gx[kMaxLevels];
+  int fine_b[kMaxLevels + 1];
+  float2 *H0, *H1;  // column sums of the coarse levels, [cells][Bj] per level
 };
 
-PTY_DEVI float2 grid_dfeat(const GridArgs& g, int l, int n) {
-  if (g.planar) {
-    const float* p = g.dfeat + size_t(2 * l) * g.N + n;
-    return make_float2(__ldg(p), __ldg(p + g.N));
-  }
-  return __ldg(reinterpret_cast<const float2*>(g.dfeat) + size_t(n) * g.L + l);
-}
-
-// level, cx, cy and the contributor ranges of global vertex v
-struct VertexRange {
-  int l, cx, cy, i0, i1, j0, j1;
+// gradient value n of a level: re and im planes of [2L][N], or a pair of [N][2L]
+struct LevelGrad {
+  const float* p;
+  size_t im;  // imaginary part's distance
+  size_t es;  // element stride
 };
-PTY_DEVI VertexRange vertex_range(const GridArgs& g, long long v) {
-  VertexRange r;
-  int l = 0;
-  while (l + 1 < g.L && v >= g.voff[l + 1]) ++l;
-  const int local = int(v - g.voff[l]);
-  const int E0 = g.E0[l];
-  r.l = l;
-  r.cy = local / E0;
-  r.cx = local - r.cy * E0;
-  const int* lo0 = g.lo0 + g.lo0off[l];
-  const int* lo1 = g.lo1 + g.lo1off[l];
-  r.j0 = lo0[max(r.cx - 1, 0)];
-  r.j1 = lo0[r.cx + 1];
-  r.i0 = lo1[max(r.cy - 1, 0)];
-  r.i1 = lo1[r.cy + 1];
+PTY_DEVI LevelGrad level_grad(const GridArgs& g, int l) {
+  LevelGrad r;
+  r.p = g.dfeat + (g.planar ? size_t(2 * l) * g.N : size_t(2 * l));
+  r.im = g.planar ? size_t(g.N) : 1;
+  r.es = g.planar ? 1 : size_t(2 * g.L);
   return r;
 }
 
-PTY_DEVI float axis_weight(const int* ix, const float* fx, int k, int c) {
-  const float f = __ldg(fx + k);
-  return __ldg(ix + k) == c ? 1.f - f : f;
+// the slot of block b among levels whose blocks start at `first`
+PTY_DEVI int level_slot(int n, const int* first, int b) {
+  int k = 0;
+  while (k + 1 < n && b >= first[k + 1]) ++k;
+  return k;
 }
 
-// Sum over the flattened rectangle of vertex r: terms k = tid, tid + step, ...
-// (i = i0 + k / nj, j = j0 + k % nj), four terms' loads in flight, added in k
-// order per thread.  The row / column of the next term follow by a constant
-// increment (one division per thread).
-PTY_DEVI void rect_sum(const GridArgs& g, const VertexRange& r, int tid, int step, float& ax, float& ay) {
-  const int nj = r.j1 - r.j0, ni = r.i1 - r.i0;
-  const int total = ni * nj;
-  if (tid >= total) return;
-  const int* ix0 = g.ix0 + size_t(r.l) * g.Bj;
-  const float* fx0 = g.fx0 + size_t(r.l) * g.Bj;
-  const int* iy1 = g.iy1 + size_t(r.l) * g.A;
-  const float* fy1 = g.fy1 + size_t(r.l) * g.A;
-  const int dq = step / nj, dr = step - dq * nj;
-  int i = tid / nj, j = tid - (tid / nj) * nj;
-  int k = tid;
-  auto advance = [&]() {
-    k += step;
-    j += dr;
-    i += dq;
-    if (j >= nj) {
-      j -= nj;
-      ++i;
-    }
-  };
-  for (; k + 3 * step < total;) {
-    float w[4];
-    float2 d[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int ii = r.i0 + i, jj = r.j0 + j;
-      w[u] = axis_weight(ix0, fx0, jj, r.cx) * axis_weight(iy1, fy1, ii, r.cy);
-      d[u] = grid_dfeat(g, r.l, ii * g.Bj + jj);
-      advance();
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      ax = fmaf(w[u], d[u].x, ax);
-      ay = fmaf(w[u], d[u].y, ay);
-    }
+// Both kinds of level sum along the columns first: a thread owns a column j of
+// the grid and runs down the rows of a cell, C0 = sum (1 - fy) g and C1 = sum
+// fy g (a term's weight is wx(j, cx) * wy(i, cy)), so adjacent threads read
+// adjacent values, every value is read once and costs two loads and four FMAs.
+// Bound by instructions and load latency.  (Rows first, with lanes sharing a cell,
+// took 116 instructions per value, and a sum per vertex from a staged rectangle 240;
+// these take about 50 and 80: the backward of 1024^2 coordinates and 16 levels 118 ->
+// 80 us.)
+
+// C0 and C1 of one column
+struct ColumnSum {
+  float2 c0 = make_float2(0.f, 0.f), c1 = make_float2(0.f, 0.f);
+  PTY_DEVI void add(float w, float re, float im) {
+    const float v = 1.f - w;
+    c0.x = fmaf(v, re, c0.x);
+    c0.y = fmaf(v, im, c0.y);
+    c1.x = fmaf(w, re, c1.x);
+    c1.y = fmaf(w, im, c1.y);
   }
-  for (; k < total; advance()) {
-    const int ii = r.i0 + i, jj = r.j0 + j;
-    const float wt = axis_weight(ix0, fx0, jj, r.cx) * axis_weight(iy1, fy1, ii, r.cy);
-    const float2 d = grid_dfeat(g, r.l, ii * g.Bj + jj);
-    ax = fmaf(wt, d.x, ax);
-    ay = fmaf(wt, d.y, ay);
+};
+
+// R rows of a column from row i, the loads in flight together; then use(row, re,
+// im) in row order.  Fewer than R where the rows end at i1.
+template <int R, bool ALL, class F>
+PTY_DEVI void column_batch(const float*& p, size_t im_off, size_t rs, int i, int i1, F& use) {
+  float re[R], im[R];
+#pragma unroll
+  for (int u = 0; u < R; ++u) {
+    re[u] = im[u] = 0.f;
+    if (ALL || i + u < i1) {
+      re[u] = __ldg(p);
+      im[u] = __ldg(p + im_off);
+    }
+    p += rs;
+  }
+#pragma unroll
+  for (int u = 0; u < R; ++u)
+    if (ALL || i + u < i1) use(i + u, re[u], im[u]);
+}
+
+// rows [i, i1) of a column
+template <class F>
+PTY_DEVI void column_rows(const float* p, size_t im_off, size_t rs, int i, int i1, F use) {
+  for (; i + 8 <= i1; i += 8) column_batch<8, true>(p, im_off, rs, i, i1, use);
+  if (i + 4 <= i1) {
+    column_batch<4, true>(p, im_off, rs, i, i1, use);
+    i += 4;
+  }
+  if (i < i1) column_batch<3, false>(p, im_off, rs, i, i1, use);
+}
+
+// Coarse levels, column pass: C0 and C1 of every (cell row, column) into H0, H1.
+// A block holds CB columns (a power of two) x 256 / CB row slots.  Cells shorter
+// than kShared rows: a slot runs down kc cells.  Longer ones: the slots share one
+// cell and are added by a fixed tree.  Empty cells are neither written nor
+// read; where there are more cells than rows, an occupied cell's row in H0 and H1
+// is the number of its first grid row, so that they never outgrow the grid.
+constexpr int kShared = 32;
+
+PTY_DEVI size_t sep_row(const GridArgs& g, int l, int c, int first_row) {
+  return size_t(g.E1[l] > g.A ? first_row : c) * g.Bj;
+}
+
+__global__ void __launch_bounds__(256) k_gsep_cols(const GridArgs g) {
+  __shared__ float4 part[256];
+  const int b = blockIdx.x;
+  const int k = level_slot(g.nsep, g.sep_b1, b);
+  const int l = g.sep_l[k], CB = g.sep_cb[k], RS = 256 / CB;
+  const int bl = b - g.sep_b1[k], nx = g.sep_nx[k], by = bl / nx, bx = bl - by * nx;
+  const int t = threadIdx.x, r = t / CB, j = bx * CB + (t & (CB - 1));
+  const bool in = j < g.Bj;
+  const int* lo1 = g.lo1 + g.lo1off[l];
+  const float* fy = g.fy1 + size_t(l) * g.A;
+  const LevelGrad d = level_grad(g, l);
+  const size_t rs = size_t(g.Bj) * d.es;
+  float2* h0 = g.H0 + g.sep_h[k] + j;
+  float2* h1 = g.H1 + g.sep_h[k] + j;
+  ColumnSum s;
+  if (g.cw1[l] < kShared) {
+    int c = (by * RS + r) * g.sep_kc[k];
+    const int c_end = min(c + g.sep_kc[k], g.E1[l]);
+    if (!in || c >= c_end) return;
+    const int i0 = lo1[c];
+    int first = i0, next = lo1[c + 1];  // cell c's rows
+    auto close = [&]() {
+      if (first < next) {
+        const size_t h = sep_row(g, l, c, first);
+        h0[h] = s.c0;
+        h1[h] = s.c1;
+        s = ColumnSum();
+      }
+      first = next;
+      if (++c < c_end) next = lo1[c + 1];
+    };
+    column_rows(d.p + (size_t(i0) * g.Bj + j) * d.es, d.im, rs, i0, lo1[c_end], [&](int i, float re, float im) {
+      while (i >= next) close();  // i < lo1[c_end], so c stays below c_end
+      s.add(__ldg(fy + i), re, im);
+    });
+    while (c < c_end) close();
+    return;
+  }
+  const int c = by, i0 = lo1[c], n = lo1[c + 1] - i0, m = (n + RS - 1) / RS;
+  const int ia = i0 + min(r * m, n), ib = i0 + min((r + 1) * m, n);
+  if (in)
+    column_rows(d.p + (size_t(ia) * g.Bj + j) * d.es, d.im, rs, ia, ib,
+                [&](int i, float re, float im) { s.add(__ldg(fy + i), re, im); });
+  part[t] = make_float4(s.c0.x, s.c0.y, s.c1.x, s.c1.y);
+  __syncthreads();
+  for (int o = 128; o >= CB; o >>= 1) {
+    if (t < o) {
+      const float4 a = part[t], q = part[t + o];
+      part[t] = make_float4(a.x + q.x, a.y + q.y, a.z + q.z, a.w + q.w);
+    }
+    __syncthreads();
+  }
+  if (in && r == 0 && n > 0) {
+    const float4 a = part[t];
+    const size_t h = sep_row(g, l, c, i0);
+    h0[h] = make_float2(a.x, a.y);
+    h1[h] = make_float2(a.z, a.w);
   }
 }
 
-// G lanes per vertex (G = 1 .. 32, a power of two; 32 / G vertices per warp):
-// the group strides the flattened rectangle, then a fixed xor tree within it
-template <int G>
-__global__ void __launch_bounds__(256) k_gvert_group(const GridArgs g, long long v0, long long v1) {
-  const int t = threadIdx.x, gl = t % G;
-  const long long v = v0 + ((long long)blockIdx.x * 256 + t) / G;
-  const bool in = v < v1;
+// Coarse levels, row pass: G[cy][cx] = sum over the columns of cells cx - 1 and
+// cx of wx (C1 of cell row cy - 1 + C0 of cell row cy); lanes share a vertex.
+__global__ void __launch_bounds__(256) k_gsep_rows(const GridArgs g) {
+  const int b = blockIdx.x;
+  const int k = level_slot(g.nsep, g.sep_b2, b);
+  const int l = g.sep_l[k], G = g.sep_g[k];
+  const int t = threadIdx.x, gl = t & (G - 1);
+  // 32-bit index math (vertices < 2^31; G is a power of two)
+  const unsigned item = unsigned(b - g.sep_b2[k]) * unsigned(256 / G) + (unsigned(t) >> (__ffs(G) - 1));
+  const int E0 = g.E0[l], E1 = g.E1[l];
+  const bool in = item < unsigned(E0) * unsigned(E1);
   float ax = 0.f, ay = 0.f;
   if (in) {
-    const VertexRange r = vertex_range(g, v);
-    rect_sum(g, r, gl, G, ax, ay);
-  }
-  if constexpr (G > 1) {
+    const int cy = int(item / unsigned(E0)), cx = int(item - unsigned(cy) * unsigned(E0));
+    const int* lo0 = g.lo0 + g.lo0off[l];
+    const int j1 = lo0[cx + 1];
+    const float* fx0 = g.fx0 + size_t(l) * g.Bj;
+    const int jm = lo0[cx];  // first column of cell cx: weight fx before it, 1 - fx from it
+    const int* lo1 = g.lo1 + g.lo1off[l];
+    const int ra = lo1[max(cy - 1, 0)], rb = lo1[cy];
+    const bool own = rb < lo1[cy + 1], above = ra < rb;  // cells cy and cy - 1 hold rows
+    const float2* h0 = g.H0 + g.sep_h[k] + (own ? sep_row(g, l, cy, rb) : 0);
+    const float2* h1 = g.H1 + g.sep_h[k] + (above ? sep_row(g, l, cy - 1, ra) : 0);
+    const float2 none = make_float2(0.f, 0.f);
+    int j = lo0[max(cx - 1, 0)] + gl;
+    for (; j + 3 * G < j1; j += 4 * G) {
+      float w[4];
+      float2 a[4], q[4];
 #pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) {
-      ax += __shfl_xor_sync(0xffffffffu, ax, o);
-      ay += __shfl_xor_sync(0xffffffffu, ay, o);
+      for (int u = 0; u < 4; ++u) {
+        const float f = __ldg(fx0 + j + u * G);
+        w[u] = j + u * G < jm ? f : 1.f - f;
+        a[u] = own ? h0[j + u * G] : none;
+        q[u] = above ? h1[j + u * G] : none;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        ax = fmaf(w[u], q[u].x + a[u].x, ax);
+        ay = fmaf(w[u], q[u].y + a[u].y, ay);
+      }
+    }
+    for (; j < j1; j += G) {
+      const float f = __ldg(fx0 + j), w = j < jm ? f : 1.f - f;
+      const float2 a = own ? h0[j] : none, q = above ? h1[j] : none;
+      ax = fmaf(w, q.x + a.x, ax);
+      ay = fmaf(w, q.y + a.y, ay);
     }
   }
-  if (in && gl == 0) g.G[v] = make_float2(ax, ay);
-}
-
-// Coarse levels (cw0 * cw1 >= 16) separably, since a term's weight is
-// wx(j, cx) * wy(i, cy).  Row pass: per row i and cell c (the j with
-// ix0[j] = c), S0 = sum (1 - fx) g and S1 = sum fx g, so every gradient value
-// is read once.  Column pass: G[cy][cx] = sum over i in [lo1[cy - 1],
-// lo1[cy + 1]) of wy (S1[i][cx - 1] + S0[i][cx]).  One launch per pass covers
-// every separable level (blocks by level); G lanes (uniform in a block) share
-// one output, striding its range, then a fixed xor tree.
-
-PTY_DEVI void lane_reduce(float& ax, float& ay, int G) {
   for (int o = G >> 1; o > 0; o >>= 1) {
     ax += __shfl_xor_sync(0xffffffffu, ax, o);
     ay += __shfl_xor_sync(0xffffffffu, ay, o);
   }
-}
-
-// the separable level of block b of a pass whose levels start at `first`
-PTY_DEVI int sep_slot(const GridArgs& g, const long long* first, long long b) {
-  int k = 0;
-  while (k + 1 < g.nsep && b >= first[k + 1]) ++k;
-  return k;
-}
-
-__global__ void __launch_bounds__(256) k_gsep_rows(const GridArgs g) {
-  const long long b = blockIdx.x;
-  const int k = sep_slot(g, g.sep_rb, b);
-  const int l = g.sep_l[k], G = g.sep_gr[k];
-  const int t = threadIdx.x, gl = t & (G - 1);
-  // 32-bit index math (A * E0 < 2^31; G is a power of two)
-  const unsigned item = unsigned(int(b - g.sep_rb[k]) * 256 + t) >> (__ffs(G) - 1);
-  const unsigned E0 = unsigned(g.E0[l]);
-  const bool in = item < unsigned(g.A) * E0;
-  float s0x = 0.f, s0y = 0.f, s1x = 0.f, s1y = 0.f;
-  if (in) {
-    const int i = int(item / E0);
-    const int c = int(item - unsigned(i) * E0);
-    const int* lo0 = g.lo0 + g.lo0off[l];
-    const int j0 = lo0[c], j1 = lo0[c + 1];
-    const float* fx0 = g.fx0 + size_t(l) * g.Bj;
-    const int rowbase = i * g.Bj;
-    int j = j0 + gl;
-    for (; j + 3 * G < j1; j += 4 * G) {
-      float f[4];
-      float2 d[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        f[u] = __ldg(fx0 + j + u * G);
-        d[u] = grid_dfeat(g, l, rowbase + j + u * G);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const float w0 = 1.f - f[u];
-        s0x = fmaf(w0, d[u].x, s0x);
-        s0y = fmaf(w0, d[u].y, s0y);
-        s1x = fmaf(f[u], d[u].x, s1x);
-        s1y = fmaf(f[u], d[u].y, s1y);
-      }
-    }
-    for (; j < j1; j += G) {
-      const float f = __ldg(fx0 + j);
-      const float2 d = grid_dfeat(g, l, rowbase + j);
-      s0x = fmaf(1.f - f, d.x, s0x);
-      s0y = fmaf(1.f - f, d.y, s0y);
-      s1x = fmaf(f, d.x, s1x);
-      s1y = fmaf(f, d.y, s1y);
-    }
-  }
-  lane_reduce(s0x, s0y, G);
-  lane_reduce(s1x, s1y, G);
-  if (in && gl == 0) g.H[g.sep_h[k] + item] = make_float4(s0x, s0y, s1x, s1y);
-}
-
-__global__ void __launch_bounds__(256) k_gsep_cols(const GridArgs g) {
-  const long long b = blockIdx.x;
-  const int k = sep_slot(g, g.sep_cb, b);
-  const int l = g.sep_l[k], G = g.sep_gc[k];
-  const int t = threadIdx.x, gl = t & (G - 1);
-  const unsigned item = unsigned(int(b - g.sep_cb[k]) * 256 + t) >> (__ffs(G) - 1);
-  const int E0 = g.E0[l], E1 = g.E1[l];
-  const bool in = item < unsigned(E0) * unsigned(E1);
-  const float4* H = g.H + g.sep_h[k];
-  float ax = 0.f, ay = 0.f;
-  if (in) {
-    const int cy = int(item / unsigned(E0)), cx = int(item - unsigned(cy) * unsigned(E0));
-    auto Hat = [&](int i) {  // H[i][cx] = S1[i][cx - 1] + S0[i][cx]
-      const float4 a0 = H[size_t(i) * E0 + cx];
-      float2 h = make_float2(a0.x, a0.y);
-      if (cx > 0) {
-        const float4 a1 = H[size_t(i) * E0 + cx - 1];
-        h = make_float2(a1.z + h.x, a1.w + h.y);
-      }
-      return h;
-    };
-    const int* lo1 = g.lo1 + g.lo1off[l];
-    const int i0 = lo1[max(cy - 1, 0)], i1 = lo1[cy + 1];
-    const int* iy1 = g.iy1 + size_t(l) * g.A;
-    const float* fy1 = g.fy1 + size_t(l) * g.A;
-    int i = i0 + gl;
-    for (; i + 3 * G < i1; i += 4 * G) {
-      float w[4];
-      float2 h[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        w[u] = axis_weight(iy1, fy1, i + u * G, cy);
-        h[u] = Hat(i + u * G);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        ax = fmaf(w[u], h[u].x, ax);
-        ay = fmaf(w[u], h[u].y, ay);
-      }
-    }
-    for (; i < i1; i += G) {
-      const float w = axis_weight(iy1, fy1, i, cy);
-      const float2 h = Hat(i);
-      ax = fmaf(w, h.x, ax);
-      ay = fmaf(w, h.y, ay);
-    }
-  }
-  lane_reduce(ax, ay, G);
   if (in && gl == 0) g.G[g.voff[l] + item] = make_float2(ax, ay);
 }
 
@@ -573,113 +560,92 @@ static int lanes_for_terms(double n) {
   return G;
 }
 
-// a level takes the separable passes when its cells hold at least 16 terms
-static bool separable_level(const int32_t* extents, int l) { return extents[4 * l + 2] * extents[4 * l + 3] >= 16; }
+// Fine levels: one block per kx x kFY vertices, all such levels in one launch
+// (blocks by level).  The block's threads own the columns that its vertices
+// touch and run down the rows of cells cy0 - 1 .. cy0 + kFY - 1; a finished cell
+// gives vertex row cy its column sums V = C1(cy - 1) + C0(cy) in shared memory.
+// Then a thread per vertex column sums wx V for all kFY rows.  The halo is one
+// cell row per kFY and one cell column per tile.
+constexpr int kFY = 8;
+constexpr int kFineCell = 32;  // most axis values in a fine level's cell
 
-// Fine levels (a few contributors per vertex): one CTA per kTX x kTY vertices of
-// a level, all tiled levels in one launch (blocks by level).  The gradient sub-rectangle those vertices touch (rows i in
-// [lo1[cy0 - 1], lo1[cy0 + kTY + 1]), columns likewise) and its axis tables are
-// staged in shared memory with coalesced loads; each thread then sums its
-// vertex's rectangle from shared memory in row-major order.
-constexpr int kTX = 32, kTY = 8;
-constexpr size_t kTileSmemCap = 96 * 1024;
-
-__global__ void __launch_bounds__(256) k_gvert_tile(const GridArgs g) {
-  extern __shared__ __align__(16) unsigned char tsm[];
-  const long long b = blockIdx.x;
-  int k = 0;
-  while (k + 1 < g.ntile && b >= g.tile_b[k + 1]) ++k;
-  const int l = g.tile_l[k];
-  const int bl = int(b - g.tile_b[k]);
+__global__ void __launch_bounds__(256) k_gfine(const GridArgs g) {
+  __shared__ float2 V[kFY][256];
+  __shared__ float sfx[256];
+  __shared__ float2 sy[(kFY + 1) * kFineCell];  // a row's cell (as bits) and fraction
+  const int b = blockIdx.x;
+  const int k = level_slot(g.nfine, g.fine_b, b);
+  const int l = g.fine_l[k], kx = g.fine_kx[k];
+  const int bl = b - g.fine_b[k], by = bl / g.fine_gx[k], bx = bl - by * g.fine_gx[k];
   const int E0 = g.E0[l], E1 = g.E1[l];
-  const int cx0 = (bl % g.tile_gx[k]) * kTX, cy0 = (bl / g.tile_gx[k]) * kTY;
+  const int cx0 = bx * kx, cy0 = by * kFY, cx1 = min(cx0 + kx, E0), cy1 = min(cy0 + kFY, E1);
   const int* lo0 = g.lo0 + g.lo0off[l];
   const int* lo1 = g.lo1 + g.lo1off[l];
-  const int j_lo = lo0[max(cx0 - 1, 0)], j_hi = lo0[min(cx0 + kTX + 1, E0)];
-  const int i_lo = lo1[max(cy0 - 1, 0)], i_hi = lo1[min(cy0 + kTY + 1, E1)];
-  const int nc = j_hi - j_lo, nr = i_hi - i_lo;
-  float* sre = reinterpret_cast<float*>(tsm);
-  float* sim = sre + nr * nc;
-  int* six = reinterpret_cast<int*>(sim + nr * nc);
-  float* sfx = reinterpret_cast<float*>(six + nc);
-  int* siy = reinterpret_cast<int*>(sfx + nc);
-  float* sfy = reinterpret_cast<float*>(siy + nr);
+  const int j_lo = lo0[max(cx0 - 1, 0)], nc = min(lo0[cx1] - j_lo, 256);
+  const int i_lo = lo1[max(cy0 - 1, 0)], nr = min(lo1[cy1] - i_lo, (kFY + 1) * kFineCell);
   const int t = threadIdx.x;
-  for (int q = t; q < nc; q += 256) {
-    six[q] = __ldg(g.ix0 + size_t(l) * g.Bj + j_lo + q);
-    sfx[q] = __ldg(g.fx0 + size_t(l) * g.Bj + j_lo + q);
-  }
   for (int q = t; q < nr; q += 256) {
-    siy[q] = __ldg(g.iy1 + size_t(l) * g.A + i_lo + q);
-    sfy[q] = __ldg(g.fy1 + size_t(l) * g.A + i_lo + q);
+    sy[q] = make_float2(__int_as_float(__ldg(g.iy1 + size_t(l) * g.A + i_lo + q)),
+                        __ldg(g.fy1 + size_t(l) * g.A + i_lo + q));
   }
-  for (int r = t >> 5; r < nr; r += 8) {  // a warp per row, lanes along it
-    for (int c = t & 31; c < nc; c += 32) {
-      const float2 d = grid_dfeat(g, l, (i_lo + r) * g.Bj + j_lo + c);
-      sre[r * nc + c] = d.x;
-      sim[r * nc + c] = d.y;
-    }
+  if (t < nc) sfx[t] = __ldg(g.fx0 + size_t(l) * g.Bj + j_lo + t);
+  __syncthreads();
+  if (t < nc) {
+    const LevelGrad d = level_grad(g, l);
+    const float* p = d.p + (size_t(i_lo) * g.Bj + j_lo + t) * d.es;
+    const size_t rs = size_t(g.Bj) * d.es;
+    ColumnSum s;
+    float2 up = make_float2(0.f, 0.f);
+    int c = max(cy0 - 1, 0);
+    auto close = [&]() {  // cell row c is complete
+      if (c >= cy0) V[c - cy0][t] = make_float2(up.x + s.c0.x, up.y + s.c0.y);
+      up = s.c1;
+      s = ColumnSum();
+      ++c;
+    };
+    column_rows(p, d.im, rs, 0, nr, [&](int i, float re, float im) {
+      const float2 y = sy[i];
+      const int ci = min(__float_as_int(y.x), cy1 - 1);
+      while (c < ci) close();
+      s.add(y.y, re, im);
+    });
+    while (c < cy1) close();
   }
   __syncthreads();
-  const int cx = cx0 + (t % kTX), cy = cy0 + (t / kTX);
-  if (cx >= E0 || cy >= E1) return;
-  // (splitting each row's sum at lo0[cx] into two loops without the cell test
-  // measured slower on c4: 219 against 181 us)
-  const int j0 = lo0[max(cx - 1, 0)] - j_lo, j1 = lo0[cx + 1] - j_lo;
-  const int i0 = lo1[max(cy - 1, 0)] - i_lo, i1 = lo1[cy + 1] - i_lo;
-  float ax = 0.f, ay = 0.f;
-  for (int i = i0; i < i1; ++i) {
-    const float fy = sfy[i];
-    const float wy = siy[i] == cy ? 1.f - fy : fy;
-    for (int j = j0; j < j1; ++j) {
-      const float fx = sfx[j];
-      const float w = (six[j] == cx ? 1.f - fx : fx) * wy;
-      ax = fmaf(w, sre[i * nc + j], ax);
-      ay = fmaf(w, sim[i * nc + j], ay);
-    }
-  }
-  g.G[g.voff[l] + (long long)cy * E0 + cx] = make_float2(ax, ay);
-}
-
-// shared memory of a tile of level l (rows and columns bounded by the cell widths)
-static size_t tile_smem(const GridArgs& g, int l) {
-  const size_t nc = size_t(kTX + 2) * g.cw0[l], nr = size_t(kTY + 2) * g.cw1[l];
-  return (2 * nr * nc + 2 * nc + 2 * nr) * 4;
-}
-
-// WPB warps (1 or 8) per vertex: the WPB * 32 threads stride the flattened
-// rectangle; fixed xor tree per warp, then the warps' partials in warp order
-template <int WPB>
-__global__ void __launch_bounds__(256) k_gvert_warp(const GridArgs g, long long v0, long long v1) {
-  __shared__ float2 part[8];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int slot = w / WPB, ww = w % WPB;  // 8 / WPB vertices per block
-  const long long v = v0 + (long long)blockIdx.x * (8 / WPB) + slot;
-  const bool in = v < v1;
-  float ax = 0.f, ay = 0.f;
-  if (in) {
-    const VertexRange r = vertex_range(g, v);
-    rect_sum(g, r, ww * 32 + lane, WPB * 32, ax, ay);
-  }
+  const int cx = cx0 + t;
+  if (cx >= cx1) return;
+  float2 a[kFY];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    ax += __shfl_xor_sync(0xffffffffu, ax, o);
-    ay += __shfl_xor_sync(0xffffffffu, ay, o);
+  for (int q = 0; q < kFY; ++q) a[q] = make_float2(0.f, 0.f);
+  const int jm = lo0[cx] - j_lo, j1 = min(lo0[cx + 1] - j_lo, nc);
+  for (int j = lo0[max(cx - 1, 0)] - j_lo; j < j1; ++j) {
+    const float f = sfx[j], w = j < jm ? f : 1.f - f;
+#pragma unroll
+    for (int q = 0; q < kFY; ++q) {
+      const float2 v = V[q][j];
+      a[q].x = fmaf(w, v.x, a[q].x);
+      a[q].y = fmaf(w, v.y, a[q].y);
+    }
   }
-  if (WPB == 1) {
-    if (in && lane == 0) g.G[v] = make_float2(ax, ay);
-    return;
-  }
-  if (lane == 0) part[w] = make_float2(ax, ay);
-  __syncthreads();
-  if (in && ww == 0 && lane == 0) {
-    float2 t = part[w];
-    for (int k = 1; k < WPB; ++k) t = c_add(t, part[w + k]);
-    g.G[v] = t;
-  }
+  float2* G = g.G + g.voff[l] + (long long)cy0 * E0 + cx;
+#pragma unroll
+  for (int q = 0; q < kFY; ++q)
+    if (cy0 + q < cy1) G[(long long)q * E0] = a[q];
 }
 
-// per table entry: the G of its vertices, in vertex-list order
+// A level takes the two passes when its cells hold at least kSepTerms values or
+// are too long for a fine tile's tables.  1024^2 coordinates, 16 levels, forward and
+// backward: 140, 135.5 and 135.4 us with the line at 16, 36 and 64 values; 900 x 1000:
+// 124, 119 and 121
+constexpr int kSepTerms = 36;
+constexpr int kSepRows = 16;  // rows of a row slot in the coarse levels' column pass
+static bool separable_level(const int32_t* extents, int l) {
+  const int32_t cw0 = extents[4 * l + 2], cw1 = extents[4 * l + 3];
+  return cw0 > kFineCell || cw1 > kFineCell || cw0 * cw1 >= kSepTerms;
+}
+
+// per table entry: the G of its vertices, in vertex-list order (four entries per
+// thread: 18.7 against 14.3 us, fewer warps for the gathers)
 __global__ void __launch_bounds__(256) k_gentry(const int* __restrict__ vstart, const int* __restrict__ vorder,
                                                 const float2* __restrict__ G, int E, float2* __restrict__ dtable,
                                                 int accumulate) {
@@ -714,9 +680,8 @@ int ptycho_hashgrid_forward(const float* coords, int N, const float* table, int 
   if (!pty_aligned(coords, 8) || !pty_aligned(table, 8) || !pty_aligned(features, 8))
     return PTYCHO_ERR_MISALIGNED;
   if (N == 0) return PTYCHO_OK;
-  k_hash_fwd<<<(unsigned)((N + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const float2*>(coords), N, reinterpret_cast<const float2*>(table), L,
-      reinterpret_cast<float2*>(features));
+  k_hash_fwd<false><<<(unsigned)((N + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+      reinterpret_cast<const float2*>(coords), N, reinterpret_cast<const float2*>(table), L, features);
   return cudaGetLastError() == cudaSuccess ? PTYCHO_OK : PTYCHO_ERR_LAUNCH;
 }
 
@@ -730,14 +695,8 @@ int ptycho_hashgrid_forward_planar(const float* coords, int N, const float* tabl
   if (!pty_aligned(coords, 8) || !pty_aligned(table, 8) || !pty_aligned(features_planar, 4))
     return PTYCHO_ERR_MISALIGNED;
   if (N == 0) return PTYCHO_OK;
-#ifndef PTY_HASH_FWD_PER_LEVEL
-  k_hash_fwd_planar_all<<<(unsigned)((N + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  k_hash_fwd<true><<<(unsigned)((N + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       reinterpret_cast<const float2*>(coords), N, reinterpret_cast<const float2*>(table), L, features_planar);
-#else
-  const dim3 grid((unsigned)((N + 255) / 256), (unsigned)L.levels);
-  k_hash_fwd_planar<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const float2*>(coords), N, reinterpret_cast<const float2*>(table), L, features_planar);
-#endif
   return cudaGetLastError() == cudaSuccess ? PTYCHO_OK : PTYCHO_ERR_LAUNCH;
 }
 
@@ -832,10 +791,10 @@ size_t ptycho_hashgrid_grid_scratch_size(const int32_t* extents, int n_levels, i
   for (int l = 0; l < n_levels; ++l) {
     if (extents[4 * l] < 1 || extents[4 * l + 1] < 1 || extents[4 * l + 2] < 1 || extents[4 * l + 3] < 1) return 0;
     n += size_t(extents[4 * l]) * size_t(extents[4 * l + 1]);
-    if (separable_level(extents, l)) h += size_t(A) * size_t(extents[4 * l]);
+    if (separable_level(extents, l)) h += size_t(Bj) * size_t(extents[4 * l + 1] < A ? extents[4 * l + 1] : A);
   }
-  // vertex sums (float2), then every separable level's (S0, S1) rows (float4)
-  return n * sizeof(float2) + 16 + h * sizeof(float4);
+  // vertex sums, then every coarse level's column sums C0 and C1
+  return (n + 2 * h) * sizeof(float2);
 }
 
 int ptycho_hashgrid_backward_grid(const int32_t* grid_int, const float* grid_frac, const int32_t* extents, int A,
@@ -893,77 +852,49 @@ int ptycho_hashgrid_backward_grid(const int32_t* grid_int, const float* grid_fra
   g.fx0 = grid_frac;
   g.fy1 = grid_frac + size_t(n_levels) * Bj;
   g.G = static_cast<float2*>(scratch);
-  // lanes per vertex by the level's average contributors per vertex: 256 (a
-  // block) from 2048 terms, else the power of two nearest terms / 4 in 1 .. 32
-  // (about four terms per lane); levels run coarse to fine, so equal choices
-  // form runs of levels, one launch each
-  auto lanes_for = [&](int l) {
-    const double terms = (2.0 * Bj / g.E0[l]) * (2.0 * A / g.E1[l]);
-    if (terms >= 2048.0) return 256;
-    int G = 1;
-    while (G < 32 && 4.0 * G * 2 <= terms) G *= 2;
-    return G;
-  };
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  g.H = reinterpret_cast<float4*>(pty_align_up(reinterpret_cast<uintptr_t>(g.G + g.voff[n_levels]), 16));
-  // plan the levels: separable ones (two launches for all of them), tiled fine
-  // levels (one launch), the rest per vertex with G lanes (runs of equal G)
-  long long hoff = 0, rb = 0, cb = 0, tb = 0;
-  size_t tsmem = 0;
-  int rest[kMaxLevels], nrest = 0;
+  // plan the levels: the coarse ones take two launches for all of them, the fine
+  // ones one
+  long long hoff = 0, b1 = 0, b2 = 0, tb = 0;
   for (int l = 0; l < n_levels; ++l) {
+    const int cw0 = g.cw0[l], cw1 = g.cw1[l];
     if (separable_level(extents, l)) {
       const int k = g.nsep++;
       g.sep_l[k] = l;
-      g.sep_gr[k] = lanes_for_terms(double(g.cw0[l]));  // one cell per row item
-      g.sep_gc[k] = lanes_for_terms(2.0 * A / g.E1[l]);
+      // columns of a block: the grid's, at most 256, and fewer where the slots share
+      // a cell, so that a thread adds about 16 rows
+      int CB = 256;
+      while (CB > 1 && (CB / 2 >= Bj || (CB > 32 && cw1 >= kShared && cw1 >= 32 * (256 / CB)))) CB /= 2;
+      const int RS = 256 / CB;
+      g.sep_cb[k] = CB;
+      g.sep_kc[k] = cw1 >= kShared ? 1 : (kSepRows + cw1 - 1) / cw1;
+      const int cells = cw1 >= kShared ? 1 : g.sep_kc[k] * RS;  // of a block
+      g.sep_nx[k] = (Bj + CB - 1) / CB;
+      g.sep_g[k] = lanes_for_terms(2.0 * Bj / g.E0[l]);
       g.sep_h[k] = hoff;
-      hoff += (long long)A * g.E0[l];
-      g.sep_rb[k] = rb;
-      rb += ((long long)A * g.E0[l] * g.sep_gr[k] + 255) / 256;
-      g.sep_cb[k] = cb;
-      cb += ((long long)g.E0[l] * g.E1[l] * g.sep_gc[k] + 255) / 256;
-    } else if (lanes_for(l) <= 8 && tile_smem(g, l) <= kTileSmemCap) {
-      const int k = g.ntile++;
-      g.tile_l[k] = l;
-      g.tile_gx[k] = (g.E0[l] + kTX - 1) / kTX;
-      g.tile_b[k] = tb;
-      tb += (long long)g.tile_gx[k] * ((g.E1[l] + kTY - 1) / kTY);
-      tsmem = tile_smem(g, l) > tsmem ? tile_smem(g, l) : tsmem;
+      hoff += (long long)(g.E1[l] < A ? g.E1[l] : A) * Bj;
+      g.sep_b1[k] = int(b1);
+      b1 += (long long)g.sep_nx[k] * ((g.E1[l] + cells - 1) / cells);
+      g.sep_b2[k] = int(b2);
+      b2 += ((long long)g.E0[l] * g.E1[l] * g.sep_g[k] + 255) / 256;
     } else {
-      rest[nrest++] = l;
+      const int k = g.nfine++;
+      const int most = 256 / cw0 - 1;  // kx + 1 cells' columns fit the block
+      g.fine_l[k] = l;
+      g.fine_gx[k] = (g.E0[l] + most - 1) / most;
+      g.fine_kx[k] = (g.E0[l] + g.fine_gx[k] - 1) / g.fine_gx[k];
+      g.fine_b[k] = int(tb);
+      tb += (long long)g.fine_gx[k] * ((g.E1[l] + kFY - 1) / kFY);
     }
   }
-  g.sep_rb[g.nsep] = rb;
-  g.sep_cb[g.nsep] = cb;
-  g.tile_b[g.ntile] = tb;
+  g.H0 = g.G + g.voff[n_levels];
+  g.H1 = g.H0 + hoff;
+  if (b1 >= (1ll << 31) || b2 >= (1ll << 31) || tb >= (1ll << 31)) return PTYCHO_ERR_UNSUPPORTED_SIZE;
   if (g.nsep) {
-    k_gsep_rows<<<unsigned(rb), 256, 0, s>>>(g);
-    k_gsep_cols<<<unsigned(cb), 256, 0, s>>>(g);
+    k_gsep_cols<<<unsigned(b1), 256, 0, s>>>(g);
+    k_gsep_rows<<<unsigned(b2), 256, 0, s>>>(g);
   }
-  if (g.ntile) {
-    if (tsmem > 48 * 1024 &&
-        cudaFuncSetAttribute(k_gvert_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTileSmemCap)) !=
-            cudaSuccess)
-      return PTYCHO_ERR_LAUNCH;
-    k_gvert_tile<<<unsigned(tb), 256, tsmem, s>>>(g);
-  }
-  for (int r = 0; r < nrest;) {
-    const int l0 = rest[r], G = lanes_for(l0);
-    int r1 = r + 1;
-    while (r1 < nrest && rest[r1] == rest[r1 - 1] + 1 && lanes_for(rest[r1]) == G) ++r1;
-    const long long va = g.voff[l0], vb = g.voff[rest[r1 - 1] + 1], nvv = vb - va;
-    switch (G) {
-      case 256: k_gvert_warp<8><<<unsigned(nvv), 256, 0, s>>>(g, va, vb); break;
-      case 32: k_gvert_group<32><<<unsigned((nvv * 32 + 255) / 256), 256, 0, s>>>(g, va, vb); break;
-      case 16: k_gvert_group<16><<<unsigned((nvv * 16 + 255) / 256), 256, 0, s>>>(g, va, vb); break;
-      case 8: k_gvert_group<8><<<unsigned((nvv * 8 + 255) / 256), 256, 0, s>>>(g, va, vb); break;
-      case 4: k_gvert_group<4><<<unsigned((nvv * 4 + 255) / 256), 256, 0, s>>>(g, va, vb); break;
-      case 2: k_gvert_group<2><<<unsigned((nvv * 2 + 255) / 256), 256, 0, s>>>(g, va, vb); break;
-      default: k_gvert_group<1><<<unsigned((nvv + 255) / 256), 256, 0, s>>>(g, va, vb); break;
-    }
-    r = r1;
-  }
+  if (g.nfine) k_gfine<<<unsigned(tb), 256, 0, s>>>(g);
   k_gentry<<<unsigned((L.total + 255) / 256), 256, 0, s>>>(g.vstart, g.vorder, g.G, L.total,
                                                            reinterpret_cast<float2*>(dtable), accumulate);
   return cudaGetLastError() == cudaSuccess ? PTYCHO_OK : PTYCHO_ERR_LAUNCH;
