@@ -201,7 +201,7 @@ def parity_vs_cpu(pkg, work, first, dev):
 
 def side_workload(pkg, key, dev, steps=30, warmup=5, n_check=8):
     """Throughput and parity of the fused path on another workload's shapes
-    (c3 / c4: the 256^2 cluster kernel), run inside the default c1 bench.
+    (c3 / c4: the 256^2 line kernels), run inside the default c1 bench.
 
     Same object, probe and raster recipe as ``synth.make_workload(key)``; the
     measurements are generated for 2 x batch frames taken at a regular stride
@@ -534,7 +534,7 @@ def run_ours(args):
                                            f"{n_settle} identical untimed steps on either side "
                                            f"(~{args.settle_s:.1f} s each)")}
         if world == 1 and not args.no_side and args.workload == "c1":
-            # the 256^2 cluster path on the c3 / c4 shapes, recorded beside the headline
+            # the 256^2 path on the c3 / c4 shapes, recorded beside the headline
             side = {}
             for key in ("c3", "c4"):
                 try:

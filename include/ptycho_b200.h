@@ -294,7 +294,7 @@ int ptycho_residual_backward(const float* k, const float* m, const float* g, lon
  * conjugate transpose).  h, w, h*s and w*s must be powers of two in
  * [64, 4096] with s in {1, 2, 4}; otherwise PTYCHO_ERR_UNSUPPORTED_SIZE.
  * workspace: device scratch of ptycho_fourier_upsample_workspace_size()
- * bytes (the intermediate after the row pass), 8-byte aligned.
+ * bytes (the intermediate between the two passes), 8-byte aligned.
  * ---------------------------------------------------------------------- */
 size_t ptycho_fourier_upsample_workspace_size(int h, int w, int s);
 
