@@ -437,20 +437,23 @@ static int launch(int n, int s, const float2* in, float2* out, int nlines, long 
     g.ngroups = (nlines + lines - 1) / lines;
   };
   if constexpr (COL) {
-    // 16 adjacent columns (128-byte pieces) while two CTAs fit an SM, else 4 or 1
+    // 16 adjacent columns (128-byte pieces) while two CTAs fit an SM, else 4 or 1; four
+    // long columns leave room for one CTA, so it has 1024 threads (1500^2 by 2, up and
+    // down: 419 us with 512, 403 with 768, 395 with 1024)
     if (smem_of(g, 16) <= 112 * 1024) {
       groups(16);
       return launch_k<16, 256, ADJ>(g, st);
     }
     if (smem_of(g, 4) <= ln::kSmemCap) {
       groups(4);
-      return launch_k<4, 512, ADJ>(g, st);
+      return launch_k<4, 1024, ADJ>(g, st);
     }
     groups(1);
     return launch_k<1, 512, ADJ>(g, st);
   } else {
-    // about 3072 values per CTA
-    int lines = 3072 / g.plan.m;
+    // about 1536 values per CTA: four CTAs of a long line fit an SM (1500^2 by 2: 419
+    // -> 396 us, 500^2 by 3 126 -> 115, 999 x 1500 463 -> 435 against 3072 values)
+    int lines = 1536 / g.plan.m;
     lines = lines < 1 ? 1 : lines;
     while (lines > 1 && smem_of(g, lines) > ln::kSmemCap) --lines;
     groups(lines);
