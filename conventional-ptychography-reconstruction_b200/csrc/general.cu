@@ -314,12 +314,19 @@ static void set_groups(Args* g, int per_pattern_lines) {
 template <bool INV>
 static int run_rows(Args g, cudaStream_t s) {
   if (!ln::make_plan(g.N, 0, &g.plan)) return PTYCHO_ERR_UNSUPPORTED_SIZE;
-  // about 3072 values per CTA (four CTAs per SM), never more rows than there are
-  int lines = 3072 / g.plan.m;
-  lines = lines < 1 ? 1 : (lines > g.M ? g.M : lines);
-  while (lines > 1 && ln::smem_bytes(g.plan, lines, 0) > ln::kSmemCap) --lines;
-  g.lines = lines;
-  set_groups(&g, g.M);
+  // about 3072 values per CTA (four CTAs per SM), never more rows than there are; half
+  // of that where the batch would not fill the slots (148 x 4): steps of 1 x 150^2 47.6 ->
+  // 43.5 us, 32 x 100 x 120 51.7 -> 47.7, 64 x 96^2 60.0 -> 58.1.  On full grids the
+  // larger CTA is better: 40 x 320^2 171 against 183, 64 x 192^2 91 against 96
+  int lines = 0;
+  for (int values = 3072; values >= 1536; values /= 2) {
+    lines = values / g.plan.m;
+    lines = lines < 1 ? 1 : (lines > g.M ? g.M : lines);
+    while (lines > 1 && ln::smem_bytes(g.plan, lines, 0) > ln::kSmemCap) --lines;
+    g.lines = lines;
+    set_groups(&g, g.M);
+    if (g.ngroups >= 148 * 4) break;
+  }
   static PtyDevCache attr;
   return launch(k_rows<INV>, attr, g, ln::smem_bytes(g.plan, lines, 0), s);
 }
