@@ -17,6 +17,8 @@
 // narrow side, in pieces of a few columns; the wide side moves as whole rows.
 // Twiddles of the power-of-two kernels come from the correctly rounded build-time
 // table kTw4096 (twiddle4096.cuh).
+// A NaN or infinity anywhere reaches every output of its line, hence of the plane, as
+// it does through the transforms of the reference, also where phase 0 is copied.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -26,6 +28,10 @@
 #include "twiddle4096.cuh"
 
 namespace pty {
+
+// x, not finite where z is not
+PTY_DEVI float2 c_taint(float2 x, float2 z) { return make_float2(fmaf(0.f, z.x, x.x), fmaf(0.f, z.y, x.y)); }
+
 namespace sh {
 
 // ---------------------------------------------------------------------------
@@ -139,6 +145,7 @@ __global__ void __launch_bounds__(Cfg<N, COL>::NT, Cfg<N, COL>::MINB) k_shift(co
         const int m = q + T * e;
         v[e] = make_float2(0.f, 0.f);
         if (ok) v[e] = ADJ ? __ldg(at(g.in, g.ld_in, s * m + p)) : __ldg(at(g.in, g.ld_in, m));
+        if (ADJ && ok && p == 1) v[e] = c_taint(v[e], __ldg(at(g.in, g.ld_in, s * m)));
         if (COL && !ADJ && ok && p == 1) *at(g.out, g.ld_out, s * m) = v[e];  // phase 0
       }
       prefetch_line<N, COL, ADJ>(g, l0 + gridDim.x * LINES, t);
@@ -202,10 +209,11 @@ __global__ void __launch_bounds__(Cfg<N, COL>::NT, Cfg<N, COL>::MINB) k_shift(co
           float2* o = at(g.out, g.ld_out, m);
           *o = c_add(p == 1 ? __ldg(at(g.in, g.ld_in, s * m)) : *o, v[e]);
         } else if (!COL && s == 2 && g.vec) {
-          const float2 x = __ldg(at(g.in, g.ld_in, m));
+          const float2 x = c_taint(__ldg(at(g.in, g.ld_in, m)), v[e]);
           *reinterpret_cast<float4*>(at(g.out, g.ld_out, 2 * m)) = make_float4(x.x, x.y, v[e].x, v[e].y);
         } else {
-          if (!COL && p == 1) *at(g.out, g.ld_out, s * m) = __ldg(at(g.in, g.ld_in, m));
+          if (!COL && p == 1) *at(g.out, g.ld_out, s * m) = c_taint(__ldg(at(g.in, g.ld_in, m)), v[e]);
+          if (COL && p == 1 && !(isfinite(v[e].x) && isfinite(v[e].y))) *at(g.out, g.ld_out, s * m) = v[e];
           *at(g.out, g.ld_out, s * m + p) = v[e];
         }
       }
@@ -342,6 +350,7 @@ __global__ void __launch_bounds__(NT, LINES == 16 || LINES == 0 ? 4 : 1) k_resam
         float2 v = make_float2(0.f, 0.f);
         if (l0 + l < g.nlines)
           v = ADJ ? turn(__ldg(at(g.in, g.ld_in, l0 + l, s * k + p)), k, wp) : __ldg(at(g.in, g.ld_in, l0 + l, k));
+        if (ADJ && p == 1 && l0 + l < g.nlines) v = c_taint(v, __ldg(at(g.in, g.ld_in, l0 + l, s * k)));
         ln.put(g.plan, l, k, v);
       }
       ln.pad(g.plan);
@@ -373,7 +382,7 @@ __global__ void __launch_bounds__(NT, LINES == 16 || LINES == 0 ? 4 : 1) k_resam
       } else {
         const float2 z = turn(v, k, wp);
         float2 x = make_float2(0.f, 0.f);
-        if (p0 == 1) x = turn(__ldg(at(g.in, g.ld_in, l0 + l, k)), k, one);
+        if (p0 == 1) x = c_taint(turn(__ldg(at(g.in, g.ld_in, l0 + l, k)), k, one), z);
         if (!COL && s == 2 && g.vec) {
           *reinterpret_cast<float4*>(at(g.out, g.ld_out, l0 + l, 2 * k)) = make_float4(x.x, x.y, z.x, z.y);
         } else {
@@ -480,11 +489,29 @@ int axis_pass(int n, int s, const float2* in, float2* out, int nlines, long long
   return rsg::launch<COL, ADJ>(n, s, in, out, nlines, ld_in, ld_out, st);
 }
 
-// s = 1: the operator is the identity
-int copy_plane(const float* in, float* out, size_t n, cudaStream_t st) {
-  return cudaMemcpyAsync(out, in, n * sizeof(float2), cudaMemcpyDeviceToDevice, st) == cudaSuccess
-             ? PTYCHO_OK
-             : PTYCHO_ERR_LAUNCH;
+// s = 1: the operator is the identity, and NaN throughout where any input is not
+// finite: every block says whether its share is, then every block copies
+constexpr int kCopyBlocks = 148 * 4;
+__global__ void __launch_bounds__(256) k_nonfinite(const float* __restrict__ in, size_t n, int* __restrict__ bad) {
+  int b = 0;
+  for (size_t i = size_t(blockIdx.x) * 256 + threadIdx.x; i < n; i += size_t(gridDim.x) * 256) b |= !isfinite(in[i]);
+  b = __syncthreads_or(b);
+  if (threadIdx.x == 0) bad[blockIdx.x] = b;
+}
+__global__ void __launch_bounds__(256) k_copy(const float* in, float* out, size_t n, const int* __restrict__ bad) {
+  int b = 0;
+  for (int i = threadIdx.x; i < gridDim.x; i += 256) b |= bad[i];
+  b = __syncthreads_or(b);
+  for (size_t i = size_t(blockIdx.x) * 256 + threadIdx.x; i < n; i += size_t(gridDim.x) * 256)
+    out[i] = b ? __int_as_float(0x7fc00000) : in[i];
+}
+int copy_plane(const float* in, float* out, size_t n, void* workspace, cudaStream_t st) {
+  n *= 2;  // floats
+  const size_t need = (n + 255) / 256;  // blocks; their flags (n / 64 bytes) fit the workspace (4 n bytes)
+  const unsigned grid = unsigned(need < kCopyBlocks ? need : kCopyBlocks);
+  k_nonfinite<<<grid, 256, 0, st>>>(in, n, static_cast<int*>(workspace));
+  k_copy<<<grid, 256, 0, st>>>(in, out, n, static_cast<const int*>(workspace));
+  return cudaGetLastError() == cudaSuccess ? PTYCHO_OK : PTYCHO_ERR_LAUNCH;
 }
 
 bool supported_upsample(int h, int w, int s) {
@@ -511,7 +538,7 @@ int ptycho_fourier_upsample(const float* x, int h, int w, int s, float* y, void*
   if (!pty_aligned(x, 8) || !pty_aligned(y, 8) || !pty_aligned(workspace, 8)) return PTYCHO_ERR_MISALIGNED;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int W = w * s, H = h * s;
-  if (s == 1) return copy_plane(x, y, size_t(h) * w, st);
+  if (s == 1) return copy_plane(x, y, size_t(h) * w, workspace, st);
   float2* tmp = static_cast<float2*>(workspace);  // [H][w]: the column pass moves the narrow side
   int rc = axis_pass<true, false>(h, s, reinterpret_cast<const float2*>(x), tmp, w, w, w, st);  // columns
   if (rc) return rc;
@@ -527,7 +554,7 @@ int ptycho_fourier_upsample_adjoint(const float* gy, int h, int w, int s, float*
   if (!pty_aligned(gy, 8) || !pty_aligned(gx, 8) || !pty_aligned(workspace, 8)) return PTYCHO_ERR_MISALIGNED;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int W = w * s, H = h * s;
-  if (s == 1) return copy_plane(gy, gx, size_t(h) * w, st);
+  if (s == 1) return copy_plane(gy, gx, size_t(h) * w, workspace, st);
   float2* tmp = static_cast<float2*>(workspace);  // [H][w]
   int rc = axis_pass<false, true>(w, s, reinterpret_cast<const float2*>(gy), tmp, H, W, w, st);  // rows
   if (rc) return rc;
