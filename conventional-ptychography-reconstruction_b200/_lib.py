@@ -126,6 +126,14 @@ _torchext = None
 _torchext_tried = False
 
 
+def plain(x):
+    """``x`` as a kernel reads it: contiguous, and with no pending conjugation or
+    negation (``contiguous()`` alone keeps those, and ``data_ptr()`` knows neither)."""
+    if x.is_conj() or x.is_neg():
+        x = x.resolve_conj().resolve_neg()
+    return x.contiguous()
+
+
 def torchext():
     """The C++ autograd nodes (csrc/torch_ext.cpp) bound to this process's
     library, or None when they are not built."""

@@ -66,8 +66,8 @@ def object_error(recon: torch.Tensor, truth: torch.Tensor, box=None) -> dict:
         raise ValueError(f"recon and truth must be 2-D of one shape, got {tuple(recon.shape)}, {tuple(truth.shape)}")
     H, W = recon.shape
     y0, y1, x0, x1 = box if box is not None else (0, H, 0, W)
-    r = recon.detach().to(torch.complex64).contiguous()
-    t = truth.detach().to(device=r.device, dtype=torch.complex64).contiguous()
+    r = _lib.plain(recon.detach().to(torch.complex64))
+    t = _lib.plain(truth.detach().to(device=r.device, dtype=torch.complex64))
     out = torch.empty(7, dtype=torch.float64, device=r.device)
     n = int(_lib.lib().ptycho_object_error_workspace_size())
     ws = torch.empty(n, dtype=torch.uint8, device=r.device)

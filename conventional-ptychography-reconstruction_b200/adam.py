@@ -60,7 +60,7 @@ class FusedAdam(torch.optim.Optimizer):
                 if not st:
                     st["exp_avg"] = torch.zeros_like(p, memory_format=torch.contiguous_format)
                     st["exp_avg_sq"] = torch.zeros_like(p, memory_format=torch.contiguous_format)
-            grads = [_real(p.grad).contiguous() for p in ps]
+            grads = [_real(_lib.plain(p.grad)) for p in ps]
             n = len(ps)
             arr = lambda xs: ctypes.cast((ctypes.c_void_p * n)(*xs), ctypes.POINTER(ctypes.c_void_p))  # noqa: E731
             N = (ctypes.c_longlong * n)(*[_real(p).numel() for p in ps])
@@ -101,7 +101,7 @@ class FusedAdam(torch.optim.Optimizer):
                 by_step.setdefault(self.state[p]["step"], []).append(p)
             chunks = [(st, lst[i:i + 48]) for st, lst in by_step.items() for i in range(0, len(lst), 48)]
             for step, chunk in chunks:
-                grads = [_real(p.grad).contiguous() for p in chunk]
+                grads = [_real(_lib.plain(p.grad)) for p in chunk]
                 n = len(chunk)
                 P = (ctypes.c_void_p * n)(*[_real(p).data_ptr() for p in chunk])
                 G = (ctypes.c_void_p * n)(*[g.data_ptr() for g in grads])

@@ -48,8 +48,8 @@ def _params(net):
 def _f32(t):
     t = t.detach()
     if t.is_complex():
-        t = torch.view_as_real(t.resolve_conj().contiguous())
-    return t.contiguous().float()
+        t = torch.view_as_real(_lib.plain(t))
+    return _lib.plain(t).float()
 
 
 def _is_planar(x: torch.Tensor) -> bool:
@@ -85,7 +85,7 @@ class _CmlpFn(torch.autograd.Function):
         x, packed = ctx.saved_tensors
         dev = x.device
         N = x.shape[0]
-        gy = gy.reshape(N).to(torch.complex64).resolve_conj().contiguous()
+        gy = _lib.plain(gy.reshape(N).to(torch.complex64))
         grad = torch.empty(int(L.ptycho_cmlp_grad_floats()), dtype=torch.float32, device=dev)
         ws = torch.empty(int(L.ptycho_cmlp_backward_workspace_size(N)), dtype=torch.uint8, device=dev)
         st = device_status(dev)
@@ -131,7 +131,7 @@ class _FusedSequential(nn.Sequential):
                              device_status(x.device))
             _lib.check(rc, "ptycho_cmlp_forward")
             return y
-        x = x.float()
+        x = x.float().resolve_neg()
         if not _is_planar(x):
             x = x.contiguous()
         return _CmlpFn.apply(x, *_params(self))

@@ -25,8 +25,8 @@ class _Residual(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, k, m, init, ws):
-        mm = m.to(torch.complex64).contiguous()
-        ii = init.to(device=mm.device, dtype=torch.complex64).contiguous()
+        mm = _lib.plain(m.to(torch.complex64))
+        ii = _lib.plain(init.to(device=mm.device, dtype=torch.complex64))
         kk = k.detach().to(torch.float32).contiguous()
         out = torch.empty_like(mm)
         _lib.check(_lib.lib().ptycho_residual(kk.data_ptr(), mm.data_ptr(), ii.data_ptr(), mm.numel(),
@@ -39,7 +39,7 @@ class _Residual(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         kk, mm = ctx.saved_tensors
-        gc = g.to(torch.complex64).contiguous()
+        gc = _lib.plain(g.to(torch.complex64))
         gm = torch.empty_like(mm) if ctx.needs_input_grad[1] else None
         gk = torch.empty((), dtype=torch.float32, device=mm.device)
         _lib.check(_lib.lib().ptycho_residual_backward(

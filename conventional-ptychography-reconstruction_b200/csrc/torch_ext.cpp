@@ -61,6 +61,14 @@ void check(int rc, const char* where) {
   TORCH_CHECK(rc == 0, where, ": ", g_status_string ? g_status_string(rc) : "error", " (status ", rc, ")");
 }
 
+// as a kernel reads it: contiguous, no pending conjugation or negation (contiguous()
+// alone keeps those)
+Tensor plain(Tensor t) {
+  if (t.is_conj()) t = t.resolve_conj();
+  if (t.is_neg()) t = t.resolve_neg();
+  return t.contiguous();
+}
+
 template <typename T>
 T* fptr(const Tensor& t) {
   return t.defined() ? reinterpret_cast<T*>(t.data_ptr()) : nullptr;
@@ -105,8 +113,8 @@ class FusedLoss : public torch::autograd::Function<FusedLoss> {
   static Tensor forward(AutogradContext* ctx, Tensor O, Tensor P, const Tensor& tl, const Tensor& Imeas,
                         int64_t loss_code, const std::optional<Tensor>& batch, const Tensor& status, bool need_grad,
                         int* rc) {
-    O = O.contiguous();
-    P = P.contiguous();
+    O = plain(O);
+    P = plain(P);
     const int64_t H = O.size(0), W = O.size(1), M = P.size(0), N = P.size(1);
     const int64_t F = tl.size(0);
     const bool has_batch = batch.has_value() && batch->defined();
@@ -136,7 +144,7 @@ class FusedLoss : public torch::autograd::Function<FusedLoss> {
     const bool nP = ctx->needs_input_grad(1) && dP.defined() && grads[0].defined();
     Tensor gO, gP;
     if (nO || nP) {
-      Tensor g = grads[0].to(torch::kFloat64).contiguous();
+      Tensor g = plain(grads[0].to(torch::kFloat64));
       gO = nO ? torch::empty_like(dO) : Tensor();
       gP = nP ? torch::empty_like(dP) : Tensor();
       // one launch scales both (out of place: the saved gradients stay valid for a second backward)
@@ -175,7 +183,7 @@ Tensor fused_loss(const Tensor& O, const Tensor& P, const Tensor& tl_in, const T
   c10::cuda::CUDAGuard guard(dev);
   // windows, measurements and frame ids carry no gradient (the node returns none for them)
   const Tensor tl = tl_in.detach().to(dev, torch::kInt32).contiguous();
-  const Tensor Imeas = Imeas_in.detach().to(dev, torch::kFloat32).contiguous();
+  const Tensor Imeas = plain(Imeas_in.detach().to(dev, torch::kFloat32));
   std::optional<Tensor> batch;
   if (batch_in.has_value() && batch_in->defined()) batch = batch_in->detach().to(dev, torch::kInt32).contiguous();
   const int64_t F = tl.dim() == 2 ? tl.size(0) : -1;
@@ -201,8 +209,8 @@ constexpr int kCmlpParams = 11;
 // that is what it is
 Tensor floats_of(const Tensor& p) {
   Tensor t = p.detach();
-  if (t.is_complex()) t = torch::view_as_real(t.resolve_conj().contiguous());
-  return t.contiguous().to(torch::kFloat32);
+  if (t.is_complex()) t = torch::view_as_real(plain(t));
+  return plain(t).to(torch::kFloat32);
 }
 
 // [N, 32] float32 view of a feature-major [32, N] buffer (the encoder's output)
@@ -250,7 +258,7 @@ class Cmlp : public torch::autograd::Function<Cmlp> {
     c10::cuda::CUDAGuard guard(x.device());
     void* s = current_stream(x);
     const int64_t N = x.size(0);
-    const Tensor gy = grads[0].reshape({N}).to(torch::kComplexFloat).resolve_conj().contiguous();
+    const Tensor gy = plain(grads[0].reshape({N}).to(torch::kComplexFloat));
     const int planar = is_planar(x);
     Tensor grad = torch::empty({g_cmlp_grad_floats}, x.options());
     Tensor ws = torch::empty({int64_t(g_cmlp_bwd_ws(int(N)))}, x.options().dtype(torch::kUInt8));
@@ -288,7 +296,7 @@ std::pair<Tensor, int> cmlp(const Tensor& x_in, const std::vector<Tensor>& p, co
   TORCH_CHECK_VALUE(x_in.is_cuda(), "features must be a CUDA tensor (there is no CPU path)");
   TORCH_CHECK_VALUE(p.size() == size_t(kCmlpParams), "the MLP has eleven parameters");
   c10::cuda::CUDAGuard guard(x_in.device());
-  Tensor x = x_in.to(torch::kFloat32);
+  Tensor x = x_in.to(torch::kFloat32).resolve_neg();
   if (!is_planar(x)) x = x.contiguous();
   int rc = 0;
   Tensor y = Cmlp::apply(x, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], p[8], p[9], p[10], status, &rc);
@@ -301,7 +309,7 @@ std::pair<Tensor, int> cmlp(const Tensor& x_in, const std::vector<Tensor>& p, co
 class Upsample : public torch::autograd::Function<Upsample> {
  public:
   static Tensor forward(AutogradContext* ctx, const Tensor& x, int64_t s, int* rc) {
-    const Tensor xc = x.to(torch::kComplexFloat).resolve_conj().contiguous();
+    const Tensor xc = plain(x.to(torch::kComplexFloat));
     const int64_t h = x.size(0), w = x.size(1);
     Tensor y = torch::empty({h * s, w * s}, xc.options());
     Tensor ws = torch::empty({int64_t(g_upsample_ws(int(h), int(w), int(s)))}, xc.options().dtype(torch::kUInt8));
@@ -315,7 +323,7 @@ class Upsample : public torch::autograd::Function<Upsample> {
 
   static tensor_list backward(AutogradContext* ctx, tensor_list grads) {
     const int64_t h = ctx->saved_data["h"].toInt(), w = ctx->saved_data["w"].toInt(), s = ctx->saved_data["s"].toInt();
-    const Tensor g = grads[0].to(torch::kComplexFloat).resolve_conj().contiguous();
+    const Tensor g = plain(grads[0].to(torch::kComplexFloat));
     c10::cuda::CUDAGuard guard(g.device());
     Tensor gx = torch::empty({h, w}, g.options());
     Tensor ws = torch::empty({int64_t(g_upsample_ws(int(h), int(w), int(s)))}, g.options().dtype(torch::kUInt8));

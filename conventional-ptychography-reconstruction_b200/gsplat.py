@@ -26,7 +26,7 @@ RS, CHOLESKY = 0, 1
 def _prep(x, shape, name):
     if not isinstance(x, torch.Tensor) or not x.is_cuda:
         raise ValueError(f"{name} must be a CUDA tensor (there is no CPU path)")
-    return x.detach().to(torch.float32).contiguous().reshape(shape)
+    return _lib.plain(x.detach().to(torch.float32)).reshape(shape)
 
 
 def _forward(kind, xy, p1, p2, weight, H, W, max_patch_radius, min_scale):
@@ -52,7 +52,7 @@ def _backward(kind, saved, ws, H, W, max_patch_radius, min_scale, gout):
     xy_, p1_, p2_, w_ = saved
     N = int(xy_.shape[0])
     dev = xy_.device
-    g = gout.detach().to(torch.float32).contiguous()
+    g = _lib.plain(gout.detach().to(torch.float32))
     dxy = torch.empty((N, 2), dtype=torch.float32, device=dev)
     dp1 = torch.empty((N, 2), dtype=torch.float32, device=dev)
     dp2 = torch.empty(N, dtype=torch.float32, device=dev)

@@ -194,9 +194,10 @@ class _HashFn(torch.autograd.Function):
         N = coords.shape[0]
         dtable = torch.empty(enc.n_entries * 2, dtype=torch.float32, device=coords.device)
         stream = _stream(coords.device)
-        planar = gout.dtype == torch.float32 and gout.dim() == 2 and N > 1 and gout.stride() == (1, N)
+        planar = (gout.dtype == torch.float32 and gout.dim() == 2 and N > 1 and gout.stride() == (1, N)
+                  and not gout.is_neg())
         if not planar:
-            gout = gout.contiguous().float()
+            gout = _lib.plain(gout).float()
         if isinstance(plan, GridPlan):
             ext = plan.hl.ctypes.data
             _lib.check(_lib.lib().ptycho_hashgrid_backward_grid(
@@ -210,7 +211,7 @@ class _HashFn(torch.autograd.Function):
                 plan.start.data_ptr(), plan.item_planar.data_ptr(), plan.weight.data_ptr(), gout.data_ptr(), N,
                 *enc.cfg, dtable.data_ptr(), 0, stream), "ptycho_hashgrid_backward_planar")
             return None, dtable, None
-        gout = gout.contiguous().float()
+        gout = _lib.plain(gout).float()
         _lib.check(_lib.lib().ptycho_hashgrid_backward(
             plan.start.data_ptr(), plan.item.data_ptr(), plan.weight.data_ptr(), gout.data_ptr(),
             N, *enc.cfg, dtable.data_ptr(), 0, stream), "ptycho_hashgrid_backward")
@@ -311,5 +312,5 @@ class Encoding(torch.nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if not x.is_cuda:
             raise ValueError("coordinates must be a CUDA tensor (there is no CPU path)")
-        x = x.float().contiguous()
+        x = _lib.plain(x.float())
         return _HashFn.apply(x, self.params, self)

@@ -104,7 +104,7 @@ def _as_c64(x: torch.Tensor, name: str) -> torch.Tensor:
         raise ValueError(f"{name} must be a CUDA tensor (there is no CPU path)")
     if x.dtype != torch.complex64:
         x = x.to(torch.complex64)
-    return x.contiguous()
+    return _lib.plain(x)
 
 
 def _check_probe(P: torch.Tensor):
@@ -215,8 +215,8 @@ def fwd_adj_raw(O, P, tl, Imeas, loss_code: int, batch=None, want_grad: bool = T
     dev = O.device
     tl = _i32(tl, dev)
     F = int(tl.shape[0])
-    if Imeas.dtype != torch.float32 or not Imeas.is_contiguous() or Imeas.device != dev:
-        Imeas = Imeas.to(device=dev, dtype=torch.float32).contiguous()
+    if Imeas.dtype != torch.float32 or not Imeas.is_contiguous() or Imeas.is_neg() or Imeas.device != dev:
+        Imeas = _lib.plain(Imeas.to(device=dev, dtype=torch.float32))
     if Imeas.shape != (F, M, N):
         raise ValueError(f"measurements must be [F, M, N] = {(F, M, N)}, got {tuple(Imeas.shape)}")
     bt = _batch_arg(batch, dev)
@@ -274,8 +274,8 @@ class FwdAdjPlan:
             raise ValueError(f"loss_type must be one of {tuple(LOSS_CODES)}")
         for name, x, dt in (("object", O, torch.complex64), ("probe", P, torch.complex64),
                             ("windows", tl, torch.int32), ("measurements", Imeas, torch.float32)):
-            if not x.is_cuda or x.dtype != dt or not x.is_contiguous():
-                raise ValueError(f"{name} must be a contiguous CUDA {dt} tensor")
+            if not x.is_cuda or x.dtype != dt or not x.is_contiguous() or x.is_conj() or x.is_neg():
+                raise ValueError(f"{name} must be a contiguous CUDA {dt} tensor without a pending conjugation")
         self.M, self.N = _check_probe(P)
         self.O, self.P, self.tl, self.Imeas = O, P, tl, Imeas
         self.dev = O.device
@@ -345,7 +345,7 @@ class _FusedLoss(torch.autograd.Function):
         if not ctx.need:
             return None, None, None, None, None, None
         dO, dP = ctx.saved_tensors
-        s = g if g.dtype == torch.float64 and g.is_contiguous() else g.to(torch.float64).contiguous()
+        s = g if g.dtype == torch.float64 and g.is_contiguous() and not g.is_neg() else _lib.plain(g.to(torch.float64))
         gO = torch.empty_like(dO) if ctx.needs_input_grad[0] else None
         gP = torch.empty_like(dP) if ctx.needs_input_grad[1] else None
         # one launch scales both gradients by the upstream scalar (out of place:
@@ -392,7 +392,7 @@ class _ForwardIntensity(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gI):
         O, P, tl = ctx.saved_tensors
-        _, _, dO, dP = fwd_adj_raw(O.detach(), P.detach(), tl, gI.contiguous(), _INTENSITY_GRAD)
+        _, _, dO, dP = fwd_adj_raw(O.detach(), P.detach(), tl, _lib.plain(gI), _INTENSITY_GRAD)
         return (dO if ctx.needs_input_grad[0] else None,
                 dP if ctx.needs_input_grad[1] else None, None)
 

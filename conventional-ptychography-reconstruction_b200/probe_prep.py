@@ -21,7 +21,7 @@ class _ProbePrep(torch.autograd.Function):
     @staticmethod
     def forward(ctx, P):
         M, N = P.shape
-        Pc = P.to(torch.complex64).contiguous()
+        Pc = _lib.plain(P.to(torch.complex64))
         out = torch.empty((M, N), dtype=torch.complex64, device=P.device)
         state = torch.empty(4, dtype=torch.float64, device=P.device)
         _lib.check(_lib.lib().ptycho_probe_center_normalize(
@@ -34,7 +34,7 @@ class _ProbePrep(torch.autograd.Function):
     def backward(ctx, g):
         out, state = ctx.saved_tensors
         M, N = out.shape
-        gc = g.to(torch.complex64).contiguous()
+        gc = _lib.plain(g.to(torch.complex64))
         gin = torch.empty((M, N), dtype=torch.complex64, device=g.device)
         _lib.check(_lib.lib().ptycho_probe_center_normalize_backward(
             out.data_ptr(), state.data_ptr(), gc.data_ptr(), M, N, gin.data_ptr(),
@@ -55,7 +55,7 @@ class _Haar(torch.autograd.Function):
     @staticmethod
     def forward(ctx, img):
         H, W = img.shape
-        x = img.to(torch.complex64).contiguous()
+        x = _lib.plain(img.to(torch.complex64))
         loss = torch.empty((), dtype=torch.float64, device=img.device)
         n = int(_lib.lib().ptycho_haar_sparsity_workspace_size(H, W))
         ws = torch.empty(max(n, 8), dtype=torch.uint8, device=img.device)
@@ -69,7 +69,7 @@ class _Haar(torch.autograd.Function):
     def backward(ctx, g):
         (x,) = ctx.saved_tensors
         H, W = x.shape
-        gd = g.to(torch.float64).contiguous()
+        gd = _lib.plain(g.to(torch.float64))
         gin = torch.empty_like(x)
         _lib.check(_lib.lib().ptycho_haar_sparsity_backward(x.data_ptr(), H, W, gd.data_ptr(), gin.data_ptr(),
                                                             torch.cuda.current_stream(x.device).cuda_stream),

@@ -36,7 +36,7 @@ class _FourierUpsample(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, s: int):
         h, w = x.shape
-        xc = x.to(torch.complex64).resolve_conj().contiguous()
+        xc = _lib.plain(x.to(torch.complex64))
         y = torch.empty((h * s, w * s), dtype=torch.complex64, device=x.device)
         ws, n = _workspace(h, w, s, x.device)
         _lib.check(_lib.lib().ptycho_fourier_upsample(
@@ -48,7 +48,7 @@ class _FourierUpsample(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gy):
         h, w, s = ctx.shape
-        g = gy.to(torch.complex64).resolve_conj().contiguous()
+        g = _lib.plain(gy.to(torch.complex64))
         gx = torch.empty((h, w), dtype=torch.complex64, device=g.device)
         ws, n = _workspace(h, w, s, g.device)
         _lib.check(_lib.lib().ptycho_fourier_upsample_adjoint(
