@@ -45,6 +45,19 @@ def _params(net):
             layers[3].weight, layers[3].bias]
 
 
+# values and type (complex or not) that the library reads at each of _params' addresses
+_SIZES = ((1024, False), (32, False), (1, False), (1024, True), (32, True), (1, False),
+          (1024, True), (32, True), (1, False), (32, True), (1, True))
+
+
+def _check_params(params, device):
+    for i, (p, (n, cplx)) in enumerate(zip(params, _SIZES)):
+        if p.device != device:
+            raise ValueError(f"parameter {i} of the MLP is on {p.device}, the features are on {device}")
+        if p.numel() != n or p.is_complex() != cplx:
+            raise ValueError(f"parameter {i} of the MLP has shape {tuple(p.shape)} and type {p.dtype}")
+
+
 def _f32(t):
     t = t.detach()
     if t.is_complex():
@@ -122,8 +135,10 @@ class _FusedSequential(nn.Sequential):
     def forward(self, x):  # noqa: D401
         if not x.is_cuda:
             raise ValueError("features must be a CUDA tensor (there is no CPU path)")
+        if x.dim() != 2 or x.shape[1] != 32:
+            raise ValueError(f"features must be [N, 32], got {tuple(x.shape)}")
         ext = _lib.torchext() if optics.USE_TORCHEXT else None
-        if ext is not None and x.dim() == 2 and x.shape[1] == 32:
+        if ext is not None:
             # the C++ autograd node: the same library calls, no Python in forward or backward
             l0, l1, l2, out = self
             y, rc = ext.cmlp(x, [l0.omega_0, l0.linear.weight, l0.linear.bias, l1.omega_0, l1.linear.weight,
@@ -134,7 +149,9 @@ class _FusedSequential(nn.Sequential):
         x = x.float().resolve_neg()
         if not _is_planar(x):
             x = x.contiguous()
-        return _CmlpFn.apply(x, *_params(self))
+        params = _params(self)
+        _check_params(params, x.device)
+        return _CmlpFn.apply(x, *params)
 
 
 class ComplexMLP(nn.Module):

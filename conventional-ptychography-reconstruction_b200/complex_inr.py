@@ -25,15 +25,19 @@ class _Residual(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, k, m, init, ws):
+        if not m.is_cuda:
+            raise ValueError("the network's output must be a CUDA tensor (there is no CPU path)")
+        if init.numel() != m.numel():
+            raise ValueError(f"the initial estimate is {tuple(init.shape)}, the network's output {tuple(m.shape)}")
         mm = _lib.plain(m.to(torch.complex64))
         ii = _lib.plain(init.to(device=mm.device, dtype=torch.complex64))
-        kk = k.detach().to(torch.float32).contiguous()
+        kk = k.detach().to(device=mm.device, dtype=torch.float32).contiguous()
         out = torch.empty_like(mm)
         _lib.check(_lib.lib().ptycho_residual(kk.data_ptr(), mm.data_ptr(), ii.data_ptr(), mm.numel(),
                                               out.data_ptr(), torch.cuda.current_stream(mm.device).cuda_stream),
                    "ptycho_residual")
         ctx.save_for_backward(kk, mm)
-        ctx.ws, ctx.kshape = ws, k.shape
+        ctx.ws, ctx.kshape, ctx.kdev = ws, k.shape, k.device
         return out
 
     @staticmethod
@@ -46,7 +50,7 @@ class _Residual(torch.autograd.Function):
             kk.data_ptr(), mm.data_ptr(), gc.data_ptr(), mm.numel(), gm.data_ptr() if gm is not None else None,
             gk.data_ptr(), ctx.ws.data_ptr(), ctx.ws.numel(), torch.cuda.current_stream(mm.device).cuda_stream),
             "ptycho_residual_backward")
-        return (gk.reshape(ctx.kshape) if ctx.needs_input_grad[0] else None, gm,
+        return (gk.reshape(ctx.kshape).to(ctx.kdev) if ctx.needs_input_grad[0] else None, gm,
                 g if ctx.needs_input_grad[2] else None, None)
 
 

@@ -294,7 +294,23 @@ class Cmlp : public torch::autograd::Function<Cmlp> {
 std::pair<Tensor, int> cmlp(const Tensor& x_in, const std::vector<Tensor>& p, const Tensor& status) {
   TORCH_CHECK(g_cmlp_pack && g_cmlp_bwd_ws, "bind_inr() was not called");
   TORCH_CHECK_VALUE(x_in.is_cuda(), "features must be a CUDA tensor (there is no CPU path)");
+  TORCH_CHECK_VALUE(x_in.dim() == 2 && x_in.size(1) == 32, "features must be [N, 32], got ", x_in.sizes());
   TORCH_CHECK_VALUE(p.size() == size_t(kCmlpParams), "the MLP has eleven parameters");
+  // the library reads these sizes at the parameters' addresses
+  struct Want {
+    int64_t numel;
+    bool cplx;
+  };
+  static constexpr Want want[kCmlpParams] = {{1, false}, {1024, false}, {32, false}, {1, false}, {1024, true}, {32, true},
+                                             {1, false}, {1024, true},  {32, true},  {32, true}, {1, true}};
+  for (int i = 0; i < kCmlpParams; ++i) {
+    TORCH_CHECK_VALUE(p[i].device() == x_in.device(), "parameter ", i, " of the MLP is on ", p[i].device(),
+                      ", the features are on ", x_in.device());
+    TORCH_CHECK_VALUE(p[i].numel() == want[i].numel && p[i].is_complex() == want[i].cplx, "parameter ", i,
+                      " of the MLP has shape ", p[i].sizes(), " and type ", p[i].scalar_type());
+  }
+  TORCH_CHECK_VALUE(status.device() == x_in.device() && status.scalar_type() == torch::kInt32,
+                    "status must be the device's int32 status word");
   c10::cuda::CUDAGuard guard(x_in.device());
   Tensor x = x_in.to(torch::kFloat32).resolve_neg();
   if (!is_planar(x)) x = x.contiguous();

@@ -312,5 +312,12 @@ class Encoding(torch.nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if not x.is_cuda:
             raise ValueError("coordinates must be a CUDA tensor (there is no CPU path)")
+        if x.dim() != 2 or x.shape[1] != 2:
+            raise ValueError(f"coordinates must be [N, 2], got {tuple(x.shape)}")
+        t = self.params
+        if t.device != x.device:
+            raise ValueError(f"the table is on {t.device}, the coordinates are on {x.device}")
+        if t.dtype != torch.float32 or t.numel() != 2 * self.n_entries or not t.is_contiguous():
+            raise ValueError(f"the table must be {2 * self.n_entries} contiguous float32, got {t.numel()} {t.dtype}")
         x = _lib.plain(x.float())
         return _HashFn.apply(x, self.params, self)

@@ -176,6 +176,8 @@ def forward_intensity(O: torch.Tensor, P: torch.Tensor, tl: torch.Tensor, batch=
     all F frames in order)."""
     O = _as_c64(O, "object")
     P = _as_c64(P, "probe")
+    if P.device != O.device:
+        raise ValueError("object and probe must be on one device")
     M, N = _check_probe(P)
     H, W = O.shape
     tl = tl.to(device=O.device, dtype=torch.int32).contiguous()
@@ -210,6 +212,8 @@ def fwd_adj_raw(O, P, tl, Imeas, loss_code: int, batch=None, want_grad: bool = T
     allocated unless given (``accumulate`` adds into given buffers)."""
     O = _as_c64(O, "object")
     P = _as_c64(P, "probe")
+    if P.device != O.device:
+        raise ValueError("object and probe must be on one device")
     M, N = _check_probe(P)
     H, W = O.shape
     dev = O.device
