@@ -1030,7 +1030,8 @@ static int cmlp_backward(int planar, const void* packed, const float* x, const f
                          float* y, void* workspace, size_t workspace_bytes, int32_t* status_out,
                          ptycho_stream_t stream) {
   if (!packed || !grad || N < 0 || (N > 0 && (!x || !gy))) return PTYCHO_ERR_INVALID_ARG;
-  if (!pty_aligned(packed, 16) || !pty_aligned(x, 16) || !pty_aligned(gy, 8) || !pty_aligned(gx, 16) ||
+  const size_t ax = planar ? 4 : 16;  // feature-major values are read and written one by one
+  if (!pty_aligned(packed, 16) || !pty_aligned(x, ax) || !pty_aligned(gy, 8) || !pty_aligned(gx, ax) ||
       !pty_aligned(y, 8))
     return PTYCHO_ERR_MISALIGNED;
   if (!workspace || workspace_bytes < ptycho_cmlp_backward_workspace_size(N)) return PTYCHO_ERR_WORKSPACE;
