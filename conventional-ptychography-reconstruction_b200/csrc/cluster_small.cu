@@ -25,6 +25,7 @@
 
 #include "dft_regs.cuh"
 #include "fused.cuh"
+#include "launch_retry.cuh"
 
 namespace pty {
 namespace csm {
@@ -335,18 +336,18 @@ static int launch(const FusedArgs& a, cudaStream_t s) {
   cfg.numAttrs = 1;
   static PtyDevCache attr;  // attributes set
   int dev = 0;
-  for (int attempt = 0; attempt < 2; ++attempt) {
-    if (!attr.get(&dev)) {
-      if (dev < 0 ||
-          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(F::SMEM)) != cudaSuccess ||
-          (F::C > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess))
-        return PTYCHO_ERR_LAUNCH;
-      attr.put(dev, 1);
-    }
-    if (cudaLaunchKernelEx(&cfg, kern, a) == cudaSuccess && cudaGetLastError() == cudaSuccess) return PTYCHO_OK;
-    attr.put(dev, 0);
-  }
-  return PTYCHO_ERR_LAUNCH;
+  const bool ok = launch_retry(
+      [&](bool again) {
+        if (!again && attr.get(&dev)) return true;
+        if (dev < 0 ||
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(F::SMEM)) != cudaSuccess ||
+            (F::C > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess))
+          return false;
+        attr.put(dev, 1);
+        return true;
+      },
+      [&] { return int(cudaLaunchKernelEx(&cfg, kern, a)); }, [] { return int(cudaGetLastError()); });
+  return ok ? PTYCHO_OK : PTYCHO_ERR_LAUNCH;
 }
 
 template <int M>
