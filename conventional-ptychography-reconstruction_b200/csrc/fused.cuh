@@ -397,8 +397,12 @@ constexpr int kIntensityChunk = PTY_S256_INTENSITY_CHUNK;
 size_t split256_intensity_scratch(int B);
 int split256_intensity(FusedArgs a, void* scratch, cudaStream_t s);
 
-// cluster_small.cu: a pattern per cluster of M / 16 CTAs, any mode and loss
+// cluster_small.cu: a pattern per thread-block cluster (those that small_batch_max lets
+// through; at M = 256 without large_clusters only the FD loss and intensities)
 int launch_small(int M, int mode, int loss, const FusedArgs& a, cudaStream_t s);
+
+// whether the current device can hold clusters of 16 CTAs, asked once per device
+bool large_clusters();
 
 // Largest batch that the cluster kernel takes: where a pattern per SM (or, at M =
 // 256, the line kernels' three launches) leaves SMs idle.  Measured, us a step on a
@@ -408,11 +412,12 @@ int launch_small(int M, int mode, int loss, const FusedArgs& a, cudaStream_t s);
 // better (10 25.0 : 24.6), M = 128 10 27.1 : 49.8, 100 50.0 : 53.8, 148 64.6 : 57.9,
 // M = 256 always (10 33.5 : 78.4, 200 347 : 532 for a 4-CTA cluster kernel).
 // M = 256 intensities: 20 16.2 : 18.7, 64 37.3 : 24.0.
+// Without clusters of 16, which M = 256 takes, the line kernels run what they can.
 inline int small_batch_max(int M, int mode, int loss) {
   const bool fd = mode != MODE_INTENSITY && loss == PTYCHO_LOSS_FD;
   if (M == 64) return fd ? 0 : 16;
   if (M == 128) return fd ? 96 : 64;
-  return fd ? 0x7fffffff : (mode == MODE_INTENSITY ? 24 : 4);
+  return fd ? 0x7fffffff : (mode == MODE_INTENSITY ? 24 : (large_clusters() ? 4 : 0));
 }
 
 }  // namespace pty
