@@ -10,8 +10,8 @@
 //
 // A CTA holds `lines` lines in two ping-pong buffers; the inverse transform is
 // conj(DFT(conj)), so only forward passes exist.  Twiddles are
-// tables in shared memory built per CTA in FP32 (cis_ratio below: correct to about
-// an ulp; building them in FP64 took a third of the short kernels).  Index
+// tables in shared memory built per CTA, in FP64 and rounded once (cis_ratio below;
+// with sincospi they took a third of the short kernels).  Index
 // divisions are multiplications by reciprocals from the plan.
 #pragma once
 #include "common.cuh"
@@ -116,16 +116,27 @@ inline bool make_plan(int n, int extra_tables, Plan* p) {
   return set_passes(p, n, r, np + q);
 }
 
-// exp(-2 pi i num / den), 0 <= num < den: the quotient's rounding error is put
-// back to first order, so the result is good to about an ulp
+// exp(-2 pi i num / den), 0 <= num < den, rounded once: the angle is taken to a
+// quarter turn's half, [-pi/4, pi/4], in whole numbers, then cos and sin are their
+// Taylor sums in FP64 (to 1e-10; about twenty instructions)
 PTY_DEVI float2 cis_ratio(int num, int den) {
-  if (2 * num > den) num -= den;  // to (-1/2, 1/2]
-  const float a = 2.0f * float(num), d = float(den);
-  const float x = a / d;
-  const float r = fmaf(-x, d, a) / d * 3.14159265358979f;  // pi times what x misses
-  float s, c;
-  sincospif(x, &s, &c);
-  return make_float2(fmaf(-s, r, c), -fmaf(c, r, s));
+  const double inv = 1.57079632679489662 / double(den);  // one division per loop
+  const int q = __float2int_rn(4.0f * float(num) / float(den));
+  const double x = double(4 * num - q * den) * inv, y = x * x;
+  double c = -1.0 / 3628800.0, s = -1.0 / 39916800.0;
+  c = fma(c, y, 1.0 / 40320.0);
+  s = fma(s, y, 1.0 / 362880.0);
+  c = fma(c, y, -1.0 / 720.0);
+  s = fma(s, y, -1.0 / 5040.0);
+  c = fma(c, y, 1.0 / 24.0);
+  s = fma(s, y, 1.0 / 120.0);
+  c = fma(c, y, -0.5);
+  s = fma(s, y, -1.0 / 6.0);
+  c = fma(c, y, 1.0);
+  s = fma(s * y, x, x);
+  const float fc = float(c), fs = float(s);
+  const float u = q & 1 ? fs : fc, v = q & 1 ? fc : fs;   // q quarter turns further
+  return make_float2((q + 1) & 2 ? -u : u, q & 2 ? v : -v);
 }
 
 // where value i of line l lives: LINES = 0: whole lines, one float2 of padding
