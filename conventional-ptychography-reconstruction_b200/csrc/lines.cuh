@@ -2,11 +2,11 @@
 //
 // Smooth lengths run as Stockham passes of register butterflies, radix 2 to 16
 // (dft_small.cuh), planned on the host for the fewest passes: 192 = 16 x 12, 1500 =
-// 15 x 10 x 10.  A length with a larger prime factor runs as Bluestein's
+// 15 x 10 x 10.  Larger primes up to kDirectPrime are passes of their own, summed in
+// pairs (pass_prime).  A length with a prime factor beyond that runs as Bluestein's
 // convolution of smooth length m >= 2n - 1 (two transforms of length m and three
-// diagonals; a 317-point line costs about two 640-point ones, where a direct sum
-// over the factor 317 costs 317 terms a value), or, when its tables do not fit
-// shared memory (n beyond about 2500), with direct-sum passes for the large primes.
+// diagonals; a 317-point line costs about two 640-point ones), or, when its tables do
+// not fit shared memory (n beyond about 2500), with the pair sums too.
 //
 // A CTA holds `lines` lines in two ping-pong buffers; the inverse transform is
 // conj(DFT(conj)), so only forward passes exist.  Twiddles are
@@ -23,6 +23,14 @@ namespace ln {
 constexpr int kMaxPasses = 8;
 constexpr int kMaxLen = 8192;
 constexpr size_t kSmemCap = 200 * 1024;
+// Largest prime that is summed directly.  The pair sums are closer to 64 bits than a
+// plain direct sum (0.46 to 0.81 of its error for any prime); Bluestein's chirp transform
+// adds an error of its own, 1.2 to 2.1 times the plain sum's for most lengths with a prime
+// of 17 to 47 and up to 1.25 at 149, always below it (0.4 to 0.8) from 157 on.  Steps of
+// 64 patterns on B200, pairs : Bluestein: 119^2 86 : 133 us, 148^2 131 : 209, 194^2 297 :
+// 470, 226^2 393 : 469, 127^2 165 : 135, 254^2 513 : 552, 149^2 248 : 213, 179^2 380 :
+// 357, 251^2 812 : 530.
+constexpr int kDirectPrime = 151;
 
 struct Pass {
   int R, NS, bpl, tws;   // radix, product of the radices before, butterflies per line, twiddle stride
@@ -32,6 +40,7 @@ struct Plan {
   int n;             // line length
   int m;             // transform length: n, or Bluestein's convolution length
   int blue;
+  int ls;            // distance of whole lines in shared memory
   int np;
   unsigned m_n;      // reciprocal of n
   Pass p[kMaxPasses];
@@ -61,6 +70,8 @@ inline int factor_smooth(int L, int* r, int limit) {
 inline bool set_passes(Plan* p, int m, const int* r, int np) {
   p->m = m;
   p->np = np;
+  p->ls = (m - 1) + ((m - 1) >> 4) + 1;
+  if (np && r[0] > 16) p->ls |= 1;  // pass_prime's neighbouring threads: lines on other banks
   int ns = 1;
   for (int i = 0; i < np; ++i) {
     Pass& q = p->p[i];
@@ -76,9 +87,8 @@ inline bool set_passes(Plan* p, int m, const int* r, int np) {
 }
 
 // shared memory of a CTA with `lines` lines
-inline int line_stride(int m) { return (m - 1) + ((m - 1) >> 4) + 1; }
 inline size_t smem_bytes(const Plan& p, int lines, int extra_tables) {
-  size_t n = size_t(2) * lines * line_stride(p.m) + p.m;
+  size_t n = size_t(2) * lines * p.ls + p.m;
   if (p.blue) n += size_t(p.m) + p.n;
   return (n + size_t(extra_tables) * p.n) * sizeof(float2);
 }
@@ -92,7 +102,10 @@ inline bool make_plan(int n, int extra_tables, Plan* p) {
   int r[kMaxPasses];
   const int k = factor_smooth(n, r, kMaxPasses);
   if (k >= 0) return set_passes(p, n, r, k);
-  for (int m = 2 * n - 1; m <= 2 * kMaxLen; ++m) {  // the next length of no more passes than its size needs
+  int big = n;  // the largest prime factor
+  for (int f = 2; f * f <= big; ++f)
+    while (big > f && big % f == 0) big /= f;
+  for (int m = 2 * n - 1; big > kDirectPrime && m <= 2 * kMaxLen; ++m) {  // the next length of no more passes than its size needs
     const int want = m <= 256 ? 2 : (m <= 4096 ? 3 : 4);
     const int q = factor_smooth(m, r, want);
     if (q < 0) continue;
@@ -101,7 +114,7 @@ inline bool make_plan(int n, int extra_tables, Plan* p) {
     if (smem_bytes(*p, 1, extra_tables) <= kSmemCap) return true;
     break;
   }
-  p->blue = 0;  // direct-sum passes for the primes above 13
+  p->blue = 0;  // pair sums for the primes above 13
   int np = 0, rest = n;
   for (int f = 17; f <= rest; f += 2)
     while (rest % f == 0 && np < kMaxPasses) {
@@ -148,19 +161,25 @@ PTY_DEVI int slot(int l, int i, int ls) {
   else return (i + (i >> 4)) * LINES + l;
 }
 
+// butterfly b of the CTA -> its line and place
+template <int LINES>
+PTY_DEVI void line_place(const Pass& ps, int b, int& l, int& j) {
+  if constexpr (LINES == 0) {
+    l = fdiv(b, ps.m_bpl);
+    j = b - l * ps.bpl;
+  } else {
+    l = b % LINES;
+    j = b / LINES;
+  }
+}
+
 template <int LINES, int NT, int R>
 PTY_DEVI void pass_r(const Pass& ps, const float2* __restrict__ src, float2* __restrict__ dst,
                      const float2* __restrict__ tw, int lines, int ls, int t) {
   const int nb = lines * ps.bpl;
   for (int b = t; b < nb; b += NT) {
     int l, j;
-    if constexpr (LINES == 0) {
-      l = fdiv(b, ps.m_bpl);
-      j = b - l * ps.bpl;
-    } else {
-      l = b % LINES;
-      j = b / LINES;
-    }
+    line_place<LINES>(ps, b, l, j);
     const int k = j - fdiv(j, ps.m_ns) * ps.NS;
     float2 v[R];
 #pragma unroll
@@ -180,29 +199,77 @@ PTY_DEVI void pass_r(const Pass& ps, const float2* __restrict__ src, float2* __r
   }
 }
 
-// direct sum for a prime radix p: output o = (j / NS) NS p + k + r NS gets
-// sum_m x[j + m L/p] exp(-2 pi i m (k + r NS) / (NS p))
-template <int LINES, int NT>
-PTY_DEVI void pass_direct(const Pass& ps, int len, const float2* __restrict__ src, float2* __restrict__ dst,
-                          const float2* __restrict__ tw, int lines, int ls, int t) {
-  const int p = ps.R, blk = ps.NS * p;
-  for (int e = t; e < lines * len; e += NT) {
-    const int l = LINES == 0 ? e / len : e % lines, o = LINES == 0 ? e - l * len : e / lines;
-    const int ob = o / blk, rem = o - ob * blk;
-    const int r = rem / ps.NS, k = rem - r * ps.NS;
-    const int j = ob * ps.NS + k;
-    const int q = (k + r * ps.NS) * ps.tws;  // < len
-    float2 acc = make_float2(0.f, 0.f);
-    int idx = 0;
-    for (int m = 0; m < p; ++m) {
-      const float2 w = tw[idx], x = src[slot<LINES>(l, j + m * ps.bpl, ls)];
-      acc.x = fmaf(x.x, w.x, fmaf(-x.y, w.y, acc.x));
-      acc.y = fmaf(x.x, w.y, fmaf(x.y, w.x, acc.y));
-      idx += q;
-      if (idx >= len) idx -= len;
+// A prime radix p beyond the register butterflies, in the symmetric pair form at run
+// time: twiddled inputs m and p - m become their sum and difference, in place, and
+// outputs r and p - r are sum_m (sum_m cos +- i diff_m sin).  A thread sums R
+// such r, so that a pair is read once for 4 R products; R of 2 to 4 by the rounds that
+// the CTA needs (a round of R costs about 2 + 8 R for each pair).
+template <int LINES, int NT, int R>
+PTY_DEVI void prime_sums(const Pass& ps, int len, const float2* __restrict__ src, float2* __restrict__ dst,
+                         const float2* __restrict__ tw, int lines, int ls, int t) {
+  const int p = ps.R, h = (p - 1) / 2, nb = lines * ps.bpl;
+  for (int e = t; e < nb * ((h + R) / R); e += NT) {
+    const int r0 = e / nb * R;  // r0 .. r0 + R - 1, of 0 .. h
+    const int b = e - e / nb * nb;
+    int l, j;
+    line_place<LINES>(ps, b, l, j);
+    const float2 x0 = src[slot<LINES>(l, j, ls)];
+    float2 a[R], d[R];  // sums by cos, differences by -sin
+    int idx[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      a[i] = x0;
+      d[i] = make_float2(0.f, 0.f);
+      idx[i] = 0;
     }
-    dst[slot<LINES>(l, o, ls)] = acc;
+#pragma unroll 1
+    for (int m = 1; m <= h; ++m) {
+      const float2 u = src[slot<LINES>(l, j + m * ps.bpl, ls)], v = src[slot<LINES>(l, j + (p - m) * ps.bpl, ls)];
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        idx[i] += (r0 + i) * ps.bpl;
+        if (idx[i] >= len) idx[i] -= len;
+        const float2 w = tw[idx[i]];
+        a[i] = make_float2(fmaf(u.x, w.x, a[i].x), fmaf(u.y, w.x, a[i].y));
+        d[i] = make_float2(fmaf(v.x, w.y, d[i].x), fmaf(v.y, w.y, d[i].y));
+      }
+    }
+    const int k = j - fdiv(j, ps.m_ns) * ps.NS, o = (j - k) * p + k;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const int r = r0 + i;
+      if (r > h) break;
+      dst[slot<LINES>(l, o + r * ps.NS, ls)] = make_float2(a[i].x - d[i].y, a[i].y + d[i].x);
+      if (r > 0) dst[slot<LINES>(l, o + (p - r) * ps.NS, ls)] = make_float2(a[i].x + d[i].y, a[i].y - d[i].x);
+    }
   }
+}
+
+template <int LINES, int NT>
+PTY_DEVI void pass_prime(const Pass& ps, int len, float2* __restrict__ src, float2* __restrict__ dst,
+                         const float2* __restrict__ tw, int lines, int ls, int t) {
+  const int p = ps.R, h = (p - 1) / 2, nb = lines * ps.bpl;
+  int l, j;
+#pragma unroll 1
+  for (int e = t; e < nb * h; e += NT) {
+    const int m = e / nb + 1;
+    line_place<LINES>(ps, e - (m - 1) * nb, l, j);
+    float2 &u = src[slot<LINES>(l, j + m * ps.bpl, ls)], &v = src[slot<LINES>(l, j + (p - m) * ps.bpl, ls)];
+    float2 x = u, y = v;
+    if (ps.NS > 1) {
+      const int k = j - fdiv(j, ps.m_ns) * ps.NS;
+      x = c_mul(x, tw[m * k * ps.tws]);
+      y = c_mul(y, tw[(p - m) * k * ps.tws]);
+    }
+    u = c_add(x, y);
+    v = c_sub(x, y);
+  }
+  __syncthreads();
+  const auto cost = [&](int R) { return (nb * ((h + R) / R) + NT - 1) / NT * (2 + 8 * R); };
+  const int c2 = cost(2), c3 = cost(3), c4 = cost(4);
+  if (c2 <= c3 && c2 <= c4) prime_sums<LINES, NT, 2>(ps, len, src, dst, tw, lines, ls, t);
+  else if (c3 <= c4) prime_sums<LINES, NT, 3>(ps, len, src, dst, tw, lines, ls, t);
+  else prime_sums<LINES, NT, 4>(ps, len, src, dst, tw, lines, ls, t);
 }
 
 // The lines and tables of a CTA of NT threads.  Use: put() every value of every
@@ -218,7 +285,7 @@ struct Lines {
   // lays out shared memory and builds the tables; returns the first free float2
   PTY_DEVI float2* init(const Plan& p, float2* smem, int nlines, int tid) {
     lines = nlines;
-    ls = (p.m - 1) + ((p.m - 1) >> 4) + 1;
+    ls = p.ls;
     t = tid;
     cur = smem;
     alt = cur + lines * ls;
@@ -272,7 +339,7 @@ struct Lines {
         PTY_LN(2) PTY_LN(3) PTY_LN(4) PTY_LN(5) PTY_LN(6) PTY_LN(7) PTY_LN(8) PTY_LN(9) PTY_LN(10) PTY_LN(11)
         PTY_LN(12) PTY_LN(13) PTY_LN(15) PTY_LN(16)
 #undef PTY_LN
-        default: pass_direct<LINES, NT>(ps, p.m, cur, alt, tw, lines, ls, t); break;
+        default: pass_prime<LINES, NT>(ps, p.m, cur, alt, tw, lines, ls, t); break;
       }
       __syncthreads();
       float2* c = cur;

@@ -274,7 +274,7 @@ static int dispatch(int n, const Args& g, cudaStream_t st) {
 // or odd n and odd N; d = -1 for odd n and even N (the reference's half-bin
 // asymmetry, kept): every sample j of the long line is turned by exp(2 pi i d j / N).
 // Measured on B200: 1500^2 to 3000^2 71 + 118 us against 213 + 141 by padded spectra
-// with run-time radix loops; 498^2 to 996^2 and back 160 against 675 us (factor 83).
+// with run-time radix loops; 498^2 to 996^2 and back 118 against 675 us (factor 83).
 // ---------------------------------------------------------------------------
 namespace rsg {
 
@@ -449,7 +449,10 @@ static int launch(int n, int s, const float2* in, float2* out, int nlines, long 
     // 16 adjacent columns (128-byte pieces) while two CTAs fit an SM, else 4 or 1; four
     // long columns leave room for one CTA, so it has 1024 threads (1500^2 by 2, up and
     // down: 419 us with 512, 403 with 768, 395 with 1024)
-    if (smem_of(g, 16) <= 112 * 1024) {
+    // lines with a large prime compute for long: four columns per CTA while 16 would leave
+    // SMs idle (249^2 by 2 133 -> 83-99 us, 255^2 107 -> 75, 222 x 333 by 3 123 -> 97)
+    const bool few = g.plan.np && g.plan.p[0].R > 16 && (nlines + 15) / 16 * (ADJ ? 1 : s - 1) < 148;
+    if (smem_of(g, 16) <= 112 * 1024 && !few) {
       groups(16);
       return launch_k<16, 256, ADJ>(g, st);
     }
