@@ -198,9 +198,13 @@ __global__ void __launch_bounds__(kNT, LINES == 16 ? 4 : 2) k_cols(const Args g)
       }
       ln.put(g.plan, cl, p, v);
     }
-    ln.pad(g.plan);
-    ln.run(g.plan);
-    if (g.mode == COLS_LOSS || g.mode == COLS_GRAD) {
+    // forward (COLS_FD_INV: inverse); COLS_GRAD comes back with the gradient's columns
+    // for a second transform (a loop, so that the passes' code is there once)
+#pragma unroll 1
+    for (int back = 0;; ++back) {
+      ln.pad(g.plan);
+      ln.run(g.plan);
+      if (back || (g.mode != COLS_LOSS && g.mode != COLS_GRAD)) break;
       double acc = 0.0;
 #pragma unroll 4
       for (int p = t / LINES; p < M; p += kNT / LINES) {
@@ -218,28 +222,24 @@ __global__ void __launch_bounds__(kNT, LINES == 16 ? 4 : 2) k_cols(const Args g)
       }
       const double tot = block_sum_nt<kNT>(acc, red);
       if (t == 0) g.lpart[size_t(b) * g.nblk + blk] = tot;
-      if (g.mode == COLS_GRAD) {
-        ln.pad(g.plan);
-        ln.run(g.plan);
-        for (int p = t / LINES; p < M; p += kNT / LINES)
-          if (in) Xb[size_t(p) * N] = c_conj(ln.get(g.plan, cl, p));
-      }
-    } else {
+      if (g.mode == COLS_LOSS) break;
+    }
+    if (g.mode != COLS_LOSS && in)
       for (int p = t / LINES; p < M; p += kNT / LINES) {
-        if (!in) break;
         const float2 v = ln.get(g.plan, cl, p);
+        if (g.mode == COLS_GRAD || g.mode == COLS_FD_INV) {
+          Xb[size_t(p) * N] = c_conj(v);
+          continue;
+        }
         const float I = fmaf(v.x, v.x, v.y * v.y);
         const int s = shifted(p, q, M, N);
         if (g.mode == COLS_INTENSITY) {
           a.I_out[size_t(b) * MN + s] = I;
-        } else if (g.mode == COLS_FD) {
+        } else {
           Xb[size_t(p) * N] = v;
           dW[s] = sqrtf(__ldg(Im + s) + kEps) - sqrtf(I + kEps);
-        } else {
-          Xb[size_t(p) * N] = c_conj(v);
         }
       }
-    }
     __syncthreads();  // the buffers are free for the next group
   }
 }
@@ -297,7 +297,7 @@ static int launch(K kern, PtyDevCache& attr, const Args& g, size_t smem, cudaStr
         return PTYCHO_ERR_LAUNCH;
       attr.put(dev, nsm);
     }
-    const int per_sm = int(233472 / (smem + 1024 + 128));
+    const int per_sm = int(233472 / (smem + 1024 + 256));
     const int slots = nsm * (per_sm < 1 ? 1 : (per_sm > 4 ? 4 : per_sm));
     kern<<<g.ngroups < slots ? g.ngroups : slots, kNT, smem, s>>>(g);
     if (cudaGetLastError() == cudaSuccess) return PTYCHO_OK;

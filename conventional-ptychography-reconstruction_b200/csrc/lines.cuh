@@ -272,6 +272,39 @@ PTY_DEVI void pass_prime(const Pass& ps, int len, float2* __restrict__ src, floa
   else prime_sums<LINES, NT, 4>(ps, len, src, dst, tw, lines, ls, t);
 }
 
+// All passes of the lines in a, with b the other buffer; the result is in b after an odd
+// number of them.  The butterflies of fourteen radices are most of a kernel's code, so
+// they are inlined once: with a copy each for the loss's second transform, Bluestein's
+// way back and its filter, the first step of a process on 192^2 took 4.6 ms (2.8 here)
+// and every later one, 64 patterns, 110 us (106).  As one function for all kernels the
+// first takes 2.4 ms, but its callers spill: 117 us.
+template <int LINES, int NT>
+PTY_DEVI void run_passes(const Pass* passes, int np, int m, float2* a, float2* b, const float2* tw, int lines, int ls,
+                         int t) {
+  __syncthreads();
+#pragma unroll 1
+  for (int i = 0; i < np; ++i) {
+    const Pass& ps = passes[i];
+    switch (ps.R) {
+#define PTY_LN(R) \
+  case R: pass_r<LINES, NT, R>(ps, a, b, tw, lines, ls, t); break;
+      PTY_LN(2) PTY_LN(3) PTY_LN(4) PTY_LN(5) PTY_LN(6) PTY_LN(7) PTY_LN(8) PTY_LN(9) PTY_LN(10) PTY_LN(11)
+      PTY_LN(12) PTY_LN(13) PTY_LN(15) PTY_LN(16)
+#undef PTY_LN
+      default: pass_prime<LINES, NT>(ps, m, a, b, tw, lines, ls, t); break;
+    }
+    __syncthreads();
+    float2* c = a;
+    a = b;
+    b = c;
+  }
+}
+// the same for Bluestein's filter, once per CTA: a function of its own
+template <int NT>
+__device__ __noinline__ void one_line(const Pass* passes, int np, int m, float2* a, float2* b, const float2* tw, int ls) {
+  run_passes<0, NT>(passes, np, m, a, b, tw, 1, ls, threadIdx.x);
+}
+
 // The lines and tables of a CTA of NT threads.  Use: put() every value of every
 // line, pad(), run(), then get() every value; put() may follow a get() of the same
 // place.  (Passes that read from and write to global memory directly would save a
@@ -298,15 +331,18 @@ struct Lines {
       // one-line transform uses whole-line addressing in the two buffers
       for (int i = t; i < p.n; i += NT) ch[i] = cis_ratio(int((long long)i * i % (2 * p.n)), 2 * p.n);
       __syncthreads();
-      Lines<0, NT> one{cur, alt, tw, bf, ch, 1, ls, t};
       const float inv = 1.0f / float(p.m);
       for (int i = t; i < p.m; i += NT) {
         const int j = i < p.n ? i : p.m - i;
         const float2 c = j < p.n ? ch[j] : make_float2(0.f, 0.f);
-        one.cur[slot<0>(0, i, ls)] = make_float2(c.x * inv, -c.y * inv);
+        cur[slot<0>(0, i, ls)] = make_float2(c.x * inv, -c.y * inv);
       }
-      one.passes(p);
-      for (int i = t; i < p.m; i += NT) bf[i] = one.cur[slot<0>(0, i, ls)];
+      __shared__ Pass sp[kMaxPasses];
+      if (t < p.np) sp[t] = p.p[t];
+      __syncthreads();
+      one_line<NT>(sp, p.np, p.m, cur, alt, tw, ls);
+      const float2* f = p.np & 1 ? alt : cur;
+      for (int i = t; i < p.m; i += NT) bf[i] = f[slot<0>(0, i, ls)];
       __syncthreads();
     }
     return ch + (p.blue ? p.n : 0);
@@ -330,18 +366,8 @@ struct Lines {
   }
 
   PTY_DEVI void passes(const Plan& p) {
-    __syncthreads();
-    for (int i = 0; i < p.np; ++i) {
-      const Pass& ps = p.p[i];
-      switch (ps.R) {
-#define PTY_LN(R) \
-  case R: pass_r<LINES, NT, R>(ps, cur, alt, tw, lines, ls, t); break;
-        PTY_LN(2) PTY_LN(3) PTY_LN(4) PTY_LN(5) PTY_LN(6) PTY_LN(7) PTY_LN(8) PTY_LN(9) PTY_LN(10) PTY_LN(11)
-        PTY_LN(12) PTY_LN(13) PTY_LN(15) PTY_LN(16)
-#undef PTY_LN
-        default: pass_prime<LINES, NT>(ps, p.m, cur, alt, tw, lines, ls, t); break;
-      }
-      __syncthreads();
+    run_passes<LINES, NT>(p.p, p.np, p.m, cur, alt, tw, lines, ls, t);
+    if (p.np & 1) {
       float2* c = cur;
       cur = alt;
       alt = c;
@@ -350,14 +376,16 @@ struct Lines {
 
   // DFT of every line (barriers on both sides)
   PTY_DEVI void run(const Plan& p) {
-    passes(p);
-    if (!p.blue) return;
-    for (int e = t; e < lines * p.m; e += NT) {
-      const int l = LINES == 0 ? e / p.m : e % lines, i = LINES == 0 ? e - l * p.m : e / lines;
-      float2& v = cur[slot<LINES>(l, i, ls)];
-      v = c_conj(c_mul(v, bf[i]));
+#pragma unroll 1
+    for (int back = 0;; ++back) {  // the passes' code once
+      passes(p);
+      if (back == p.blue) return;  // Bluestein: conj of the inverse transform; get() undoes the conj
+      for (int e = t; e < lines * p.m; e += NT) {
+        const int l = LINES == 0 ? e / p.m : e % lines, i = LINES == 0 ? e - l * p.m : e / lines;
+        float2& v = cur[slot<LINES>(l, i, ls)];
+        v = c_conj(c_mul(v, bf[i]));
+      }
     }
-    passes(p);  // conj of the inverse transform; get() undoes the conj
   }
 };
 

@@ -415,7 +415,7 @@ static int launch_k(const Args& g, cudaStream_t st) {
         return PTYCHO_ERR_LAUNCH;
       attr.put(dev, nsm);
     }
-    const int per_sm = int(233472 / (smem + 1024));
+    const int per_sm = int(233472 / (smem + 1024 + 192));
     const int slots = nsm * (per_sm < 1 ? 1 : (per_sm > 4 ? 4 : per_sm));
     kern<<<dim3(g.ngroups < slots ? g.ngroups : slots, ADJ ? 1 : g.s - 1), NT, smem, st>>>(g);
     if (cudaGetLastError() == cudaSuccess) return PTYCHO_OK;
