@@ -164,12 +164,13 @@ PTY_DEVI void sincos_rr(u64 a, u64* s, u64* c) {
   *c = pk(c0, c1);
 }
 
-// exp(x) = 2^(x log2 e) of a pair; results below the normal range flush to zero
+// exp(x) = 2^(x log2 e) of a pair, down to the smallest floats (flushing those below the
+// normal range to zero would save 0.7 % of the forward and backward together)
 PTY_DEVI u64 exp_fast(u64 x) {
   float a, b, ya, yb;
   upk(mul2(x, pk(1.44269504088896341f)), a, b);
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(ya) : "f"(a));
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(yb) : "f"(b));
+  asm("ex2.approx.f32 %0, %1;" : "=f"(ya) : "f"(a));
+  asm("ex2.approx.f32 %0, %1;" : "=f"(yb) : "f"(b));
   return pk(ya, yb);
 }
 
