@@ -150,10 +150,19 @@ PTY_DEVI void st8_split(unsigned char* hi, int f, unsigned char* lo, int f_lo, i
 
 // sin and cos of a pair after Cody-Waite reduction by 2 pi (two-constant split of
 // 2 pi: the float nearest 2 pi plus its residual), then the SFU on [-pi, pi].
-// The nearest integer comes from adding and taking off 1.5 2^23 (exact below
-// 2^22): rintf runs at 16 a clock on the unit that sin, cos and exp need.
+// The nearest integer comes from adding and taking off 1.5 2^23 (rintf runs at 16 a
+// clock on the unit that sin, cos and exp need), with the argument's sign: the sum then
+// stays where floats are whole numbers, every one below 2^22 turns and even ones beyond.
+// (Against a positive constant, turns below -2^22 came out as halves, and the phase off
+// by pi.)  The sign comes from a saturated product: as bit operations, whose unit the
+// BF16 conversions load, forward and backward of 4,194,304 coordinates take 1836 us, this
+// way 1795, without the sign 1766.
 PTY_DEVI void sincos_rr(u64 a, u64* s, u64* c) {
-  const u64 k = add2(add2(mul2(a, pk(0.159154943091895336f)), pk(12582912.f)), pk(-12582912.f));
+  float a0, a1;
+  upk(a, a0, a1);
+  const u64 pos = pk(__saturatef(fmaf(a0, 1e30f, 0.5f)), __saturatef(fmaf(a1, 1e30f, 0.5f)));  // 1, or 0 where negative
+  const u64 m = fma2(pos, pk(25165824.f), pk(-12582912.f));
+  const u64 k = sub2(fma2(a, pk(0.159154943091895336f), m), m);
   u64 r = fma2(k, pk(-6.28318548202514648f), a);
   r = fma2(k, pk(1.74845553e-7f), r);
   float r0, r1, s0, s1, c0, c1;
