@@ -5,8 +5,8 @@
 //   X[k] = sum_n a[n*S] * exp(-+ 2 pi i n k / R)   (minus: forward, plus: INV).
 // All indices are compile-time constants, so after inlining the arrays live in
 // registers.  Radix 16 is 4x4 Cooley-Tukey, radix 8 is 2x4; the internal
-// twiddles are the exact constants cos/sin(pi/8), cos/sin(pi/4).  Radix 3, 5
-// and 7 use the symmetric pair form with exact cos/sin(2 pi q / P).
+// twiddles are the exact constants cos/sin(pi/8), cos/sin(pi/4).  Radices 3 to 13
+// that are odd primes use the symmetric pair form (dft_odd).
 #pragma once
 #include "common.cuh"
 
@@ -114,25 +114,43 @@ PTY_DEVI void dft16(float2* a) {
     for (int k2 = 0; k2 < 4; ++k2) a[(k1 + 4 * k2) * S] = t[4 * k1 + k2];
 }
 
-// exact cos / sin(2 pi q / P) for the odd primes 3, 5, 7 (q = 0 .. P-1)
-template <int P>
-__host__ __device__ constexpr float odd_cos(int q) {
-  q %= P;
-  if (q > P / 2) q = P - q;
-  if (q == 0) return 1.f;
-  if constexpr (P == 3) return -0.5f;
-  if constexpr (P == 5) return q == 1 ? 0.30901699437494742410f : -0.80901699437494742410f;
-  return q == 1 ? 0.62348980185873353053f : (q == 2 ? -0.22252093395631440429f : -0.90096886790241912624f);
+// cos and sin of 2 pi j / n at compile time: the angle is brought to [0, pi/4] by
+// symmetry, then summed as a Taylor series in double
+struct CosSin {
+  double c, s;
+};
+__host__ __device__ constexpr CosSin cos_sin_2pi(int j, int n) {
+  j %= n;
+  const int oct = 8 * j / n;  // octant
+  // angle = oct pi/4 + rest, rest = 2 pi (8 j - oct n) / (8 n); odd octants run backwards
+  const double step = 0.78539816339744830962 * double(8 * j - oct * n) / double(n);
+  const double x = (oct & 1) ? 0.78539816339744830962 - step : step;
+  double c = 1.0, s = x, tc = 1.0, ts = x;
+  for (int k = 1; k < 12; ++k) {
+    tc *= -x * x / double((2 * k - 1) * (2 * k));
+    ts *= -x * x / double((2 * k) * (2 * k + 1));
+    c += tc;
+    s += ts;
+  }
+  const bool swap = (((oct + 1) / 2) & 1) != 0;  // octants 1, 2, 5, 6
+  const double u = swap ? s : c, v = swap ? c : s;
+  return {(oct >= 2 && oct < 6) ? -u : u, oct >= 4 ? -v : v};
 }
-template <int P>
-__host__ __device__ constexpr float odd_sin(int q) {
-  q %= P;
-  const float sg = q > P / 2 ? -1.f : 1.f;
-  if (q > P / 2) q = P - q;
-  if (q == 0) return 0.f;
-  if constexpr (P == 3) return sg * 0.86602540378443864676f;
-  if constexpr (P == 5) return sg * (q == 1 ? 0.95105651629515357212f : 0.58778525229247312917f);
-  return sg * (q == 1 ? 0.78183148246802980871f : (q == 2 ? 0.97492791218182360702f : 0.43388373911755812048f));
+
+// cos, sin(2 pi j / n) rounded to float, as a table that unrolled code indexes
+template <int N>
+struct CosSinTable {
+  float c[N], s[N];
+};
+template <int N>
+__host__ __device__ constexpr CosSinTable<N> cos_sin_table() {
+  CosSinTable<N> t{};
+  for (int j = 0; j < N; ++j) {
+    const CosSin w = cos_sin_2pi(j, N);
+    t.c[j] = float(w.c);
+    t.s[j] = float(w.s);
+  }
+  return t;
 }
 
 // odd prime P: pairs a_m +- a_{P-m} give, for r = 1 .. (P-1)/2,
@@ -142,6 +160,7 @@ __host__ __device__ constexpr float odd_sin(int q) {
 template <int P, bool INV, int S>
 PTY_DEVI void dft_odd(float2* a) {
   constexpr int h = (P - 1) / 2;
+  constexpr CosSinTable<P> w = cos_sin_table<P>();
   float2 sp[h], sm[h];
   float2 x0 = a[0], sum = a[0];
 #pragma unroll
@@ -155,7 +174,7 @@ PTY_DEVI void dft_odd(float2* a) {
     float2 A = x0, Bv = make_float2(0.f, 0.f);
 #pragma unroll
     for (int m = 1; m <= h; ++m) {
-      const float c = odd_cos<P>(m * r), s = odd_sin<P>(m * r);
+      const float c = w.c[m * r % P], s = w.s[m * r % P];
       A = make_float2(fmaf(sp[m - 1].x, c, A.x), fmaf(sp[m - 1].y, c, A.y));
       Bv = make_float2(fmaf(sm[m - 1].x, s, Bv.x), fmaf(sm[m - 1].y, s, Bv.y));
     }

@@ -324,7 +324,6 @@ __global__ void __launch_bounds__(256) k_hash_bwd_thread(const int* __restrict__
 // hashgrid.py GridPlan).
 // ---------------------------------------------------------------------------
 struct GridArgs {
-  const int* ix0;
   const int* iy1;
   const int* lo0;
   const int* lo1;
@@ -823,8 +822,7 @@ int ptycho_hashgrid_backward_grid(const int32_t* grid_int, const float* grid_fra
   // layout of grid_int: ix0 [L][Bj], iy1 [L][A], lo0 [sum (E0 + 1)], lo1 [sum (E1 + 1)],
   // vstart [entries + 1], vorder [vertices]; grid_frac: fx0 [L][Bj], fy1 [L][A]
   size_t off = 0;
-  g.ix0 = grid_int + off;
-  off += size_t(n_levels) * Bj;
+  off += size_t(n_levels) * Bj;  // (ix0: no kernel reads it)
   g.iy1 = grid_int + off;
   off += size_t(n_levels) * A;
   g.lo0 = grid_int + off;
