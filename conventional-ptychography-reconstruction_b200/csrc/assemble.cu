@@ -293,8 +293,8 @@ int launch_assemble(const float2* Eb, const float2* O, const float2* P, const in
   // dO tiles 64 columns wide for windows of 256 columns or more (fewer
   // blocks scanning the batch, more pixels per hit: c3 +3 %, c4 +6 %), 32
   // below (c1: 64 measured 1 % slower).  Compile-time row lengths and signs and
-  // row tests taken out of the inner sums: c1 66.7 -> 63.0, c3 70.1 -> 67.5, c4 429
-  // -> 423 us a step
+  // row tests taken out of the inner sums: c1 67.1 -> 64.3, c3 68.5 -> 66.8, c4 427
+  // -> 420 us a step
   const int tw = N >= 256 ? 64 : 32;
   a.ntx = (W + tw - 1) / tw;
   const int ntiles = dO ? a.ntx * ((H + kTile - 1) / kTile) : 0;

@@ -8,8 +8,8 @@ under ``_build/`` and linked into ``../libptycho_b200.so``.  Objects are rebuilt
 when their source or any header in this folder (or ``include/``) is newer.
 ``fastabi.c`` (a CPython fast-call binding of the per-step entry points) is
 compiled by the host C compiler into ``../_fastabi<EXT_SUFFIX>``, and
-``torch_ext.cpp`` (the fused loss's autograd node, host C++ against libtorch)
-by the host C++ compiler into ``../_torchext<EXT_SUFFIX>``.
+``torch_ext.cpp`` (the autograd nodes of the fused loss, the MLP and the
+upsampling, host C++ against libtorch) by the host C++ compiler into ``../_torchext<EXT_SUFFIX>``.
 No GPU is needed: nvcc cross-compiles.
 """
 from __future__ import annotations
@@ -77,8 +77,8 @@ def build_fastabi(force: bool = False) -> str:
 
 
 def build_torchext(force: bool = False) -> str:
-    """The torch autograd node of the fused loss (host C++ against libtorch,
-    no CUDA code: it calls libptycho_b200.so through bound addresses)."""
+    """The torch autograd nodes of the fused loss, the MLP and the upsampling (host
+    C++ against libtorch, no CUDA code: it calls libptycho_b200.so through bound addresses)."""
     import torch
 
     src = os.path.join(HERE, "torch_ext.cpp")

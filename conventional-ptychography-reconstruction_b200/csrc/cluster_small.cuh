@@ -17,9 +17,9 @@
 // cluster barriers).  Every sum has a fixed order: results are bitwise
 // deterministic.
 // Bound by latency: two global round trips, four line transforms and two (FD: four)
-// cluster barriers.  Whole steps on B200 against a pattern per SM: 10 patterns of
-// 128^2 33.2 -> 23.0 us, FD 49.8 -> 27.1; 10 of 256^2, FD, 78.4 -> 33.5 (a cluster of
-// four, 32 values a thread).  small_batch_max (fused.cuh) says which batches come here.
+// cluster barriers.  Whole captured steps on B200 against a pattern per SM: 10 patterns
+// of 128^2 33.2 -> 23.0 us, FD 49.8 -> 27.1; 10 of 256^2, FD, 78.4 -> 33.5 (a cluster of
+// four, 32 values a thread); an eager call of that takes 86 us of host time either way.  small_batch_max (fused.cuh) says which batches come here.
 // Sixteen CTAs are more than the portable eight: a partition of the chip may not hold
 // them together.  M = 256 runs eight CTAs of 32 rows there (large_clusters, fused.cuh):
 // on a whole B200 10 FD patterns 30.8 us against 26.9, 200 355 : 343, intensities

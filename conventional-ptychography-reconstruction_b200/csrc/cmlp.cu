@@ -36,11 +36,11 @@
 // ones column yields the bias gradients).  In a tile's 256 threads, warp w
 // reads TMEM lane quarter w & 3 (tile rows 32 (w & 3) .. +31) and does the
 // elementwise work of half w >> 2 of each layer's complex units.
-// Measured on B200, 4,194,304 coordinates: forward 495 us (820 as four serial
-// steps, two CTAs per SM, rintf and single conversions), backward 1312 us (1905
+// Measured on B200, 4,194,304 coordinates: forward 523 us (820 as four serial
+// steps, two CTAs per SM, rintf and single conversions), backward 1322 us (1905
 // as nine serial steps, one tile in flight).  The forward is bound by its 256
-// sin / cos / exp results per coordinate (236 us) and issue (60 %); the backward
-// by latency with two tiles in flight (issue 35 %), which is all that shared
+// sin / cos / exp results per coordinate (236 us) and issue (65 %); the backward
+// by latency with two tiles in flight (issue 39 %), which is all that shared
 // memory (100 KB a tile) and TMEM (256 accumulator columns + 128 a tile) hold.
 //
 // Each CTA writes its raw accumulators once; k_cmlp_reduce sums the CTA

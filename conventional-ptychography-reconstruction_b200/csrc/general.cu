@@ -17,11 +17,11 @@
 // pattern forms the stencil through three float planes of the workspace, and a
 // second column pass starts from the gradient.  Every reduction has a fixed
 // order: results are bitwise deterministic.
-// Measured on B200 (batch 64 of 192^2, smooth L1, a step with its assembly): 111 us
+// Measured on B200 (batch 64 of 192^2, smooth L1, a step with its assembly): 106 us
 // against 241 as seven passes with run-time radix loops (gather 9, lines 31 + 43 +
-// 43 + 32, one CTA per pattern for the loss 43); here rows 21, columns 34, inverse
-// rows 17, assembly 12.  251^2, batch 32: 291 against 1815 us (prime length).  Bound
-// by issue and latency: about 110 instructions a value and transform.
+// 43 + 32, one CTA per pattern for the loss 43).  251^2, batch 32: 285 against 1815 us
+// (prime length).  Bound by issue and latency: about 110 instructions a value and
+// transform.
 #include <cuda_runtime.h>
 #include <stdint.h>
 

@@ -106,9 +106,10 @@ PTY_DEVI int cell_of(float p, float& f) {
 // adds, the dense and hashed levels in loops of their own (one compare covers a
 // dense cell's four corners, the modulo only where the last is past the level's
 // end), 1024^2 coordinates and 16 levels take 51 us
-// (57 with floorf and corner_entry; 1.9 TB/s; two or four coordinates per thread
-// measured 3 and 15 us more).  The short loops hold for coordinates in [0, 1] and scales below 2^20; any other
-// coordinate takes the general one, bitwise the same where both apply.
+// (57 with floorf and corner_entry; 134 MB of features, 2.6 TB/s; two or four
+// coordinates per thread measured 3 and 15 us more).  The short loops hold for
+// coordinates in [0, 1] and scales below 2^20; any other coordinate takes the
+// general one, bitwise the same where both apply.
 template <bool PLANAR>
 __global__ void __launch_bounds__(256) k_hash_fwd(const float2* __restrict__ coords, int N,
                                                   const float2* __restrict__ table, const LevelTable L,

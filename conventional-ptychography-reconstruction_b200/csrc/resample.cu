@@ -55,8 +55,8 @@ namespace sh {
 // a and b are part of the inverse's twiddles.  An exchange writes value (a, q) at a P + q or
 // (a, q0, b) at a P + 17 q0 + b, P = 17 C: conflict free both ways for 8-byte
 // accesses of a half-warp (P = C, 17 = 1 mod 16).
-// Measured on B200, 2048^2 to 4096^2 and back: 286 us for the four passes (49 + 77
-// up, 93 + 64 down) against 668 us by padded spectra; bound by latency (issue 35 to
+// Measured on B200, 2048^2 to 4096^2 and back: 279 us for the four passes (48 + 72
+// up, 79 + 66 down) against 668 us by padded spectra; bound by latency (issue 35 to
 // 40 %, four to seven barriers between loads and stores), 336 MB would take 51 us.
 // Columns: COLS adjacent columns per CTA, interleaved in shared memory the same
 // way, so global accesses are pieces of 8 COLS bytes.
@@ -273,7 +273,7 @@ static int dispatch(int n, const Args& g, cudaStream_t st) {
 // at (k + d) mod N, d = floor(n/2) + floor((N-n)/2) - floor(N/2): d = 0 for even n,
 // or odd n and odd N; d = -1 for odd n and even N (the reference's half-bin
 // asymmetry, kept): every sample j of the long line is turned by exp(2 pi i d j / N).
-// Measured on B200: 1500^2 to 3000^2 71 + 118 us against 213 + 141 by padded spectra
+// Measured on B200: 1500^2 to 3000^2 61 + 113 us against 213 + 141 by padded spectra
 // with run-time radix loops; 498^2 to 996^2 and back 118 against 675 us (factor 83).
 // ---------------------------------------------------------------------------
 namespace rsg {

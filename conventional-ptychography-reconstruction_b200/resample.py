@@ -6,9 +6,10 @@ models/complex_inr.py:252-271 computes with torch.fft:
 backward pass (the operator's conjugate transpose) on the same kernels
 (``ptycho_fourier_upsample`` / ``ptycho_fourier_upsample_adjoint``).
 Sizes: any h, w >= 1 and integer s >= 1 with h*s, w*s <= 8192 (``supported``).
-Power-of-two lines run compile-time radix-8/16 kernels; every other length
-(the multiples of 3 that Recovery.py's canvases give, odd lengths, large
-prime factors) runs the run-time-planned mixed-radix kernel.  There is no
+Lines of 256, 512, 1024 and 2048 points with s = 2 or 4 and s times the length
+at most 4096 run compile-time radix-16 kernels; every other length (the
+multiples of 3 that Recovery.py's canvases give, odd lengths, large prime
+factors) and scale runs the run-time-planned mixed-radix kernel.  There is no
 torch.fft path: other shapes raise.
 """
 from __future__ import annotations

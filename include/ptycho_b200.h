@@ -81,13 +81,17 @@ int ptycho_version(void);
  *   I_out[b] = | fftshift( fft2( P * O[tlY_f : tlY_f+M, tlX_f : tlX_f+N] ) ) |^2
  * O [H][W] complex64, P [M][N] complex64, I_out [B][M][N] float32.
  * ptycho_forward_intensity takes M == N in {64, 128, 256} (a pattern per SM,
- * or per thread-block cluster of M / 16 CTAs) and needs no scratch memory; other shapes return PTYCHO_ERR_UNSUPPORTED_SIZE.
+ * or per thread-block cluster) and needs no scratch memory; other shapes
+ * return PTYCHO_ERR_UNSUPPORTED_SIZE.
  * ptycho_forward_intensity_ws takes any 1 <= M, N <= 4096 (the reference
  * accepts any probe shape, Recovery.py:290): shapes the fused kernels do not
- * cover run as gather, mixed-radix row and column DFTs and an intensity
- * pass over a workspace of ptycho_forward_intensity_workspace_size(M, N, B)
- * bytes (256-byte aligned).  64 and 128 need none; 256 runs row and column
- * kernels over it, or with a smaller (or no) workspace the cluster kernel.
+ * cover run as two passes (gather and row DFTs, column DFTs and |F|^2) over
+ * a workspace of ptycho_forward_intensity_workspace_size(M, N, B) bytes
+ * (256-byte aligned).  64 and 128 need none; 256 runs row and column kernels
+ * over it (up to 256 MB), or with a smaller (or no) workspace the cluster
+ * kernel.  Which kernel runs depends on the batch, so a pattern's intensities
+ * (and below its loss and gradient terms) can differ in their last bits from
+ * one batch size to another.
  * ---------------------------------------------------------------------- */
 int ptycho_forward_intensity(const float* O, int H, int W, const float* P, int M, int N,
                              const int32_t* tl, int F, const int32_t* batch, int B,
@@ -119,12 +123,13 @@ int ptycho_forward_intensity_ws(const float* O, int H, int W, const float* P, in
  * three line-DFT kernels over the workspace (smooth-L1, Poisson and the
  * intensity-gradient code; batches of 192 or more also take dP from the
  * inverse-row kernel); small batches of the three, and the FD loss at 256, run
- * one thread-block cluster of M / 16 CTAs per pattern; any other
+ * one thread-block cluster per pattern (M / 16 CTAs; at 256, where the device
+ * cannot hold 16 together, 8 for the FD loss, and the line-DFT kernels for
+ * the others); any other
  * 1 <= M, N <= 4096 (non-square, odd, 96, 192, ...) runs the general path: the
  * same losses and gradients through three workspace passes (gather and row
  * DFTs of any length, column DFTs with the loss and their inverse, inverse
- * row DFTs), then the
- * same assembly.
+ * row DFTs), then the same assembly.
  * ---------------------------------------------------------------------- */
 size_t ptycho_fwd_adj_workspace_size(int H, int W, int M, int N, int B);
 
@@ -291,8 +296,9 @@ int ptycho_residual_backward(const float* k, const float* m, const float* g, lon
  * x [h][w] complex64 -> y [h*s][w*s] complex64, the pad centred at
  * ((h*s - h)/2, (w*s - w)/2).  The adjoint maps an upstream gradient gy
  * [h*s][w*s] to gx [h][w] (torch's complex convention; the operator's
- * conjugate transpose).  h, w, h*s and w*s must be powers of two in
- * [64, 4096] with s in {1, 2, 4}; otherwise PTYCHO_ERR_UNSUPPORTED_SIZE.
+ * conjugate transpose).  Any h, w, s >= 1 with h*s, w*s <= 8192; beyond,
+ * PTYCHO_ERR_UNSUPPORTED_SIZE.  A NaN or infinity anywhere in the input
+ * leaves no output finite, as through the FFTs.
  * workspace: device scratch of ptycho_fourier_upsample_workspace_size()
  * bytes (the intermediate between the two passes), 8-byte aligned.
  * ---------------------------------------------------------------------- */
