@@ -24,13 +24,14 @@ constexpr int kMaxPasses = 8;
 constexpr int kMaxLen = 8192;
 constexpr size_t kSmemCap = 200 * 1024;
 // Largest prime that is summed directly.  The pair sums are closer to 64 bits than a
-// plain direct sum (0.46 to 0.81 of its error for any prime); Bluestein's chirp transform
-// adds an error of its own, 1.2 to 2.1 times the plain sum's for most lengths with a prime
-// of 17 to 47 and up to 1.25 at 149, always below it (0.4 to 0.8) from 157 on.  Steps of
-// 64 patterns on B200, pairs : Bluestein: 119^2 86 : 133 us, 148^2 131 : 209, 194^2 297 :
-// 470, 226^2 393 : 469, 127^2 165 : 135, 254^2 513 : 552, 149^2 248 : 213, 179^2 380 :
-// 357, 251^2 812 : 530.
-constexpr int kDirectPrime = 151;
+// plain direct sum (0.46 to 0.81 of its error for any prime).  Bluestein's chirp transform
+// adds an error of its own: 1.2 to 2.1 times the plain sum's for most lengths with a prime
+// of 17 to 47, 0.5 to 1.5 for 53 to 97, and 0.4 to 0.9 beyond (149 alone 0.8 to 1.25,
+// by loss).  Steps on B200, pairs : Bluestein: 64 patterns 119^2 86 : 133 us, 148^2 131 :
+// 209, 194^2 297 : 470, 226^2 393 : 469, 127^2 165 : 135, 149^2 248 : 213, 251^2 812 : 530;
+// 100 patterns 101^2 160 : 154, 113^2 203 : 193, 127^2 264 : 176, 151^2 409 : 307; 4 of
+// 226^2 82 : 72, 254^2 92 : 70, 302^2 121 : 98.
+constexpr int kDirectPrime = 113;
 
 struct Pass {
   int R, NS, bpl, tws;   // radix, product of the radices before, butterflies per line, twiddle stride

@@ -104,7 +104,9 @@ def _as_c64(x: torch.Tensor, name: str) -> torch.Tensor:
         raise ValueError(f"{name} must be a CUDA tensor (there is no CPU path)")
     if x.dtype != torch.complex64:
         x = x.to(torch.complex64)
-    return _lib.plain(x)
+    if x.is_conj() or x.is_neg():  # _lib.plain without its call (host time of small calls)
+        x = _lib.plain(x)
+    return x.contiguous()
 
 
 def _check_probe(P: torch.Tensor):
@@ -180,7 +182,7 @@ def forward_intensity(O: torch.Tensor, P: torch.Tensor, tl: torch.Tensor, batch=
         raise ValueError("object and probe must be on one device")
     M, N = _check_probe(P)
     H, W = O.shape
-    tl = tl.to(device=O.device, dtype=torch.int32).contiguous()
+    tl = _i32(tl, O.device)
     F = int(tl.shape[0])
     bt = _batch_arg(batch, O.device)
     B = F if bt is None else int(bt.numel())
