@@ -131,6 +131,10 @@ def device_status(device) -> torch.Tensor:
     st = _status_cache.get(device)
     if st is None:
         st = torch.zeros(1, dtype=torch.int32, device=device)
+        try:
+            st.data_ptr()
+        except RuntimeError:  # a functorch transform's wrapper: its call is refused, later ones are not
+            return st
         _status_cache[device] = st
     return st
 
